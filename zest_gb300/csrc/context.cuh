@@ -77,7 +77,7 @@ struct EvalBufs {
 
 struct FftEntry {
     FftPlan plan;
-    DevBuf tw;
+    DevBuf tab, rows;
 };
 
 // Folded Legendre tables (forward: weights * quadrature prefactor folded in;

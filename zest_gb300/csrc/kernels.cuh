@@ -4,17 +4,32 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <vector>
 
 namespace zgpu {
 
 // ---- longitude FFT ----------------------------------------------------------
-struct FftPlan {
-    int N = 0;            // transform length
-    int nst = 0;          // number of Stockham stages
-    int radix[24] = {};   // radix of each stage (product = N)
-    const double2* tw = nullptr;  // device table W_t = exp(-2 pi i t / N), t < N
+// One operation of a plan (fft.cu) on the rows of a CTA's column block: a
+// Stockham stage of radix R along a dimension of Nd rows, `inner` rows apart,
+// in `outer` slices `ostride` rows apart from row `base`; R = 0: the product in
+// the middle of a Rader dimension.  tab: its roots in the plan's table.
+struct FftOp {
+    int R, Nd, Ns, base, outer, ostride, inner, tab;
 };
-size_t fft_smem_bytes(int N, int NC);
+constexpr int kFftMaxOps = 40;
+struct FftPlan {
+    int N = 0;     // transform length
+    int nops = 0;
+    int ntab = 0;  // complex entries of the table
+    FftOp ops[kFftMaxOps] = {};
+    const double2* tab = nullptr;    // device: roots of unity and Rader products
+    const int* in_row = nullptr;     // device: row of input index i, i < N
+    const int* out_row = nullptr;    // device: row of output index k, k < N
+};
+// Plan of length N: its operations, the table (re, im pairs) and the row maps
+// (in_row, then out_row) for the caller to upload.
+int build_fft_plan(int N, FftPlan& plan, std::vector<double>& tab, std::vector<int>& rows, bool allow_rader);
+size_t fft_smem_bytes(const FftPlan& plan, int NC);
 // forward: x(b, i, col) at x + b*xb + i*si + col*sc, i < N, col < C
 //          -> F[((b*nm + m)*C + col)*2 + {re,im}] = conj(X_m), m < nm
 int launch_rfft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, long long xb, long long si, long long sc,

@@ -52,33 +52,22 @@ static int set_device(zest_gpu_context* ctx) {
     return ZEST_GPU_OK;
 }
 
-static void factorize(int N, FftPlan& p) {
-    p.N = N;
-    p.nst = 0;
-    int n = N;
-    while (n % 4 == 0) { p.radix[p.nst++] = 4; n /= 4; }
-    while (n % 2 == 0) { p.radix[p.nst++] = 2; n /= 2; }
-    for (int q = 3; n > 1; q += 2)
-        while (n % q == 0) { p.radix[p.nst++] = q; n /= q; }
-}
-
 static int get_fft(zest_gpu_context* ctx, int N, const FftPlan** out) {
     auto it = ctx->ffts.find(N);
     if (it == ctx->ffts.end()) {
         auto e = std::make_unique<FftEntry>();
-        factorize(N, e->plan);
-        if (e->plan.nst > 24) return fail(ZEST_GPU_ERR_UNSUPPORTED, "FFT length has too many factors");
-        if (fft_smem_bytes(N, 1) > 220 * 1024) return fail(ZEST_GPU_ERR_UNSUPPORTED, "FFT length too large");
-        std::vector<double> tw(2 * (size_t)N);
-        const double pi = 3.14159265358979323846264338327950288;
-        for (int t = 0; t < N; ++t) {
-            // W_t = exp(-2 pi i t/N), evaluated on the reduced angle for accuracy
-            const double ang = 2.0 * pi * double(t) / double(N);
-            tw[2 * t] = std::cos(ang);
-            tw[2 * t + 1] = -std::sin(ang);
-        }
-        ZG_TRY(upload(e->tw, tw, ctx->stream));
-        e->plan.tw = e->tw.as<double2>();
+        std::vector<double> tab;
+        std::vector<int> rows;
+        int rc = build_fft_plan(N, e->plan, tab, rows, true);
+        if (rc != ZEST_GPU_OK || fft_smem_bytes(e->plan, 1) > 220 * 1024)
+            rc = build_fft_plan(N, e->plan, tab, rows, false);
+        if (rc != ZEST_GPU_OK) return fail(rc, "FFT length has too many factors");
+        if (fft_smem_bytes(e->plan, 1) > 220 * 1024) return fail(ZEST_GPU_ERR_UNSUPPORTED, "FFT length too large");
+        ZG_TRY(upload(e->tab, tab, ctx->stream));
+        ZG_TRY(upload(e->rows, rows, ctx->stream));
+        e->plan.tab = e->tab.as<double2>();
+        e->plan.in_row = e->rows.as<int>();
+        e->plan.out_row = e->plan.in_row + N;
         it = ctx->ffts.emplace(N, std::move(e)).first;
     }
     *out = &it->second->plan;
