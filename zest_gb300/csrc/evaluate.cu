@@ -134,12 +134,12 @@ __global__ void __launch_bounds__(256) zt_spectrum_kernel(int L, int batch, cons
     if (sum && gl == 0) out[bb * ostride + idx] = __dmul_rn(__dmul_rn(p[0], p[0]) + s, norm);
 }
 
-int upload_tiles(zest_gpu_context* ctx, DevBuf& buf, const std::vector<int4>& v, TileList* tl) {
+int upload_tiles(zest_gpu_context* ctx, DevBuf& buf, const std::vector<int4>& v, int variant, TileList* tl) {
     if (v.size() > 0x7fffffff) return fail(ZEST_GPU_ERR_UNSUPPORTED, "tile count overflow");
     ZG_TRY(upload(buf, v, ctx->stream));
     tl->tiles = buf.as<int4>();
     tl->count = int(v.size());
-    tl->variant = 0;
+    tl->variant = variant;
     return ZEST_GPU_OK;
 }
 
@@ -238,22 +238,27 @@ int zt_evaluate_dev(zest_gpu_context* ctx, int zn, int sn, int sp, int L, int ba
     const int per = eval_items_per_pass(per_item, batch);
     ZG_TRY(E.flm.ensure((size_t)tri_size(L) * per * nrad * 2 * sizeof(double)));
     ZG_TRY(E.G.ensure((size_t)L * nlat * per * nrad * 2 * sizeof(double)));
-    int bm, bn;
-    zt_tile_shape(0, bm, bn);
     int tiled_for = -1;
     TileList tr, tg, tn;
     for (int b0 = 0; b0 < batch; b0 += per) {
         const int nb = std::min(per, batch - b0);
         if (nb != tiled_for) {
             std::vector<int4> v;
+            int bm, bn;
+            int w = zt_tile_rule((long long)L * L * nb * nrad, nrad);
+            zt_tile_shape(w, bm, bn);
             for (int l = 0; l < L; ++l) add_tiles(v, l, nrad, (long long)(l + 1) * nb * 2, bm, bn);
-            ZG_TRY(upload_tiles(ctx, E.tiles[0], v, &tr));
+            ZG_TRY(upload_tiles(ctx, E.tiles[0], v, w, &tr));
             v.clear();
+            w = zt_tile_rule((long long)L * nlat * nb * 2 * nrad, nlat);
+            zt_tile_shape(w, bm, bn);
             for (int m = 0; m < L; ++m) add_tiles(v, m, nlat, (long long)nb * 2 * nrad, bm, bn);
-            ZG_TRY(upload_tiles(ctx, E.tiles[1], v, &tg));
+            ZG_TRY(upload_tiles(ctx, E.tiles[1], v, w, &tg));
             v.clear();
+            w = zt_tile_rule(nb * nlon * npts, nlon);
+            zt_tile_shape(w, bm, bn);
             for (int b = 0; b < nb; ++b) add_tiles(v, b, nlon, npts, bm, bn);
-            ZG_TRY(upload_tiles(ctx, E.tiles[2], v, &tn));
+            ZG_TRY(upload_tiles(ctx, E.tiles[2], v, w, &tn));
             tiled_for = nb;
         }
         {
@@ -292,20 +297,22 @@ int st_evaluate_dev(zest_gpu_context* ctx, int sn, int sp, int L, int batch, con
     const long long csz = 2 * tri_size(L);
     const int per = eval_items_per_pass((size_t)L * nlat * 2 * sizeof(double), batch);
     ZG_TRY(E.G.ensure((size_t)L * nlat * per * 2 * sizeof(double)));
-    int sbm, sbn, bm, bn;
-    st_tile_shape(sbm, sbn);
-    zt_tile_shape(0, bm, bn);
     int tiled_for = -1;
     TileList tg, tn;
     for (int b0 = 0; b0 < batch; b0 += per) {
         const int nb = std::min(per, batch - b0);
         if (nb != tiled_for) {
             std::vector<int4> v;
-            for (int m = 0; m < L; ++m) add_tiles(v, m, nlat, 2LL * nb, sbm, sbn);
-            ZG_TRY(upload_tiles(ctx, E.tiles[1], v, &tg));
+            int bm, bn;
+            int w = st_tile_variant(2 * nb);
+            st_tile_shape(w, bm, bn);
+            for (int m = 0; m < L; ++m) add_tiles(v, m, nlat, 2LL * nb, bm, bn);
+            ZG_TRY(upload_tiles(ctx, E.tiles[1], v, w, &tg));
             v.clear();
+            w = zt_tile_rule((long long)nb * nlon * nlat, nlon);
+            zt_tile_shape(w, bm, bn);
             for (int b = 0; b < nb; ++b) add_tiles(v, b, nlon, nlat, bm, bn);
-            ZG_TRY(upload_tiles(ctx, E.tiles[2], v, &tn));
+            ZG_TRY(upload_tiles(ctx, E.tiles[2], v, w, &tn));
             tiled_for = nb;
         }
         {

@@ -37,6 +37,17 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm64_kernel(const Pro
     const int M = P.M(g), N = P.N(g);
     const int tx = threadIdx.x % (BN / TN);
     const int ty = threadIdx.x / (BN / TN);
+    // The FP64 pipe sets the pace, so rows and K that do not exist are not
+    // multiplied: a warp covers few rows of the tile and all of its columns, and
+    // one whose rows all lie past M skips the products (the tile's padding
+    // costs its rows rounded up to WR, not to BM), and the K loop ends at K.
+    // Measured (whole tiles and K rounded up to BK before), ms:
+    // SH order 1024 x 8 forward 8.9 -> 7.7, Zernike order 100 x 32 Legendre 4.5 ->
+    // 3.4 and 4.2 -> 3.1, radial 1.4 -> 1.0; evaluation of 8 expansions of order
+    // 100 at 200 x 100 x 100 points 9.8 -> 7.8.
+    constexpr int WR = 32 / (BN / TN) * TM;  // rows per warp
+    const bool active = row0 + int(threadIdx.x) / 32 * WR < M;
+    static_assert(32 % (BN / TN) == 0, "a warp covers whole rows of the tile");
     double acc[NA][TM][TN];
 #pragma unroll
     for (int a = 0; a < NA; ++a)
@@ -64,8 +75,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm64_kernel(const Pro
                 Bs[k][n] = v;
             }
             __syncthreads();
-#pragma unroll
-            for (int k = 0; k < BK; ++k) {
+            auto step = [&](int k) {
                 double av[TM], bv[TN];
 #pragma unroll
                 for (int i = 0; i < TM; ++i) av[i] = As[k][ty * TM + i];
@@ -75,6 +85,15 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm64_kernel(const Pro
                 for (int i = 0; i < TM; ++i)
 #pragma unroll
                     for (int j = 0; j < TN; ++j) acc[par][i][j] = fma(av[i], bv[j], acc[par][i][j]);
+            };
+            if (active) {
+                if (k0 + BK <= K) {
+#pragma unroll
+                    for (int k = 0; k < BK; ++k) step(k);
+                } else {
+#pragma unroll 1
+                    for (int k = 0; k < K - k0; ++k) step(k);
+                }
             }
             __syncthreads();
         }
@@ -335,12 +354,17 @@ struct EvLon {
 };
 
 // tile shapes: Zernike sums have few rows and many columns; SH sums have
-// many rows (or K) and 2*batch columns.  The Zernike sums come in three
+// many rows (or K) and 2*batch columns.  The Zernike sums come in four
 // shapes of 256 threads (the autotuner picks one per stage and size): groups
-// have (L - m)/2 or (L + 1)/2 rows, so small orders waste most of a 64-row tile.
-//   variant 0: 64 x 64 (4 x 4 per thread), 1: 32 x 128 (2 x 8), 2: 16 x 128 (1 x 8)
+// have (L - m)/2 or (L + 1)/2 rows, so small orders waste most of a 64-row tile,
+// and a small batch of a small order needs one output per thread to reach all
+// SMs (order 20 x 1, forward and backward: 105 us with shapes 0 to 2, 54 with 3).
+//   variant 0: 64 x 64 (4 x 4 per thread), 1: 32 x 128 (2 x 8), 2: 16 x 128 (1 x 8),
+//   3: 8 x 32 (1 x 1)
+// SH shapes by the columns, since lanes past the last column multiply zeros:
+//   variant 0: 128 x 16 (4 x 2), 1: 64 x 8 (2 x 1), 2: 64 x 4 (1 x 1), 3: 128 x 2 (1 x 1)
 constexpr int ZBK = 8;
-constexpr int SBM = 128, SBN = 16, STM = 4, STN = 2, SBK = 8;
+constexpr int SBK = 8;
 
 template <class Prob, int BM, int BN, int TM, int TN, int BK>
 int run(cudaStream_t s, const Prob& p, const TileList& tl, const char* name) {
@@ -354,7 +378,18 @@ int run_zt(cudaStream_t s, const Prob& p, const TileList& tl, const char* name) 
     switch (tl.variant) {
     case 1: return run<Prob, 32, 128, 2, 8, ZBK>(s, p, tl, name);
     case 2: return run<Prob, 16, 128, 1, 8, ZBK>(s, p, tl, name);
+    case 3: return run<Prob, 8, 32, 1, 1, 2 * ZBK>(s, p, tl, name);
     default: return run<Prob, 64, 64, 4, 4, ZBK>(s, p, tl, name);
+    }
+}
+
+template <class Prob>
+int run_st(cudaStream_t s, const Prob& p, const TileList& tl, const char* name) {
+    switch (tl.variant) {
+    case 1: return run<Prob, 64, 8, 2, 1, SBK>(s, p, tl, name);
+    case 2: return run<Prob, 64, 4, 1, 1, SBK>(s, p, tl, name);
+    case 3: return run<Prob, 128, 2, 1, 1, SBK>(s, p, tl, name);
+    default: return run<Prob, 128, 16, 4, 2, SBK>(s, p, tl, name);
     }
 }
 
@@ -368,7 +403,7 @@ int launch_ev_zt_leg(cudaStream_t s, const LegMeta& lm, const TileList& tl, cons
 int launch_ev_st_leg(cudaStream_t s, const LegMeta& lm, const TileList& tl, const double* coeffs, double* G, int L,
                      int nlat, int batch, long long coeff_stride) {
     EvStLeg p{lm, coeffs, G, L, nlat, batch, coeff_stride};
-    return run<EvStLeg, SBM, SBN, STM, STN, SBK>(s, p, tl, "ev_st_leg");
+    return run_st(s, p, tl, "ev_st_leg");
 }
 int launch_ev_lon(cudaStream_t s, const TileList& tl, const double* trig, const double* G, double* values, int L,
                   int nlon, int npts) {
@@ -377,10 +412,28 @@ int launch_ev_lon(cudaStream_t s, const TileList& tl, const double* trig, const 
 }
 
 void zt_tile_shape(int variant, int& bm, int& bn) {
-    bm = variant == 1 ? 32 : (variant == 2 ? 16 : 64);
-    bn = variant == 0 ? 64 : 128;
+    constexpr int shape[kZtTileVariants][2] = {{64, 64}, {32, 128}, {16, 128}, {8, 32}};
+    bm = shape[variant][0];
+    bn = shape[variant][1];
 }
-void st_tile_shape(int& bm, int& bn) { bm = SBM; bn = SBN; }
+int zt_tile_rule(long long outputs, int rows) {
+    // below two 8 x 32 tiles per SM nothing but the spread over the SMs counts
+    if (outputs < 2 * 152 * 256) return 3;
+    return rows < 24 ? 2 : (rows < 48 ? 1 : 0);
+}
+int st_tile_variant(int columns) {
+    // the fewest padded columns, the widest tile of those
+    int best = 0;
+    for (int v = 1; v < 4; ++v) {
+        const int w = 16 >> v, wb = 16 >> best;
+        if ((columns + w - 1) / w * w < (columns + wb - 1) / wb * wb && (v < 3 || columns == 2)) best = v;
+    }
+    return best;
+}
+void st_tile_shape(int variant, int& bm, int& bn) {
+    bm = (variant == 0 || variant == 3) ? 128 : 64;
+    bn = 16 >> variant;
+}
 
 int launch_zt_leg_fwd(cudaStream_t s, const LegMeta& lm, const TileList& tl, const double* G, double* flm, int Lg,
                       int nlat, int nrad, int batch) {
@@ -405,12 +458,12 @@ int launch_zt_rad_bwd(cudaStream_t s, const RadMeta& rm, const TileList& tl, con
 int launch_st_leg_fwd(cudaStream_t s, const LegMeta& lm, const TileList& tl, const double* X, double* coeffs, int Lg,
                       int nlat, int batch, long long coeff_stride) {
     StLegFwd p{lm, X, coeffs, Lg, nlat, batch, coeff_stride};
-    return run<StLegFwd, SBM, SBN, STM, STN, SBK>(s, p, tl, "st_leg_fwd");
+    return run_st(s, p, tl, "st_leg_fwd");
 }
 int launch_st_leg_bwd(cudaStream_t s, const LegMeta& lm, const TileList& tl, const double* coeffs, double* X, int Lg,
                       int nlat, int batch, long long coeff_stride) {
     StLegBwd p{lm, coeffs, X, Lg, nlat, batch, coeff_stride};
-    return run<StLegBwd, SBM, SBN, STM, STN, SBK>(s, p, tl, "st_leg_bwd");
+    return run_st(s, p, tl, "st_leg_bwd");
 }
 
 }  // namespace zgpu

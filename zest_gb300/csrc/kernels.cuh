@@ -55,7 +55,7 @@ struct RadMeta {
 struct TileList {
     const int4* tiles = nullptr;    // {group, row0, col0, -}
     int count = 0;
-    int variant = 0;                // tile shape of the Zernike sums (zt_tile_shape)
+    int variant = 0;                // tile shape (zt_tile_shape, st_tile_shape)
 };
 
 // Zernike (G: [b][m][lat][rad][2], flm: [tri(l,m)][b][rad][2], coeffs: [b][zidx][2])
@@ -83,10 +83,14 @@ int launch_ev_st_leg(cudaStream_t s, const LegMeta& lm, const TileList& tl, cons
                      int nlat, int batch, long long coeff_stride);
 int launch_ev_lon(cudaStream_t s, const TileList& tl, const double* trig, const double* G, double* values, int L,
                   int nlon, int npts);
-// tile shapes (rows x cols per CTA) of the launches above
+// tile shapes (rows x cols per CTA) of the launches above; the shape for
+// groups of up to `rows` rows and `outputs` results in all where nothing was
+// timed (Zernike), and for a number of columns (SH)
+constexpr int kZtTileVariants = 4;
 void zt_tile_shape(int variant, int& bm, int& bn);
-constexpr int kZtTileVariants = 3;
-void st_tile_shape(int& bm, int& bn);
+int zt_tile_rule(long long outputs, int rows);
+int st_tile_variant(int columns);
+void st_tile_shape(int variant, int& bm, int& bn);
 
 // ---- rotations ------------------------------------------------------------------
 // Rotor::rotate on a batch of real expansions (in place).  kind 0 = Zernike,

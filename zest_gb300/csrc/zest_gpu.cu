@@ -224,13 +224,13 @@ static int get_st_plan(zest_gpu_context* ctx, int L, int sn, int sp, int layout,
 // kinds: 0 zt_leg_fwd, 1 zt_leg_bwd, 2 zt_rad_fwd, 3 zt_rad_bwd, 4 st_leg_fwd, 5 st_leg_bwd
 static int get_tiles(zest_gpu_context* ctx, int kind, int L, int Lm, int batch, int aux, TileList* tl,
                      int variant = 0) {
-    if (kind > 3) variant = 0;
+    if (kind > 3) variant = st_tile_variant(2 * batch);
     auto key = std::make_tuple(kind, L, Lm, batch, aux, variant);
     auto it = ctx->tiles.find(key);
     if (it == ctx->tiles.end()) {
         int bm, bn;
         if (kind <= 3) zt_tile_shape(variant, bm, bn);
-        else st_tile_shape(bm, bn);
+        else st_tile_shape(variant, bm, bn);
         std::vector<int4> v;
         auto add = [&](int g, long long M, long long N) {
             for (long long r = 0; r < M; r += bm)
@@ -286,7 +286,7 @@ static bool valid01(int x) { return x == 0 || x == 1; }
 // tile shape with CUDA events on the context stream (after one untimed run)
 // and keeps the fastest; the stages overwrite their outputs, so the extra runs
 // change nothing.  Without tuning, or while the stream is being captured, a
-// size rule picks the shape: small orders have few rows per group.
+// size rule picks the shape (zt_tile_rule): small orders have few rows per group.
 template <class Run>
 static int zt_tile_variant(zest_gpu_context* ctx, int kind, int L, int Lm, int batch, int aux, Run&& run,
                            int* variant) {
@@ -296,7 +296,8 @@ static int zt_tile_variant(zest_gpu_context* ctx, int kind, int L, int Lm, int b
         *variant = it->second;
         return ZEST_GPU_OK;
     }
-    *variant = Lm < 48 ? 2 : (Lm < 96 ? 1 : 0);
+    // (l, m) or (n, l) groups of up to Lm / 2 rows, about Lm^2 / 2 rows of batch * 2 nrad values
+    *variant = zt_tile_rule((long long)Lm * Lm * batch * L, Lm / 2);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     ZG_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &cap));
     if (!ctx->autotune || cap != cudaStreamCaptureStatusNone) return ZEST_GPU_OK;
