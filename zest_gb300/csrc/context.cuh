@@ -119,9 +119,10 @@ struct RaggedPlan {
     int zn = 0, sn = 0, sp = 0, type = 0, precision = 0, slices = 0;
     int Lmax = 0;
     long long nwork = 0;
-    DevBuf coff, work;                                         // per-item coefficient offsets, {item, n, l}
-    DevBuf vecl;                                               // the {item, n, l} vectors sorted by l
+    DevBuf coff;                                               // per-item coefficient offsets
+    DevBuf vecl;                                               // the {item, n, l, first pair} vectors sorted by l
     std::vector<long long> voff;                               // vecl rows of order l: [voff[l], voff[l+1])
+    DevBuf voff_dev;
     std::vector<long long> coff_h, goff_h;
     std::vector<std::tuple<int, int, int>> buckets;            // {order, first item, count}
     cudaGraph_t graph = nullptr;

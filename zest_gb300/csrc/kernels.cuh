@@ -95,25 +95,26 @@ void st_tile_shape(int variant, int& bm, int& bn);
 // ---- rotations ------------------------------------------------------------------
 // Rotor::rotate on a batch of real expansions (in place).  kind 0 = Zernike,
 // 1 = SH, 2 = SH rows of one parity in the row-skipping layout (a per-n
-// Zernike SH span); vec_list holds the nvec rotated (n, l) vectors of one
-// expansion.
-// phase_scratch: 6 * L * batch doubles.
+// Zernike SH span).  phase_scratch: 6 * L * batch doubles.
 int launch_rotate_vectors(cudaStream_t s, int kind, int L, int batch, double* coeffs, long long cstride,
-                          const int2* vec_list, int nvec, const double* wigner, const double* euler, int type,
-                          double* phase_scratch);
+                          const double* wigner, const double* euler, int type, double* phase_scratch);
+// Polar rotation of the nvec vectors (n, l) of vec_list of every expansion.
 int launch_polar_vectors(cudaStream_t s, int kind, int L, int batch, double* coeffs, long long cstride,
                          const int2* vec_list, int nvec, const double* angles, int type);
 // Gradient of <ybar, rotate(x, euler)> with respect to the Euler angles of each
-// batch item -> grad[3 * batch].  part: 3 * nvec * batch doubles of scratch.
+// batch item -> grad[3 * batch], and (xbar not null; it may be ybar) with
+// respect to x -> xbar.  nvec rotated vectors per expansion; part: 3 * nvec *
+// batch doubles of scratch.
 int launch_rotate_euler_grad(cudaStream_t s, int kind, int L, int batch, const double* x, const double* ybar,
-                             long long cstride, const int2* vec_list, int nvec, const double* wigner,
-                             const double* euler, int type, double* phase_scratch, double* part, double* grad);
-// Rotations of `items` expansions of different orders in one launch: work
-// entries {item, n, l, -}, item i's coefficients at coeffs + coff[i]; phase
-// scratch 6 * Lmax * items doubles.
-int launch_rotate_ragged(cudaStream_t s, int kind, int Lmax, int items, double* coeffs, const long long* coff,
-                         const int4* work, long long nwork, const double* wigner, const double* euler, int type,
-                         double* phase_scratch);
+                             long long cstride, int nvec, const double* wigner, const double* euler, int type,
+                             double* phase_scratch, double* part, double* grad, double* xbar);
+// Rotations of `items` Zernike expansions of different orders in one launch:
+// vecs = the {item, n, l, first pair} vectors sorted by l, those of degree l at
+// [voff[l], voff[l + 1]) (voff_dev: the same on the device), item i's
+// coefficients at coeffs + coff[i]; phase scratch 6 * Lmax * items doubles.
+int launch_rotate_ragged(cudaStream_t s, int Lmax, int items, double* coeffs, const long long* coff, const int4* vecs,
+                         const std::vector<long long>& voff, const long long* voff_dev, const double* wigner,
+                         const double* euler, int type, double* phase_scratch);
 // The phase tables e^{-i m angle} [item][alpha', beta', gamma'][m < Lmax] of a
 // ragged rotation (double2 entries in phase_scratch).
 int launch_phases(cudaStream_t s, int Lmax, int items, const double* euler, int type, double* phase_scratch);

@@ -2,17 +2,14 @@
 //
 // zest_gpu_zt_rotate_noalloc runs the kernels of zest_gpu_zt_rotate
 // (Rotor::rotate, include/rotor.hpp:214-243) on caller-owned device buffers.
-// The two scratch buffers that path keeps in the context -- the list of
-// rotated (n, l) vectors and the per-item phase tables e^{-i m angle} -- live
-// here in one fixed array compiled into the library's device image, so a call
-// makes no cudaMalloc, cudaFree or other allocating call.  The Wigner d(pi/2)
-// table is the caller's (zest_gpu_wignerd_table fills one).
+// The scratch that path keeps in the context -- the per-item phase tables
+// e^{-i m angle}, 3 tables of L double2 per batch item -- lives here in one
+// fixed array compiled into the library's device image, so a call makes no
+// cudaMalloc, cudaFree or other allocating call.  The Wigner d(pi/2) table is
+// the caller's (zest_gpu_wignerd_table fills one).  The sizes a call may have
+// count 8 bytes per rotated (n, l) vector beside the phases, room that a
+// list of them used to take.
 //
-// Layout of the array for a call of order L and batch B:
-//   [0, vec_bytes)            int2 vectors {n, l}, grouped by l, n ascending
-//                             (the order of the context path), vec_bytes =
-//                             8 * nvec(L) rounded up to 256
-//   [vec_bytes, + 48 L B)     phases, 3 tables of L double2 per batch item
 // Every byte a call reads is written earlier in the same call, so nothing in
 // the array has to start at zero.
 #include <cuda.h>
@@ -77,17 +74,6 @@ long long vec_total(int L) {
     long long t = 0;
     for (int l = 0; l < L; ++l) t += vec_count(L, l);
     return t;
-}
-
-// one thread per l writes its run of vectors at the run's offset
-__global__ void zt_vector_list_kernel(int L, int2* __restrict__ out) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= L) return;
-    long long off = 0;
-    for (int lp = 0; lp < l; ++lp) off += vec_count(L, lp);
-    const int n0 = l == 0 ? 2 : l;
-    const long long c = vec_count(L, l);
-    for (long long i = 0; i < c; ++i) out[off + i] = make_int2(n0 + 2 * int(i), l);
 }
 
 // Address of the array in the current device's current context.  The first
@@ -158,10 +144,6 @@ extern "C" int zest_gpu_zt_rotate_noalloc(void* stream, size_t order, size_t bat
         return fail(ZEST_GPU_ERR_INVALID, "Wigner d table of order " + std::to_string(wignerd_order) +
                                               " is smaller than the expansion order " + std::to_string(order));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int2* vecs = reinterpret_cast<int2*>(scratch);
-    double* phases = reinterpret_cast<double*>(scratch + vec_bytes);
-    zt_vector_list_kernel<<<(L + 127) / 128, 128, 0, s>>>(L, vecs);
-    ZG_TRY(launch_check("zt_vector_list_kernel"));
-    return launch_rotate_vectors(s, 0, L, B, coeffs, 2 * zsize(L), vecs, int(nvec), wignerd, euler, rotation_type,
-                                 phases);
+    return launch_rotate_vectors(s, 0, L, B, coeffs, 2 * zsize(L), wignerd, euler, rotation_type,
+                                 reinterpret_cast<double*>(scratch));
 }

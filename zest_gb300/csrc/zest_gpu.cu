@@ -604,13 +604,10 @@ int rotate_dev(zest_gpu_context* ctx, int kind, int L, int batch, double* coeffs
                                    coeffs, wig, euler, type, ctx->phase.as<double>()));
         return split_finish(ctx);
     }
-    const int2* vl;
-    int nvec;
-    ZG_TRY(get_vectors(ctx, kind, L, &vl, &nvec));
     ZG_TRY(ctx->phase.ensure((size_t)batch * 6 * L * sizeof(double)));
     const long long cstride = 2 * coeff_pairs(kind, L);
     StageScope sc(ctx, ST_ROTATE);
-    return launch_rotate_vectors(ctx->stream, kind, L, batch, coeffs, cstride, vl, nvec, wig, euler, type,
+    return launch_rotate_vectors(ctx->stream, kind, L, batch, coeffs, cstride, wig, euler, type,
                                  ctx->phase.as<double>());
 }
 
@@ -743,7 +740,9 @@ int rotate_vjp_dev(zest_gpu_context* ctx, int kind, int L, int batch, const doub
     if (batch == 0) return ZEST_GPU_OK;
     cudaStream_t s = ctx->stream;
     const long long cstride = kind == 0 ? 2 * zsize(L) : 2 * tri_size(L);
-    if (xbar) {
+    // the FP64 gradient kernel gives the coefficient cotangent on its way
+    const bool fused = xbar && ebar && L > 1 && ctx->precision != ZEST_PRECISION_SPLIT;
+    if (xbar && !fused) {
         ZG_CUDA_TRY(cudaMemcpyAsync(xbar, ybar, (size_t)batch * cstride * sizeof(double), cudaMemcpyDeviceToDevice, s));
         ZG_TRY(ctx->adj1.ensure((size_t)batch * 3 * sizeof(double)));
         ZG_TRY(launch_invert_euler(s, batch, euler, ctx->adj1.as<double>()));
@@ -762,8 +761,9 @@ int rotate_vjp_dev(zest_gpu_context* ctx, int kind, int L, int batch, const doub
         ZG_TRY(ctx->phase.ensure((size_t)batch * 6 * L * sizeof(double)));
         ZG_TRY(ctx->adj2.ensure((size_t)batch * nvec * 3 * sizeof(double) + 16));
         StageScope sc(ctx, ST_ROTATE);
-        ZG_TRY(launch_rotate_euler_grad(s, kind, L, batch, x, ybar, cstride, vl, nvec, wig, euler, type,
-                                        ctx->phase.as<double>(), ctx->adj2.as<double>(), ebar));
+        ZG_TRY(launch_rotate_euler_grad(s, kind, L, batch, x, ybar, cstride, nvec, wig, euler, type,
+                                        ctx->phase.as<double>(), ctx->adj2.as<double>(), ebar,
+                                        fused ? xbar : nullptr));
     }
     return ZEST_GPU_OK;
 }
@@ -786,8 +786,9 @@ static int ragged_sequence(zest_gpu_context* ctx, RaggedPlan& P, double* coeffs,
                                    coeffs, wig, euler, P.type, ctx->phase.as<double>()));
     } else {
         StageScope sc(ctx, ST_ROTATE);
-        ZG_TRY(launch_rotate_ragged(ctx->stream, 0, P.Lmax, int(P.orders.size()), coeffs, P.coff.as<long long>(),
-                                    P.work.as<int4>(), P.nwork, wig, euler, P.type, ctx->phase.as<double>()));
+        ZG_TRY(launch_rotate_ragged(ctx->stream, P.Lmax, int(P.orders.size()), coeffs, P.coff.as<long long>(),
+                                    P.vecl.as<int4>(), P.voff, P.voff_dev.as<long long>(), wig, euler, P.type,
+                                    ctx->phase.as<double>()));
     }
     for (const auto& bk : P.buckets) {
         const int L = std::get<0>(bk), first = std::get<1>(bk), count = std::get<2>(bk);
@@ -871,7 +872,6 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
     np->goff_h[n] = go;
     np->nwork = (long long)work.size();
     ZG_TRY(upload(np->coff, np->coff_h, ctx->stream));
-    ZG_TRY(upload(np->work, work, ctx->stream));
     {
         // the same vectors grouped by l (stable: item, then n, within a group)
         std::vector<int4> byl(work.size());
@@ -881,6 +881,7 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
         std::vector<long long> fill(np->voff.begin(), np->voff.end() - 1);
         for (const int4& w : work) byl[(size_t)fill[(size_t)w.z]++] = w;
         ZG_TRY(upload(np->vecl, byl, ctx->stream));
+        ZG_TRY(upload(np->voff_dev, np->voff, ctx->stream));
     }
     ZG_TRY(ctx->phase.ensure((size_t)n * 6 * std::max(np->Lmax, 1) * sizeof(double)));
     ctx->ragged = std::move(np);
