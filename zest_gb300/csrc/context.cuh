@@ -77,7 +77,7 @@ struct EvalBufs {
 
 struct FftEntry {
     FftPlan plan;
-    DevBuf tab, rows;
+    DevBuf tab, itab, rows;
 };
 
 // Folded Legendre tables (forward: weights * quadrature prefactor folded in;
@@ -209,6 +209,9 @@ struct zest_gpu_context {
 };
 
 namespace zgpu {
+// The plan of the longitude transforms of length N, cached (zest_gpu.cu).
+int get_fft(zest_gpu_context* ctx, int N, const FftPlan** out);
+
 // Brackets one pipeline stage with events when profiling is on.
 struct StageScope {
     zest_gpu_context* ctx;

@@ -485,6 +485,13 @@ int build_fft_plan(int N, FftPlan& plan, std::vector<double>& tab, std::vector<i
     };
     auto add_op = [&](FftOp op) {
         if (plan.nops == kFftMaxOps) return false;
+        auto rcp = [](long long d) { return d == 1 ? 0u : unsigned((1ll << 32) / d + 1); };
+        op.nr = op.R ? op.Nd / op.R : 1;
+        op.step = op.R ? op.nr / op.Ns : 0;
+        op.rcp_inner = rcp(op.inner);
+        op.rcp_nr = rcp(op.nr);
+        op.rcp_ns = rcp(op.Ns ? op.Ns : 1);
+        for (int k = 0; k < 4; ++k) op.rcp_nb[k] = rcp(((long long)op.outer * op.nr * op.inner) << k);
         plan.ops[plan.nops++] = op;
         return true;
     };

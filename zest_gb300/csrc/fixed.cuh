@@ -1,0 +1,55 @@
+// FP64 values to and from 64-bit fixed point by integer operations (the FP64 pipe
+// of GB300 retires one operation per 64 of the integer pipe).
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace zgpu {
+
+// 2^E T for a signed 64-bit T, rounded to nearest even, without FP64 operations
+// and without branches (so that independent elements interleave), in 32-bit
+// halves: |T| below 2^32 is moved
+// up by 32 bits first, so that one 32-bit leading-zero count and two funnel
+// shifts normalise it; the rounding carry runs into the exponent field through
+// the bit pattern; zero, results below the normal range and overflow are
+// selected at the end.
+__device__ __forceinline__ double i64_ldexp(long long T, int E) {
+    const unsigned long long sm = (unsigned long long)(T >> 63);  // all ones for T < 0
+    const unsigned long long a = ((unsigned long long)T ^ sm) - sm;
+    const bool small = (a >> 32) == 0;
+    const unsigned ah = small ? (unsigned)a : (unsigned)(a >> 32);
+    const unsigned al = small ? 0u : (unsigned)a;
+    const int lz = __clz(ah);                           // 32 only for T = 0
+    const unsigned nh = __funnelshift_l(al, ah, lz);    // leading one at bit 31
+    const unsigned nl = al << (lz & 31);
+    const unsigned mh = nh >> 11;                       // mantissa bits 52..32 (the leading one at bit 20)
+    const unsigned ml = __funnelshift_r(nl, nh, 11);    // mantissa bits 31..0
+    const unsigned inc = ((nl & 0x7FFu) + (ml & 1u) + 0x3FFu) >> 11;  // round half to even
+    const int e = E + 1023 + 63 - (small ? 32 : 0) - lz;  // exponent field of the leading one
+    const unsigned lo = ml + inc;
+    const unsigned mc = mh + (lo < ml ? 1u : 0u);
+    const int eff = e + int(mc >> 21);                  // after a rounding carry
+    const unsigned hi = (eff >= 2047 ? 0x7FF00000u : ((unsigned)(e - 1) << 20) + mc) |
+                        ((unsigned)(sm >> 32) & 0x80000000u);
+    const double v = __hiloint2double((int)hi, eff >= 2047 ? 0 : (int)lo);
+    return (a == 0 || eff <= 0) ? 0.0 : v;
+}
+
+// fixed point: round(x 2^{nbits-e}) as int64 (|x| < 2^(e-1)), ties away from
+// zero, with Cr = 1074 + e - nbits.  q = |x| 2^{nbits-e+1} truncated (one bit
+// more than kept), then ((q ^ s) + 1) >> 1 with s the sign mask is
+// floor(q/2 + 1/2) for x >= 0 and its negative for x < 0.  The shift
+// Cr - E(x) is at least 5 for every element of a row (the row exponent keeps
+// a bit of headroom); PTX shifts of 64 or more give 0, so a zero or an element
+// far below the row's largest rounds to 0 without a branch.
+__device__ __forceinline__ long long to_fixed_c(double x, int Cr) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+    const unsigned E = unsigned(bits >> 52) & 0x7FFu;
+    const unsigned long long M = (bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+    unsigned long long q;
+    asm("shr.b64 %0, %1, %2;" : "=l"(q) : "l"(M), "r"(unsigned(Cr) - E));
+    const long long sg = (long long)bits >> 63;  // 0 or -1
+    return (((long long)q ^ sg) + 1) >> 1;
+}
+
+}  // namespace zgpu

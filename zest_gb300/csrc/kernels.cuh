@@ -15,6 +15,10 @@ namespace zgpu {
 // the middle of a Rader dimension.  tab: its roots in the plan's table.
 struct FftOp {
     int R, Nd, Ns, base, outer, ostride, inner, tab;
+    // derived: Nd / R, Nd / (Ns R), and reciprocals (2^32 / d rounded up, 0 for d = 1)
+    // of inner, Nd / R, Ns and of the butterflies for 1, 2, 4 and 8 column pairs
+    int nr, step;
+    unsigned rcp_inner, rcp_nr, rcp_ns, rcp_nb[4];
 };
 constexpr int kFftMaxOps = 40;
 struct FftPlan {
@@ -23,6 +27,7 @@ struct FftPlan {
     int ntab = 0;  // complex entries of the table
     FftOp ops[kFftMaxOps] = {};
     const double2* tab = nullptr;    // device: roots of unity and Rader products
+    const int4* itab = nullptr;      // device: the same in fixed point (fixed_fft.cu)
     const int* in_row = nullptr;     // device: row of input index i, i < N
     const int* out_row = nullptr;    // device: row of output index k, k < N
 };
@@ -37,6 +42,19 @@ int launch_rfft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, long l
 // inverse (Hermitian, factor 1): F as above -> x
 int launch_rfft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int batch, int lon_fast,
                     double* x, long long xb, long long si, long long sc);
+
+// The same transforms in 64-bit fixed point (fixed_fft.cu): F holds ms orders per
+// item, of which m < nm are written or read (the others count as zero).  The
+// parity form reads the sums E_p[b][m][j'][rad][2] of folded Legendre sums,
+// E_0 +- E_1 at the nodes j0u + j' and j0d - j'.
+void fixed_fft_table(const std::vector<double>& tab, std::vector<int4>& itab);
+int launch_fixed_fft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, long long xb, long long si,
+                         long long sc, int C, int nm, int ms, int batch, int lon_fast, double* F);
+int launch_fixed_fft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int ms, int batch,
+                         int lon_fast, double* x, long long xb, long long si, long long sc);
+int launch_fixed_fft_inv_parity(cudaStream_t s, const FftPlan& plan, const double* E, int nlat, int nrad, int kh,
+                                int j0u, int j0d, int nm, int ms, int batch, int lon_fast, double* x, long long xb,
+                                long long si, long long sc);
 
 // ---- grouped FP64 contractions ------------------------------------------------
 // Per-call metadata of the folded Legendre / radial stages, all device pointers.

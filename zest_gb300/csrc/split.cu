@@ -1,9 +1,10 @@
 // Split-precision form of the GLQ contractions on tcgen05 tensor cores: every
 // Zernike contraction and the SH Legendre sums.
 //
-// Every dense contraction -- the longitude DFT of the Zernike path (as a
-// matrix product with the cos/sin table, folded over x_i +- x_{N-i}), the
-// folded Legendre sums and the radial sums -- is evaluated as
+// Every dense contraction -- the longitude DFT of the Zernike path up to order
+// 256 (as a matrix product with the cos/sin table, folded over x_i +- x_{N-i};
+// longer ones and the SH transforms take the FFT of fixed_fft.cu), the folded
+// Legendre sums and the radial sums -- is evaluated as
 //     C[r, n] = sum_k A[r, k] B[n, k]
 // with FP64 operands represented in BF16 fixed-point slices:
 //   * each operand row gets an exponent e (|x| < 2^(e-1) over the row) and
@@ -51,6 +52,7 @@
 
 #include "common.cuh"
 #include "context.cuh"
+#include "fixed.cuh"
 #include "split.cuh"
 
 namespace zgpu {
@@ -192,57 +194,6 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
            | ((uint32_t)(M >> 4) << 24);   // M / 16
 }
 
-// (-1)^neg 2^E a for a 64-bit magnitude a, assembled with integer operations
-// (round to nearest even to 53 bits; results below the normal range flush to 0).
-__device__ __forceinline__ double u64_ldexp(unsigned long long a, bool neg, int E) {
-    if (a == 0) return 0.0;
-    const unsigned long long sgn = neg ? (1ull << 63) : 0ull;
-    int lz = __clzll((long long)a);
-    unsigned long long n = a << lz;
-    unsigned long long mant = n >> 11;
-    const unsigned long long rest = n & 0x7FFull;
-    if (rest > 0x400ull || (rest == 0x400ull && (mant & 1ull))) {
-        ++mant;
-        if (mant >> 53) {
-            mant >>= 1;
-            --lz;
-        }
-    }
-    const int biased = (63 - lz) + E + 1023;
-    if (biased <= 0) return 0.0;
-    if (biased >= 2047) return __longlong_as_double((long long)(sgn | 0x7FF0000000000000ull));
-    return __longlong_as_double((long long)(sgn | ((unsigned long long)biased << 52) | (mant & 0xFFFFFFFFFFFFFull)));
-}
-
-
-// The same for a signed 64-bit T, without branches (so that the epilogue's
-// independent elements interleave), in 32-bit halves: |T| below 2^32 is moved
-// up by 32 bits first, so that one 32-bit leading-zero count and two funnel
-// shifts normalise it; the rounding carry runs into the exponent field through
-// the bit pattern; zero, results below the normal range and overflow are
-// selected at the end.  Bit-identical to u64_ldexp.
-__device__ __forceinline__ double i64_ldexp(long long T, int E) {
-    const unsigned long long sm = (unsigned long long)(T >> 63);  // all ones for T < 0
-    const unsigned long long a = ((unsigned long long)T ^ sm) - sm;
-    const bool small = (a >> 32) == 0;
-    const unsigned ah = small ? (unsigned)a : (unsigned)(a >> 32);
-    const unsigned al = small ? 0u : (unsigned)a;
-    const int lz = __clz(ah);                           // 32 only for T = 0
-    const unsigned nh = __funnelshift_l(al, ah, lz);    // leading one at bit 31
-    const unsigned nl = al << (lz & 31);
-    const unsigned mh = nh >> 11;                       // mantissa bits 52..32 (the leading one at bit 20)
-    const unsigned ml = __funnelshift_r(nl, nh, 11);    // mantissa bits 31..0
-    const unsigned inc = ((nl & 0x7FFu) + (ml & 1u) + 0x3FFu) >> 11;  // round half to even
-    const int e = E + 1023 + 63 - (small ? 32 : 0) - lz;  // exponent field of the leading one
-    const unsigned lo = ml + inc;
-    const unsigned mc = mh + (lo < ml ? 1u : 0u);
-    const int eff = e + int(mc >> 21);                  // after a rounding carry
-    const unsigned hi = (eff >= 2047 ? 0x7FF00000u : ((unsigned)(e - 1) << 20) + mc) |
-                        ((unsigned)(sm >> 32) & 0x80000000u);
-    const double v = __hiloint2double((int)hi, eff >= 2047 ? 0 : (int)lo);
-    return (a == 0 || eff <= 0) ? 0.0 : v;
-}
-
 }  // namespace
 
 // ===========================================================================
@@ -252,7 +203,7 @@ namespace {
 
 constexpr int SL_KMAX = 2048;  // longest operand row the slicing stages (and longest sum)
 constexpr int SL_K8MAX = 256;  // K bound of exact level sums with balanced 8-bit digits
-constexpr int SL_UNROLL = 8;   // independent loads per thread in the staging loops (halved for 4 inputs)
+constexpr int SL_UNROLL = 8;   // independent loads per thread in the staging loops
 
 // Digits are 8 bits wide at any length: sums longer than SL_K8MAX terms run
 // as K-chunks of at most SL_K8MAX whose FP64 results are added.
@@ -292,7 +243,7 @@ inline int slice_rows_per_block(int row_bytes) {
     return r;
 }
 
-enum { SL_ONE = 0, SL_FOLD = 1, SL_PAIR = 2, SL_PFOLD = 3 };
+enum { SL_ONE = 0, SL_FOLD = 1, SL_PAIR = 2 };
 
 // Loaders give the pair (up, dn) of operand element (row, k) through a per-row
 // handle computed once per block row.  ROW_FAST loaders read consecutive rows
@@ -482,38 +433,6 @@ struct StLegBwdLoader {
 };
 
 // rows (b, col = (lat, rad)); k = m: the spectrum (Re F_m, Im F_m) at
-// latitude lat (the sin operand takes Im F_k at k - 1), formed from the two
-// parity sums E_p[b][m][j'][2 rad + {re, im}] of the Legendre stage: E_0 + E_1
-// at the north node lat = j0u + j', E_0 - E_1 at the south node lat = j0d - j'
-// (the equator, j0u = j0d, is north).  The sums are formed exactly in
-// integers by the slicing (SL_PFOLD): the loader gives (Re E_0, Im E_0,
-// Re E_1, Im E_1), E_1 negated for a south row by a sign-bit flip.
-struct DftBwdLoader {
-    static constexpr bool ROW_FAST = true, TWO = true;
-    static constexpr int MODE = SL_PFOLD, SHIFT = 1;
-    const double* E;
-    int L, C, nrad, kh, j0u, j0d, B;
-    struct Row { const double* e0; int neg; };  // neg: the sign bit of E_1's high word
-    __device__ Row row(long long r) const {
-        const long long b = r / C;
-        const int col = int(r - b * C);
-        const int lat = col / nrad, rad = col - lat * nrad;
-        const bool north = lat >= j0u;
-        const int jf = north ? lat - j0u : j0d - lat;
-        return Row{E + ((b * L) * kh + jf) * (2LL * nrad) + 2 * rad, north ? 0 : int(0x80000000u)};
-    }
-    __device__ void get4(const Row& R, int k, double* v) const {
-        const long long mo = (long long)k * kh * 2 * nrad;
-        const double2 a = *reinterpret_cast<const double2*>(R.e0 + mo);
-        const double2 c = *reinterpret_cast<const double2*>(R.e0 + mo + (long long)B * L * kh * 2 * nrad);
-        v[0] = a.x;
-        v[1] = a.y;
-        v[2] = __hiloint2double(__double2hiint(c.x) ^ R.neg, __double2loint(c.x));
-        v[3] = __hiloint2double(__double2hiint(c.y) ^ R.neg, __double2loint(c.y));
-    }
-};
-
-// rows (b, col = (lat, rad)); k = m: the spectrum (Re F_m, Im F_m) at
 // latitude lat, E[b][m][lat][2 rad + {re, im}] of the unfolded backward
 // Legendre sums (the sin operand takes Im F_k at k - 1)
 struct DftBwdGridLoader {
@@ -536,9 +455,8 @@ struct DftBwdGridLoader {
 };
 
 // One slicing job: one operand array (SL_ONE) or two from one read of the
-// input (SL_FOLD: up + dn and up - dn; SL_PAIR: up and dn; SL_PFOLD: the
-// sums of two pairs), the second at index k - shift.  Both share the row
-// exponents.  Each loader fixes its mode and shift (Loader::MODE,
+// input (SL_FOLD: up + dn and up - dn; SL_PAIR: up and dn), the second at index
+// k - shift.  Both share the row exponents.  Each loader fixes its mode and shift (Loader::MODE,
 // Loader::SHIFT), so the kernel is specialised.
 struct SliceJob {
     long long rows;
@@ -555,10 +473,10 @@ struct SliceJob {
     int* ex1;
 };
 
-// Staged inputs per operand row: 1 (SL_ONE), 2 (SL_FOLD, SL_PAIR) or 4 (SL_PFOLD).
+// Staged inputs per operand row: 1 (SL_ONE) or 2 (SL_FOLD, SL_PAIR).
 template <class Loader>
 __host__ __device__ constexpr int staged_arrays() {
-    return Loader::MODE == SL_ONE ? 1 : (Loader::MODE == SL_PFOLD ? 4 : 2);
+    return Loader::MODE == SL_ONE ? 1 : 2;
 }
 
 // Ragged loaders (a member kvalid(row): the row's inputs are zero from that k
@@ -584,23 +502,6 @@ __device__ __forceinline__ int sl_pos(int k) { return k + (k >> 3); }
 inline int sl_row_stride(int KS) {
     const int p = KS + (KS >> 3) + 1;
     return p + ((6 - p % 4) % 4);
-}
-
-// fixed point: round(x 2^{nbits-e}) as int64 (|x| < 2^(e-1)), ties away from
-// zero, with Cr = 1074 + e - nbits.  q = |x| 2^{nbits-e+1} truncated (one bit
-// more than kept), then ((q ^ s) + 1) >> 1 with s the sign mask is
-// floor(q/2 + 1/2) for x >= 0 and its negative for x < 0.  The shift
-// Cr - E(x) is at least 5 for every element of a row (the row exponent keeps
-// a bit of headroom); PTX shifts of 64 or more give 0, so a zero or an element
-// far below the row's largest rounds to 0 without a branch.
-__device__ __forceinline__ long long to_fixed_c(double x, int Cr) {
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
-    const unsigned E = unsigned(bits >> 52) & 0x7FFu;
-    const unsigned long long M = (bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    unsigned long long q;
-    asm("shr.b64 %0, %1, %2;" : "=l"(q) : "l"(M), "r"(unsigned(Cr) - E));
-    const long long sg = (long long)bits >> 63;  // 0 or -1
-    return (((long long)q ^ sg) + 1) >> 1;
 }
 
 // Balanced 8-bit digits of 8 neighbouring elements (slice 0 most
@@ -647,13 +548,9 @@ __device__ __forceinline__ void store_digits8(const long long (&w)[8], __nv_bflo
 
 template <class Loader>
 __device__ __forceinline__ void load_staged(const Loader& ld, const typename Loader::Row& R, int k, double* v) {
-    if constexpr (Loader::MODE == SL_PFOLD) {
-        ld.get4(R, k, v);
-    } else {
-        double dn = 0.0;
-        ld.get(R, k, v[0], dn);
-        if constexpr (Loader::TWO) v[1] = dn;
-    }
+    double dn = 0.0;
+    ld.get(R, k, v[0], dn);
+    if constexpr (Loader::TWO) v[1] = dn;
 }
 
 // One CTA converts R rows (R a power of two, <= 32) of staged values.
@@ -669,8 +566,8 @@ __device__ __forceinline__ void load_staged(const Loader& ld, const typename Loa
 template <class Loader, int S>
 __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
     constexpr int MODE = Loader::MODE, SHIFT = Loader::SHIFT, NA = staged_arrays<Loader>();
-    constexpr int fold_bit = (MODE == SL_FOLD || MODE == SL_PFOLD) ? 1 : 0;
-    constexpr int UNR = NA == 4 ? SL_UNROLL / 2 : SL_UNROLL;  // loads in flight per thread and input
+    constexpr int fold_bit = MODE == SL_FOLD ? 1 : 0;
+    constexpr int UNR = SL_UNROLL;  // loads in flight per thread and input
     static_assert((NA > 1) == Loader::TWO && (SHIFT == 0 || (NA > 1 && SHIFT == 1)), "loader mode");
     extern __shared__ double sl_smem[];
     constexpr bool RAGGED = ragged_loader<Loader>::value;
@@ -805,22 +702,16 @@ __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
                     store_digits8<S>(w, J.out1 + row * J.Kp1 + 8 * c, J.stride1);
                 }
             } else {
-                // SL_PAIR: up | dn; SL_PFOLD: up + up2 | dn + dn2 (inputs 0, 2 | 1, 3)
+                // SL_PAIR: up | dn
                 long long w[8];
                 if (c < nch0) {
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        w[q] = to_fixed_c(at(0, q), Cr);
-                        if constexpr (MODE == SL_PFOLD) w[q] += to_fixed_c(at(2, q), Cr);
-                    }
+                    for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(0, q), Cr);
                     store_digits8<S>(w, J.out0 + row * J.Kp0 + 8 * c, J.stride0);
                 }
                 if (c < nch1) {
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        w[q] = to_fixed_c(at(1, q + SHIFT), Cr);
-                        if constexpr (MODE == SL_PFOLD) w[q] += to_fixed_c(at(3, q + SHIFT), Cr);
-                    }
+                    for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(1, q + SHIFT), Cr);
                     store_digits8<S>(w, J.out1 + row * J.Kp1 + 8 * c, J.stride1);
                 }
             }
@@ -872,10 +763,9 @@ struct EpiDense {  // C[row][b_row0 + n] (utility GEMM)
         R.p[n] = ACC ? old[0] + v : v;
     }
 };
-template <bool ACC = false>
 struct EpiDftFwd {  // rows (b, col): conj X_m -> G[b][m][col][re, im]
-    static constexpr bool RMW = ACC;
-    static constexpr bool CHUNK = ACC;
+    static constexpr bool RMW = false;
+    static constexpr bool CHUNK = false;
     double* G;
     int C, L;
     struct Row { double* p; };  // &G[b][m0][col][re or im]
@@ -885,11 +775,11 @@ struct EpiDftFwd {  // rows (b, col): conj X_m -> G[b][m][col][re, im]
         const int m0 = u.aux + sin;
         return Row{G + (((long long)b * L + m0) * C + col) * 2 + sin};
     }
-    __device__ void load(const Row& R, int n, double* old) const { old[0] = R.p[(long long)n * C * 2]; }
-    __device__ void store(const Row& R, const SplitUnit& u, int n, double v, const double* old) const {
+    __device__ void load(const Row&, int, double*) const {}
+    __device__ void store(const Row& R, const SplitUnit& u, int n, double v, const double*) const {
         double* g = R.p + (long long)n * C * 2;
-        g[0] = ACC ? old[0] + v : v;
-        if (!ACC && ((u.flags >> 1) & 1) == 0 && u.aux + n == 0) g[1] = 0.0;  // Im X_0 = 0
+        g[0] = v;
+        if (((u.flags >> 1) & 1) == 0 && u.aux + n == 0) g[1] = 0.0;  // Im X_0 = 0
     }
 };
 template <bool ACC = false>
@@ -1032,14 +922,13 @@ struct EpiStLegFwd {
 };
 // Backward: table row r of group (m, p) is folded node j = r - (2m + p) kh;
 // the parity sums go to E[p][b][m][j][c], the imaginary parts with the sign bit
-// flipped (flip_im: conjugated, as the inverse longitude DFT reads them).
+// flipped (conjugated, as the inverse longitude transform reads them).
 template <bool ACC>
 struct EpiStLegBwdE {
     static constexpr bool RMW = ACC;
     static constexpr bool CHUNK = ACC;
     double* E;
     int B, L, kh;
-    unsigned long long flip_im;  // 1 << 63: the imaginary parts conjugated (a sign-bit flip), else 0
     struct Row { double* p; };
     __device__ Row row(const SplitUnit& u, int r) const {
         const int m = u.g, par = (u.flags >> 2) & 1;
@@ -1050,73 +939,19 @@ struct EpiStLegBwdE {
         old[0] = R.p[(long long)(n >> 1) * L * kh * 2 + (n & 1)];
     }
     __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double* old) const {
-        const double w = __longlong_as_double(__double_as_longlong(v) ^ (long long)((n & 1) ? flip_im : 0ull));
+        const double w = __longlong_as_double(__double_as_longlong(v) ^ (long long)((n & 1) ? 1ull << 63 : 0ull));
         R.p[(long long)(n >> 1) * L * kh * 2 + (n & 1)] = ACC ? old[0] + w : w;
     }
 };
 
-// Inverse DFT, rows (b, col).  The cos pass writes x_0 = C_0 to the grid and
-// C_i (i >= 1) to the scratch Cs[b][i][col]; the sin pass reads C_i once and
-// writes x_i = C_i + S_i and x_{N-i} = C_i - S_i.
-template <bool ACC = false>
-struct EpiDftBwdCos {
-    static constexpr bool RMW = ACC;
-    static constexpr bool CHUNK = ACC;
-    double* grid;
-    double* Cs;
-    int C, N, L;
-    long long gsz;
-    struct Row { double* x; double* c; int aux; };
-    __device__ Row row(const SplitUnit& u, int r) const {
-        const long long b = r / C, col = r - b * C;
-        return Row{grid + b * gsz + col, Cs + (b * L + u.aux) * C + col, u.aux};
-    }
-    __device__ double* at(const Row& R, int n) const { return R.aux + n == 0 ? R.x : R.c + (long long)n * C; }
-    __device__ void load(const Row& R, int n, double* old) const { old[0] = *at(R, n); }
-    __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double* old) const {
-        *at(R, n) = ACC ? old[0] + v : v;
-    }
-};
-// The first chunk reads the finished cos sums C_i and writes x_i = C_i + S_i,
-// x_{N-i} = C_i - S_i; later chunks add their S_i to x_i and subtract it from x_{N-i}.
-template <bool ACC = false>
-struct EpiDftBwdSin {
-    static constexpr bool RMW = true;
-    static constexpr bool CHUNK = ACC;
-    double* grid;
-    const double* Cs;
-    int C, N, L;
-    long long gsz;
-    struct Row { double* x; const double* c; int i0; };
-    __device__ Row row(const SplitUnit& u, int r) const {
-        const long long b = r / C, col = r - b * C;
-        return Row{grid + b * gsz + col, Cs + (b * L + u.aux + 1) * C + col, u.aux + 1};
-    }
-    __device__ void load(const Row& R, int n, double* old) const {
-        if (ACC) {
-            const int i = R.i0 + n;
-            old[0] = R.x[(long long)i * C];
-            old[1] = R.x[(long long)(N - i) * C];
-        } else {
-            old[0] = old[1] = R.c[(long long)n * C];
-        }
-    }
-    __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double* old) const {
-        const int i = R.i0 + n;
-        R.x[(long long)i * C] = old[0] + v;
-        R.x[(long long)(N - i) * C] = old[1] - v;
-    }
-};
-
-// The same inverse DFT for sums of at most 256 terms, combined in integers:
-// the cos and sin tables are sliced together, so that row i of both shares
-// one exponent, and the data operands share theirs (one slicing job), so
-// C_i and S_i are exact integers T_c, T_s on the same scale 2^e.  The cos
-// pass writes x_0 = C_0 and the raw T_c (int64) of i >= 1 to the scratch; the
-// sin pass forms x_i = 2^e (T_c + T_s) and x_{N-i} = 2^e (T_c - T_s) exactly
-// before one rounding each, with integer operations only (no FP64 adds).
-// The table digits are at most 64 in magnitude (|2 cos|, |2 sin| <= 2), so
-// |T| < 2^61 and the sums cannot overflow.
+// Inverse DFT, rows (b, col), combined in integers: the cos and sin tables are
+// sliced together, so that row i of both shares one exponent, and the data
+// operands share theirs (one slicing job), so C_i and S_i are exact integers T_c,
+// T_s on the same scale 2^e.  The cos pass writes x_0 = C_0 and the raw T_c
+// (int64) of i >= 1 to the scratch; the sin pass forms x_i = 2^e (T_c + T_s) and
+// x_{N-i} = 2^e (T_c - T_s) exactly before one rounding each, with integer
+// operations only (no FP64 adds).  The table digits are at most 64 in magnitude
+// (|2 cos|, |2 sin| <= 2), so |T| < 2^61 and the sums cannot overflow.
 // Epilogues whose rows 2i and 2i + 1 are the two halves of one 16-byte pair
 // at each column (PAIR_ROWS; store_pair writes both)
 template <class E, class = void>
@@ -1631,17 +1466,14 @@ struct SliceArray {
 // Sliced tables of one Zernike plan for one slice count.
 // work-list keys: (stage, Lg, Lm, batch, S, pass)
 enum {
-    WK_DFT_F = 0, WK_LEG_F, WK_RAD_F, WK_RAD_B, WK_LEG_B, WK_DFT_B, WK_DENSE, WK_ST_LEG_F, WK_ST_LEG_B,
-    WK_ST_DFT_F, WK_ST_DFT_B, WK_ROT
+    WK_DFT_F = 0, WK_LEG_F, WK_RAD_F, WK_RAD_B, WK_LEG_B, WK_DFT_B, WK_DENSE, WK_ST_LEG_F, WK_ST_LEG_B, WK_ROT
 };
 
-// Sliced longitude DFT tables of one (order L, longitude count N): shared by
-// the Zernike grids and the SH LonLat grids of the same order.
+// Sliced longitude DFT tables of one (order L <= 256, longitude count N); the
+// inverse tables are sliced together: row i of both (sin row 0 = 0) shares one
+// exponent, the sin slices hold m >= 1 at m - 1.
 struct DftTables {
-    SliceArray cos_f, sin_f, cos_b, sin_b;
-    // the inverse tables sliced together (orders up to 256): row i of both
-    // (sin row 0 = 0) shares one exponent; the sin slices hold m >= 1 at m - 1
-    SliceArray cos_bj, sin_bj;
+    SliceArray cos_f, sin_f, cos_bj, sin_bj;
 };
 
 // Sliced tables of the two X(+-pi/2) products of a rotation, all l < Lmax:
@@ -1652,7 +1484,7 @@ struct RotTables {
 
 struct ZtSplitTables {
     int S = 0;
-    const DftTables* dft = nullptr;
+    const DftTables* dft = nullptr;  // orders up to 256
     SliceArray leg_f, rad_f, rad_bT, leg_bT;
     // orders up to 256: the backward Legendre table at every latitude node,
     // rows (m, lat), K = l - m (no fold over the equator)
@@ -1784,9 +1616,8 @@ int launch_slice(cudaStream_t s, const Loader& ld, long long rows, int K, int S,
     return run_slice(s, ld, J);
 }
 
-// Two operand arrays from one read: SL_FOLD (up + dn, up - dn), SL_PAIR
-// (up, dn) or SL_PFOLD (up + up2, dn + dn2); the second holds k in
-// [shift, shift + K1) at k - shift.  A fold needs K0 = K1 + shift (both sums
+// Two operand arrays from one read: SL_FOLD (up + dn, up - dn) or SL_PAIR (up,
+// dn); the second holds k in [shift, shift + K1) at k - shift.  A fold needs K0 = K1 + shift (both sums
 // end at the same input).
 template <class Loader>
 int launch_slice2(cudaStream_t s, const Loader& ld, long long rows, int K0, int K1, int shift, int S, int bits,
@@ -1835,10 +1666,10 @@ int get_state(zest_gpu_context* ctx, SplitState** out) {
             }
         }
         // tuning override of the column tiles, "stage=nt,..." with stage one of
-        // dft_f leg_f rad_f rad_b leg_b dft_b st_dft_f st_dft_b and nt 32 or 80
+        // dft_f leg_f rad_f rad_b leg_b dft_b and nt 32 or 80
         if (const char* e = std::getenv("ZEST_GPU_SPLIT_NT")) {
             static const char* names[] = {"dft_f", "leg_f", "rad_f", "rad_b", "leg_b", "dft_b", "dense",
-                                          "st_leg_f", "st_leg_b", "st_dft_f", "st_dft_b"};
+                                          "st_leg_f", "st_leg_b"};
             std::string spec(e);
             size_t pos = 0;
             while (pos < spec.size()) {
@@ -1863,29 +1694,6 @@ int get_state(zest_gpu_context* ctx, SplitState** out) {
     }
     *out = ctx->split.get();
     return ZEST_GPU_OK;
-}
-
-// SH backward: the parity sums E[p][b][m][j][c] (groups with no degree below Lm
-// read as 0) unfolded to X[b][m][lat][c], conjugated as the reference's sum_l
-// writes them: north lat = j0u + j gets E_0 + E_1, south lat = j0d - j gets
-// E_0 - E_1 (the equator of an odd grid, j0u = j0d, where E_1 = 0, is written
-// twice with the same value).
-__global__ void st_unfold_kernel(const double* __restrict__ E, double* __restrict__ X, int B, int L, int Lm, int kh,
-                                 int nlat, int j0u, int j0d) {
-    const long long n = (long long)B * L * kh * 2;
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const int c = int(t & 1);
-    const long long q = t >> 1;
-    const int j = int(q % kh);
-    const long long bm = q / kh;
-    const int m = int(bm % L), b = int(bm / L);
-    const double e0 = (Lm - m > 0) ? E[(((long long)b * L + m) * kh + j) * 2 + c] : 0.0;
-    const double e1 = (Lm - m - 1 > 0) ? E[((((long long)B + b) * L + m) * kh + j) * 2 + c] : 0.0;
-    const double sg = c ? -1.0 : 1.0;
-    double* x = X + (((long long)b * L + m) * nlat) * 2 + c;
-    x[(long long)(j0u + j) * 2] = sg * (e0 + e1);
-    x[(long long)(j0d - j) * 2] = sg * (e0 - e1);
 }
 
 // FP64 table generators
@@ -1970,12 +1778,8 @@ int build_dft_tables(zest_gpu_context* ctx, SplitState* st, int L, int N, int S,
     };
     // forward: cos rows m in [0,L), cols i in [0,L); sin rows m in [1,L), cols i in [1,L)
     ZG_TRY(gen(L, L, 0, 0, 0, t->cos_f));
-    if (L > 1) ZG_TRY(gen(L - 1, L - 1, 1, 1, 1, t->sin_f));
-    // backward: cos rows i in [0,L), cols m in [0,L); sin rows i in [1,L), cols m in [1,L)
-    // (K-chunked sums, orders above 256; single sums use the joint tables below)
-    if (L > KCHUNK || L == 1) ZG_TRY(gen(L, L, 0, 0, 2, t->cos_b));
-    if (L > KCHUNK) ZG_TRY(gen(L - 1, L - 1, 1, 1, 3, t->sin_b));
-    if (L > 1 && L <= KCHUNK) {
+    ZG_TRY(gen(L - 1, L - 1, 1, 1, 1, t->sin_f));
+    {
         // both inverse tables over all rows i and m, sliced in one job with shared row
         // exponents (the earlier tables' slicing jobs are queued before these writes)
         ZG_CUDA_TRY(cudaStreamSynchronize(s));
@@ -2007,7 +1811,7 @@ int build_zt_tables(zest_gpu_context* ctx, SplitState* st, ZtPlan& plan, int S, 
     auto t = std::make_unique<ZtSplitTables>();
     t->S = S;
     const int L = int(plan.sh.L), N = int(plan.sh.nlon), nr = int(plan.sh.nrad), kh = plan.leg.nnodes;
-    ZG_TRY(build_dft_tables(ctx, st, L, N, S, &t->dft));
+    if (L <= KCHUNK) ZG_TRY(build_dft_tables(ctx, st, L, N, S, &t->dft));
     // forward Legendre and radial tables (FP64 tables of the plain form)
     ZG_TRY(slice_table(ctx, plan.leg.Pf.as<double>(), plan.leg.off_h[2 * (size_t)L], kh, kh, S, digit_bits(kh),
                        t->leg_f));
@@ -2308,11 +2112,11 @@ int tuned_stage(zest_gpu_context* ctx, SplitState* st, int wk, int S, int Lg, in
     return run(choice & 0xFF, choice >> 8);
 }
 
-// Longitude DFT of `batch` grids x[b][lon][col] (C columns, item stride gsz)
-// to the spectra G[b][m][col][re, im], m < Lm (L = Lg orders per item):
-// folded cos/sin products (x_k + x_{N-k} against cos, x_k - x_{N-k} against
-// sin), K-chunked.  `wk` keys the work lists of the caller's grid family.
-int dft_forward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t, int S, int wk, const double* grids,
+// Longitude DFT of `batch` grids x[b][lon][col] (C columns, item stride gsz) of
+// order Lg <= 256 to the spectra G[b][m][col][re, im], m < Lm (Lg orders per
+// item): folded cos/sin products (x_k + x_{N-k} against cos, x_k - x_{N-k}
+// against sin).
+int dft_forward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t, int S, const double* grids,
                       long long gsz, int C, int N, int Lg, int Lm, int batch, double* G) {
     const int bits = digit_bits(Lg);
     const long long rows = (long long)batch * C;
@@ -2323,52 +2127,27 @@ int dft_forward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t,
         ZG_TRY(launch_slice2(ctx->stream, DftFwdLoader{grids, gsz, C, N}, rows, Lg, Lg - 1, 1, S, bits, SL_FOLD,
                              st->op[0], st->op[1]));
     }
-    return tuned_stage(ctx, st, wk, S, Lg, Lm, batch, Lm, nchunks(Lg) == 1, [&](int NT) -> int {
-        for (int ch = 0; ch < nchunks(Lg); ++ch) {
-            const int k0 = ch * KCHUNK;
-            UnitList* u;
-            ZG_TRY(get_units(ctx, std::make_tuple(wk, Lg, Lm, batch, S, 8 * ch + nt_pass(NT)), [&](UnitList& ul) {
-                for (long long r = 0; r < rows; r += SP_M) {
-                    const long long rr = std::min<long long>(SP_M, rows - r);
-                    add_units(ul, S, bits, r, rr, 0, Lm, NT, std::min(KCHUNK, Lg - k0), 0, 0, k0);
-                    if (Lm > 1)
-                        add_units(ul, S, bits, r, rr, 0, Lm - 1, NT, std::min(KCHUNK, Lg - 1 - k0), 1 | 2, 0, k0);
-                }
-            }, &u));
-            if (ch == 0)
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], t.cos_f, t.sin_f,
-                                   EpiDftFwd<false>{G, C, Lg}));
-            else
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], t.cos_f, t.sin_f,
-                                   EpiDftFwd<true>{G, C, Lg}));
-        }
-        return ZEST_GPU_OK;
+    return tuned_stage(ctx, st, WK_DFT_F, S, Lg, Lm, batch, Lm, true, [&](int NT) -> int {
+        UnitList* u;
+        ZG_TRY(get_units(ctx, std::make_tuple(int(WK_DFT_F), Lg, Lm, batch, S, nt_pass(NT)), [&](UnitList& ul) {
+            for (long long r = 0; r < rows; r += SP_M) {
+                const long long rr = std::min<long long>(SP_M, rows - r);
+                add_units(ul, S, bits, r, rr, 0, Lm, NT, Lg, 0, 0);
+                if (Lm > 1) add_units(ul, S, bits, r, rr, 0, Lm - 1, NT, Lg - 1, 1 | 2, 0);
+            }
+        }, &u));
+        return run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], t.cos_f, t.sin_f, EpiDftFwd{G, C, Lg});
     });
 }
 
-// The parity sums E_p[b][m][j][kc] (kc < nr2) a Legendre stage leaves
-// unwritten, which the inverse DFT reads as 0: E_0 for m >= Lm, E_1 for
-// m >= Lm - 1 (its last group is empty).
-int zero_parity_tails(zest_gpu_context* ctx, double* E, int batch, int Lg, int Lm, int kh, int nr2) {
-    StageScope sc(ctx, ST_MEMSET);
-    const long long eblock = (long long)Lg * kh * nr2;  // one (p, b)
-    const size_t row = (size_t)kh * nr2 * sizeof(double);
-    if (Lm < Lg)
-        ZG_CUDA_TRY(cudaMemset2DAsync(E + (size_t)Lm * kh * nr2, eblock * sizeof(double), 0, (size_t)(Lg - Lm) * row,
-                                      batch, ctx->stream));
-    ZG_CUDA_TRY(cudaMemset2DAsync(E + (size_t)batch * eblock + (size_t)(Lm - 1) * kh * nr2, eblock * sizeof(double), 0,
-                                  (size_t)(Lg - Lm + 1) * row, batch, ctx->stream));
-    return ZEST_GPU_OK;
-}
-
-// Inverse longitude DFT of the spectra the loader forms (rows (b, col), C
-// columns) to the grids x[b][lon][col] (item stride gsz): a cos pass writing
-// x_0 and the cos sums C_i (to Cs, batch * Lg * C doubles), then a sin pass
-// reading them and writing x_i = C_i + S_i, x_{N-i} = C_i - S_i; both K-chunked.
+// Inverse longitude DFT (order Lg <= 256) of the spectra the loader forms (rows
+// (b, col), C columns) to the grids x[b][lon][col] (item stride gsz): a cos pass
+// writing x_0 and the cos sums C_i (as integers, to Cs, batch * Lg * C of 8
+// bytes), then a sin pass reading them and writing x_i = C_i + S_i, x_{N-i} =
+// C_i - S_i.  The pair of launches overwrites its outputs: tuned.
 template <class Loader>
-int dft_backward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t, int S, int wk,
-                       const Loader& ld, int C, int N, int Lg, int Lm, int batch, double* grids, long long gsz,
-                       double* Cs) {
+int dft_backward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t, int S, const Loader& ld, int C,
+                       int N, int Lg, int Lm, int batch, double* grids, long long gsz, double* Cs) {
     const int bits = digit_bits(Lg);
     const long long rows = (long long)batch * C;
     ZG_TRY(st->op[0].ensure(rows, r16(Lg), S));
@@ -2377,61 +2156,24 @@ int dft_backward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t
         StageScope sc(ctx, ST_SPLIT_SLICE);
         ZG_TRY(launch_slice2(ctx->stream, ld, rows, Lg, Lg - 1, 1, S, bits, Loader::MODE, st->op[0], st->op[1]));
     }
-    if (Lg > 1 && Lg <= KCHUNK && t.cos_bj.rows) {
-      // single sums: the cos and sin results combined in integers (the pair of
-      // launches overwrites its outputs: tuned)
-      return tuned_stage(ctx, st, wk, S, Lg, Lm, batch, Lg, true, [&](int NT) -> int {
+    return tuned_stage(ctx, st, WK_DFT_B, S, Lg, Lm, batch, Lg, true, [&](int NT) -> int {
         long long* Ts = reinterpret_cast<long long*>(Cs);
         UnitList* u;
-        ZG_TRY(get_units(ctx, std::make_tuple(wk, Lg, Lm, batch, S, 4 + nt_pass(NT)), [&](UnitList& ul) {
+        ZG_TRY(get_units(ctx, std::make_tuple(int(WK_DFT_B), Lg, Lm, batch, S, 4 + nt_pass(NT)), [&](UnitList& ul) {
             for (long long r = 0; r < rows; r += SP_M)
                 add_units(ul, S, bits, r, std::min<long long>(SP_M, rows - r), 0, Lg, NT, Lg, 0, 0, 0);
         }, &u));
         ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], t.cos_bj, t.sin_bj,
                            EpiDftBwdCosRaw{grids, Ts, C, N, Lg, gsz}));
         UnitList* v;
-        ZG_TRY(get_units(ctx, std::make_tuple(wk, Lg, Lm, batch, S, 5 + nt_pass(NT)), [&](UnitList& ul) {
+        ZG_TRY(get_units(ctx, std::make_tuple(int(WK_DFT_B), Lg, Lm, batch, S, 5 + nt_pass(NT)), [&](UnitList& ul) {
             for (long long r = 0; r < rows; r += SP_M)  // sin rows i = 1 + (0 .. Lg - 2) of the joint table
                 add_units(ul, S, bits, r, std::min<long long>(SP_M, rows - r), 1, Lg - 1, NT, Lg - 1, 1 | 2 | 4, 0,
                           0);
         }, &v));
         return run_gemm_nt(ctx, NT, S, *v, st->op[0], st->op[1], t.cos_bj, t.sin_bj,
                            EpiDftBwdSinRaw{grids, Ts, C, N, Lg, gsz});
-      });
-    }
-    const int NT = stage_nt(st, wk, S, Lg);
-    for (int ch = 0; ch < nchunks(Lg); ++ch) {
-        const int k0 = ch * KCHUNK;
-        UnitList* u;
-        ZG_TRY(get_units(ctx, std::make_tuple(wk, Lg, Lm, batch, S, 8 * ch + nt_pass(NT)), [&](UnitList& ul) {
-            for (long long r = 0; r < rows; r += SP_M)
-                add_units(ul, S, bits, r, std::min<long long>(SP_M, rows - r), 0, Lg, NT, std::min(KCHUNK, Lg - k0),
-                          0, 0, k0);
-        }, &u));
-        if (ch == 0)
-            ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], t.cos_b, t.sin_b,
-                            EpiDftBwdCos<false>{grids, Cs, C, N, Lg, gsz}));
-        else
-            ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], t.cos_b, t.sin_b,
-                            EpiDftBwdCos<true>{grids, Cs, C, N, Lg, gsz}));
-    }
-    // the sin pass after every cos chunk: its first chunk reads the finished C_i
-    for (int ch = 0; Lg > 1 && ch < nchunks(Lg - 1); ++ch) {
-        const int k0 = ch * KCHUNK;
-        UnitList* v;
-        ZG_TRY(get_units(ctx, std::make_tuple(wk, Lg, Lm, batch, S, 1 + 8 * ch + nt_pass(NT)), [&](UnitList& ul) {
-            for (long long r = 0; r < rows; r += SP_M)
-                add_units(ul, S, bits, r, std::min<long long>(SP_M, rows - r), 0, Lg - 1, NT,
-                          std::min(KCHUNK, Lg - 1 - k0), 1 | 2 | 4, 0, k0);
-        }, &v));
-        if (ch == 0)
-            ZG_TRY(run_gemm_nt(ctx, NT, S, *v, st->op[0], st->op[1], t.cos_b, t.sin_b,
-                            EpiDftBwdSin<false>{grids, Cs, C, N, Lg, gsz}));
-        else
-            ZG_TRY(run_gemm_nt(ctx, NT, S, *v, st->op[0], st->op[1], t.cos_b, t.sin_b,
-                            EpiDftBwdSin<true>{grids, Cs, C, N, Lg, gsz}));
-    }
-    return ZEST_GPU_OK;
+    });
 }
 
 // SH Legendre tables in digit slices: the forward table (weights and the
@@ -2515,8 +2257,15 @@ int split_zt_forward(zest_gpu_context* ctx, ZtPlan& plan, int Lg, int Le, int Lm
     double* G = ctx->s0.as<double>();
     double* flm = ctx->s1.as<double>();
 
-    // ---- longitude DFT: folded cos/sin products ----
-    ZG_TRY(dft_forward_stage(ctx, st, *tb->dft, S, WK_DFT_F, grids, sh.size(), C, N, Lg, Lm, batch, G));
+    // ---- longitude: folded cos/sin products, above 256 terms the fixed-point FFT ----
+    if (tb->dft) {
+        ZG_TRY(dft_forward_stage(ctx, st, *tb->dft, S, grids, sh.size(), C, N, Lg, Lm, batch, G));
+    } else {
+        const FftPlan* fft;
+        ZG_TRY(get_fft(ctx, N, &fft));
+        StageScope sc(ctx, ST_FFT_FWD);
+        ZG_TRY(launch_fixed_fft_fwd(s, *fft, grids, sh.size(), C, 1, C, Lm, Lg, batch, 0, G));
+    }
     // ---- Legendre (folded over the equator) ----
     {
         const int bits = digit_bits(kh);
@@ -2659,8 +2408,8 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
         }));
         // ---- longitude: inverse real DFT of the spectra at every latitude ----
         // (the cos sums C_i go to the scratch of the spectra, consumed by the slicing)
-        ZG_TRY(dft_backward_stage(ctx, st, *tb->dft, S, WK_DFT_B, DftBwdGridLoader{E, Lg, C, nr, nlat}, C, N, Lg,
-                                  Lm, batch, grids, sh.size(), E));
+        ZG_TRY(dft_backward_stage(ctx, st, *tb->dft, S, DftBwdGridLoader{E, Lg, C, nr, nlat}, C, N, Lg, Lm, batch,
+                                  grids, sh.size(), E));
         return split_finish(ctx);
     }
     // ---- Legendre: flm -> G (north/south unfold; parity 1 read-modify-write) ----
@@ -2675,7 +2424,6 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
             ZG_TRY(launch_slice2(s, LegBwdLoader{flm, batch, nr2, Lm}, rows, (Lm + 1) / 2, Lm / 2, 0, S, bits,
                                  SL_PAIR, st->op[0], st->op[1]));
         }
-        ZG_TRY(zero_parity_tails(ctx, E, batch, Lg, Lm, kh, nr2));
         ZG_TRY(tuned_stage(ctx, st, WK_LEG_B, S, Lg, Lm, batch, kh, nchunks((Lm + 1) / 2) == 1, [&](int NT) -> int {
         for (int p = 0; p < 2; ++p)
             for (int ch = 0; ch < nchunks((Lm + 1) / 2); ++ch) {
@@ -2699,11 +2447,14 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
         return ZEST_GPU_OK;
         }));
     }
-    // ---- longitude: inverse real DFT, cos pass then sin read-modify-write pass ----
-    // (the cos sums C_i go to the scratch of the parity sums, consumed by the slicing)
-    ZG_TRY(dft_backward_stage(ctx, st, *tb->dft, S, WK_DFT_B,
-                              DftBwdLoader{E, Lg, C, nr, kh, plan.leg.j0u, plan.leg.j0d, batch}, C, N,
-                              Lg, Lm, batch, grids, sh.size(), E));
+    // ---- inverse longitude transform, from the parity sums ----
+    {
+        const FftPlan* fft;
+        ZG_TRY(get_fft(ctx, N, &fft));
+        StageScope sc(ctx, ST_FFT_INV);
+        ZG_TRY(launch_fixed_fft_inv_parity(s, *fft, E, int(sh.nlat), nr, kh, plan.leg.j0u, plan.leg.j0d, Lm, Lg,
+                                           batch, 0, grids, sh.size(), C, 1));
+    }
     return split_finish(ctx);
 }
 
@@ -2733,8 +2484,8 @@ int run_gemm_st(zest_gpu_context* ctx, UnitList& ul, const SliceArray& A, const 
 }
 }  // namespace
 
-int split_st_forward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int batch, const double* grids, double* X,
-                     double* coeffs, long long csz) {
+int split_st_forward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int batch, const double* X, double* coeffs,
+                     long long csz) {
     const int S = ctx->slices;
     if (S != 6) return fail(ZEST_GPU_ERR_UNSUPPORTED, "split SH transforms need 6 slices");
     cudaStream_t s = ctx->stream;
@@ -2744,13 +2495,6 @@ int split_st_forward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int ba
     if (Lg > SL_KMAX || kh > SL_KMAX) return fail(ZEST_GPU_ERR_UNSUPPORTED, "split SH path: orders up to 2048");
     StSplitTables* tb;
     ZG_TRY(build_st_tables(ctx, st, plan, S, &tb));
-    if (split_st_tensor_dft(plan.sh.latlon, Lg)) {
-        // LonLat grids [lon][lat]: the longitude DFT on the tensor cores, to X[b][m][lat][re, im]
-        const DftTables* dt;
-        ZG_TRY(build_dft_tables(ctx, st, Lg, int(plan.sh.nlon), S, &dt));
-        ZG_TRY(dft_forward_stage(ctx, st, *dt, S, WK_ST_DFT_F, grids, plan.sh.size(), nlat, int(plan.sh.nlon), Lg, Lm,
-                                 batch, X));
-    }
     const int bits = 8;
     const long long per_m = 2LL * batch, rows = (long long)Lm * per_m;
     ZG_TRY(st->op[0].ensure(rows, r16(kh), S));
@@ -2787,15 +2531,14 @@ int split_st_forward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int ba
 }
 
 int split_st_backward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int batch, const double* coeffs,
-                      long long csz, double* X, double* grids) {
+                      long long csz, double** Eout) {
     const int S = ctx->slices;
     if (S != 6) return fail(ZEST_GPU_ERR_UNSUPPORTED, "split SH transforms need 6 slices");
     cudaStream_t s = ctx->stream;
     SplitState* st;
     ZG_TRY(get_state(ctx, &st));
-    const int kh = plan.leg.nnodes, nlat = int(plan.sh.nlat), kl = r16((Lg + 1) / 2);
+    const int kh = plan.leg.nnodes, kl = r16((Lg + 1) / 2);
     if (Lg > SL_KMAX || kh > SL_KMAX) return fail(ZEST_GPU_ERR_UNSUPPORTED, "split SH path: orders up to 2048");
-    const bool lonlat = split_st_tensor_dft(plan.sh.latlon, Lg);
     StSplitTables* tb;
     ZG_TRY(build_st_tables(ctx, st, plan, S, &tb));
     const int bits = 8;
@@ -2807,8 +2550,9 @@ int split_st_backward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int b
         ZG_TRY(launch_slice2(s, StLegBwdLoader{coeffs, csz, batch, Lm}, rows, (Lm + 1) / 2, Lm / 2, 0, S, bits,
                              SL_PAIR, st->op[0], st->op[1]));
     }
-    // parity sums E[p][b][m][j][c]; groups with no degree below Lm are not
-    // written and the unfolding reads them as 0
+    // parity sums E[p][b][m][j][c], conjugated for the inverse longitude
+    // transform; groups with no degree below Lm are not written and it reads
+    // them as 0
     ZG_TRY(ctx->s1.ensure((size_t)2 * batch * Lg * kh * 2 * sizeof(double)));
     double* E = ctx->s1.as<double>();
     const int nchunk = ((Lm + 1) / 2 + ST_KCHUNK - 1) / ST_KCHUNK;
@@ -2829,34 +2573,15 @@ int split_st_backward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int b
                                      }
                              },
                              &u));
-            // conjugated for the inverse DFT of a LonLat grid; the unfolding conjugates
-            const unsigned long long sgi = lonlat ? (1ull << 63) : 0ull;
             if (ch == 0)
                 return run_gemm_st<NT>(ctx, *u, tb->leg_bT, st->op[0], st->op[1],
-                                       EpiStLegBwdE<false>{E, batch, Lg, kh, sgi});
+                                       EpiStLegBwdE<false>{E, batch, Lg, kh});
             return run_gemm_st<NT>(ctx, *u, tb->leg_bT, st->op[0], st->op[1],
-                                   EpiStLegBwdE<true>{E, batch, Lg, kh, sgi});
+                                   EpiStLegBwdE<true>{E, batch, Lg, kh});
         }));
     }
-    if (lonlat) {
-        // LonLat grids [lon][lat]: the inverse longitude DFT on the tensor cores,
-        // straight from the parity sums; X holds the cos sums
-        ZG_TRY(zero_parity_tails(ctx, E, batch, Lg, Lm, kh, 2));
-        const DftTables* dt;
-        ZG_TRY(build_dft_tables(ctx, st, Lg, int(plan.sh.nlon), S, &dt));
-        ZG_TRY(dft_backward_stage(ctx, st, *dt, S, WK_ST_DFT_B,
-                                  DftBwdLoader{E, Lg, nlat, 1, kh, plan.leg.j0u, plan.leg.j0d, batch}, nlat,
-                                  int(plan.sh.nlon), Lg, Lm, batch, grids, plan.sh.size(), X));
-        return split_finish(ctx);
-    }
-    {
-        StageScope sc(ctx, ST_SPLIT_SLICE);
-        const long long n = (long long)batch * Lg * kh * 2;
-        st_unfold_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(E, X, batch, Lg, Lm, kh, nlat, plan.leg.j0u,
-                                                                  plan.leg.j0d);
-        ZG_TRY(launch_check("st_unfold_kernel"));
-    }
-    return split_finish(ctx);
+    *Eout = E;
+    return ZEST_GPU_OK;
 }
 
 // ===========================================================================

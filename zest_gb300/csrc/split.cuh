@@ -22,18 +22,14 @@ int split_zt_forward(zest_gpu_context* ctx, ZtPlan& plan, int Lg, int Le, int Lm
                      double* coeffs);
 int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int Lm, int batch, const double* coeffs,
                       double* grids);
-// True when the split SH path also runs the longitude DFT (on the tensor
-// cores, in place of the FP64 FFT): LonLat grids of order 2 and above.
-inline bool split_st_tensor_dft(bool latlon, int Lg) { return !latlon && Lg >= 2; }
-// SH transforms in split precision (6 slices).  Forward: grids -> the spectra
-// X[b][m][lat][2] (by the tensor-core DFT where split_st_tensor_dft; else X
-// already holds the forward FFT's output) -> coefficients of degrees < Lm.
-// Backward: coefficients -> grids where split_st_tensor_dft (X is scratch);
-// else -> X, for the caller's inverse FFT.
-int split_st_forward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int batch, const double* grids, double* X,
-                     double* coeffs, long long csz);
+// Legendre sums of the SH transforms in split precision (6 slices).  Forward:
+// the spectra X[b][m][lat][2] of orders m < Lm -> coefficients of degrees < Lm.
+// Backward: coefficients -> the parity sums E_p[b][m][j'][2] (in the context's
+// scratch), conjugated, for the inverse longitude transform.
+int split_st_forward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int batch, const double* X, double* coeffs,
+                     long long csz);
 int split_st_backward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int batch, const double* coeffs,
-                      long long csz, double* X, double* grids);
+                      long long csz, double** E);
 // Rotor::rotate of a batch of real expansions (Zernike, SH or row-skipping,
 // of equal or different orders) with the two X(+-pi/2) products of every
 // rotated vector as split GEMMs (orders up to 256): vecs = the

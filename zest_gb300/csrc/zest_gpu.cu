@@ -52,7 +52,7 @@ static int set_device(zest_gpu_context* ctx) {
     return ZEST_GPU_OK;
 }
 
-static int get_fft(zest_gpu_context* ctx, int N, const FftPlan** out) {
+int get_fft(zest_gpu_context* ctx, int N, const FftPlan** out) {
     auto it = ctx->ffts.find(N);
     if (it == ctx->ffts.end()) {
         auto e = std::make_unique<FftEntry>();
@@ -65,7 +65,11 @@ static int get_fft(zest_gpu_context* ctx, int N, const FftPlan** out) {
         if (fft_smem_bytes(e->plan, 1) > 220 * 1024) return fail(ZEST_GPU_ERR_UNSUPPORTED, "FFT length too large");
         ZG_TRY(upload(e->tab, tab, ctx->stream));
         ZG_TRY(upload(e->rows, rows, ctx->stream));
+        std::vector<int4> itab;
+        fixed_fft_table(tab, itab);
+        ZG_TRY(upload(e->itab, itab, ctx->stream));
         e->plan.tab = e->tab.as<double2>();
+        e->plan.itab = e->itab.as<int4>();
         e->plan.in_row = e->rows.as<int>();
         e->plan.out_row = e->plan.in_row + N;
         it = ctx->ffts.emplace(N, std::move(e)).first;
@@ -445,15 +449,19 @@ int st_forward_dev(zest_gpu_context* ctx, int sn, int sp, int layout, int Lg, in
     ZG_TRY(get_fft(ctx, int(sh.nlon), &fft));
     ZG_TRY(ctx->s0.ensure((size_t)batch * Lg * sh.nlat * 2 * sizeof(double)));
     double* X = ctx->s0.as<double>();
-    const bool split = ctx->precision == ZEST_PRECISION_SPLIT;
-    if (!split || !split_st_tensor_dft(sh.latlon, Lg)) {
-        StageScope sc(ctx, ST_FFT_FWD);
-        if (layout == ZEST_LAYOUT_LATLON)
-            ZG_TRY(launch_rfft_fwd(s, *fft, grids, sh.size(), 1, sh.nlon, int(sh.nlat), Lg, batch, 1, X));
-        else
-            ZG_TRY(launch_rfft_fwd(s, *fft, grids, sh.size(), sh.nlat, 1, int(sh.nlat), Lg, batch, 0, X));
+    const bool latlon = layout == ZEST_LAYOUT_LATLON;
+    const long long si = latlon ? 1 : sh.nlat, sc_ = latlon ? sh.nlon : 1;  // strides of longitude and latitude
+    if (ctx->precision == ZEST_PRECISION_SPLIT) {
+        {
+            StageScope sc(ctx, ST_FFT_FWD);
+            ZG_TRY(launch_fixed_fft_fwd(s, *fft, grids, sh.size(), si, sc_, int(sh.nlat), Lm, Lg, batch, latlon, X));
+        }
+        return split_st_forward(ctx, *plan, Lg, Lm, batch, X, coeffs, csz);
     }
-    if (split) return split_st_forward(ctx, *plan, Lg, Lm, batch, grids, X, coeffs, csz);
+    {
+        StageScope sc(ctx, ST_FFT_FWD);
+        ZG_TRY(launch_rfft_fwd(s, *fft, grids, sh.size(), si, sc_, int(sh.nlat), Lg, batch, latlon, X));
+    }
     LegMeta lm;
     lm.P = plan->leg.Pf.as<double>();
     lm.off = plan->leg.off.as<long long>();
@@ -483,18 +491,20 @@ int st_backward_dev(zest_gpu_context* ctx, int sn, int sp, int layout, int Le, i
     const StShape& sh = plan->sh;
     const FftPlan* fft;
     ZG_TRY(get_fft(ctx, int(sh.nlon), &fft));
+    const bool latlon = layout == ZEST_LAYOUT_LATLON;
+    const long long si = latlon ? 1 : sh.nlat, sc_ = latlon ? sh.nlon : 1;  // strides of longitude and latitude
+    if (ctx->precision == ZEST_PRECISION_SPLIT) {
+        double* E;
+        ZG_TRY(split_st_backward(ctx, *plan, Lg, Lm, batch, coeffs, csz, &E));
+        {
+            StageScope sc(ctx, ST_FFT_INV);
+            ZG_TRY(launch_fixed_fft_inv_parity(s, *fft, E, int(sh.nlat), 1, plan->leg.nnodes, plan->leg.j0u,
+                                               plan->leg.j0d, Lm, Lg, batch, latlon, grids, sh.size(), si, sc_));
+        }
+        return split_finish(ctx);
+    }
     ZG_TRY(ctx->s0.ensure((size_t)batch * Lg * sh.nlat * 2 * sizeof(double)));
     double* X = ctx->s0.as<double>();
-    const bool split = ctx->precision == ZEST_PRECISION_SPLIT;
-    if (split && split_st_tensor_dft(sh.latlon, Lg))  // grids written by the tensor-core DFT
-        return split_st_backward(ctx, *plan, Lg, Lm, batch, coeffs, csz, X, grids);
-    if (split) {
-        ZG_TRY(split_st_backward(ctx, *plan, Lg, Lm, batch, coeffs, csz, X, grids));
-        StageScope sc(ctx, ST_FFT_INV);
-        if (layout == ZEST_LAYOUT_LATLON)
-            return launch_rfft_inv(s, *fft, X, int(sh.nlat), Lg, batch, 1, grids, sh.size(), 1, sh.nlon);
-        return launch_rfft_inv(s, *fft, X, int(sh.nlat), Lg, batch, 0, grids, sh.size(), sh.nlat, 1);
-    }
     LegMeta lm;
     lm.P = plan->leg.Pb.as<double>();
     lm.off = plan->leg.off.as<long long>();
@@ -509,9 +519,7 @@ int st_backward_dev(zest_gpu_context* ctx, int sn, int sp, int layout, int Le, i
         ZG_TRY(launch_st_leg_bwd(s, lm, tl, coeffs, X, Lg, int(sh.nlat), batch, csz));
     }
     StageScope sc(ctx, ST_FFT_INV);
-    if (layout == ZEST_LAYOUT_LATLON)
-        return launch_rfft_inv(s, *fft, X, int(sh.nlat), Lg, batch, 1, grids, sh.size(), 1, sh.nlon);
-    return launch_rfft_inv(s, *fft, X, int(sh.nlat), Lg, batch, 0, grids, sh.size(), sh.nlat, 1);
+    return launch_rfft_inv(s, *fft, X, int(sh.nlat), Lg, batch, latlon, grids, sh.size(), si, sc_);
 }
 
 // ---------------------------------------------------------------------------
