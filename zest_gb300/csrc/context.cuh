@@ -118,7 +118,6 @@ struct RaggedPlan {
     const void* grids = nullptr;
     int zn = 0, sn = 0, sp = 0, type = 0, precision = 0, slices = 0;
     int Lmax = 0;
-    long long nwork = 0;
     DevBuf coff;                                               // per-item coefficient offsets
     DevBuf vecl;                                               // the {item, n, l, first pair} vectors sorted by l
     std::vector<long long> voff;                               // vecl rows of order l: [voff[l], voff[l+1])
@@ -132,14 +131,6 @@ struct RaggedPlan {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
     }
-};
-
-// The rotated vectors of a batch of expansions of one order, sorted by l
-// ({item, n, l, first coefficient}), and each item's coefficient offset.
-struct UniformRotation {
-    DevBuf vecs, coff;
-    std::vector<long long> voff;
-    long long nvec = 0;
 };
 
 struct TileEntry {
@@ -186,8 +177,8 @@ struct zest_gpu_context {
     std::map<std::tuple<int, int, int, int>, std::unique_ptr<StPlan>> st_plans;
     std::map<int, std::unique_ptr<FftEntry>> ffts;
     std::map<int, std::unique_ptr<DevBuf>> wigner;
+    std::map<int, std::unique_ptr<DevBuf>> wigner_fixed;      // the same as limbs (split rotations)
     std::map<std::tuple<int, int>, std::pair<std::unique_ptr<DevBuf>, int>> vec_lists;
-    std::map<std::tuple<int, int, int>, std::unique_ptr<UniformRotation>> uniform_rot;  // split rotations
     std::map<std::tuple<int, int, int, int, int, int>, std::unique_ptr<TileEntry>> tiles;
     bool autotune = true;                                     // time the tile shapes on first use
     size_t host_chunk_bytes = size_t(1) << 28;                // pipelined host calls: input bytes per chunk

@@ -52,4 +52,40 @@ __device__ __forceinline__ long long to_fixed_c(double x, int Cr) {
     return (((long long)q ^ sg) + 1) >> 1;
 }
 
+// A fixed-point value as h 2^31 + l with a balanced low limb, |l| <= 2^30.
+struct Limbs {
+    int h, l;
+};
+__device__ __forceinline__ Limbs limbs(long long v) {
+    const int l = int(unsigned(v) << 1) >> 1;
+    return Limbs{int((v - l) >> 31), l};
+}
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+    long long r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
+// Sum of products value x constant, the constants with CBITS fraction bits:
+// three 32 x 32 -> 64-bit multiply-adds a term (the product of the low limbs,
+// below 2^(60 - CBITS), is dropped), rounded once at the end.  The caller bounds
+// the terms: |xl ch| <= 2^(30 + CBITS - 31) each, and sum |xh| 2^30, below 2^63.
+template <int CBITS>
+struct FixedAcc {
+    long long p1 = 0, p2 = 1ll << (CBITS - 32);  // half a unit
+    __device__ __forceinline__ void add(Limbs x, int ch, int cl) {
+        p1 = mad_wide(x.h, ch, p1);
+        p2 = mad_wide(x.h, cl, p2);
+        p2 = mad_wide(x.l, ch, p2);
+    }
+    __device__ __forceinline__ long long value() const {
+        return (long long)((unsigned long long)p1 << (62 - CBITS)) + (p2 >> (CBITS - 31));
+    }
+};
+
+// Scale of a set of values from the high word of the largest magnitude:
+// |x| < 2^scale; and whether that is an infinity or a NaN.
+__device__ __forceinline__ int fixed_scale(unsigned hi) { return max(int(hi >> 20), 64) - 1022; }
+__device__ __forceinline__ bool not_finite(unsigned hi) { return hi >= 0x7FF00000u; }
+__device__ __forceinline__ double nan64() { return __longlong_as_double(0x7FF8000000000000ll); }
+
 }  // namespace zgpu

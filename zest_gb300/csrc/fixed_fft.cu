@@ -59,30 +59,7 @@ using Z = longlong2;  // re, im
 __device__ __forceinline__ Z zadd(Z a, Z b) { return make_longlong2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ Z zsub(Z a, Z b) { return make_longlong2(a.x - b.x, a.y - b.y); }
 
-struct Limbs {
-    int h, l;  // value = h 2^31 + l, |l| <= 2^30
-};
-__device__ __forceinline__ Limbs limbs(long long v) {
-    const int l = int(unsigned(v) << 1) >> 1;
-    return Limbs{int((v - l) >> LIMB), l};
-}
-__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
-    long long r;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-    return r;
-}
-// sum of products value * root
-struct Acc {
-    long long p1 = 0, p2 = 1ll << (CBITS - LIMB - 1);  // p2 starts at half a unit: rounds to nearest
-    __device__ __forceinline__ void add(Limbs x, int ch, int cl) {
-        p1 = mad_wide(x.h, ch, p1);
-        p2 = mad_wide(x.h, cl, p2);
-        p2 = mad_wide(x.l, ch, p2);
-    }
-    __device__ __forceinline__ long long value() const {
-        return (long long)((unsigned long long)p1 << (2 * LIMB - CBITS)) + (p2 >> (CBITS - LIMB));
-    }
-};
+using Acc = FixedAcc<CBITS>;  // sum of products value * root
 // a W for a root w = {ch, cl of the real part, of the imaginary part}
 __device__ __forceinline__ Z zmul(Z a, int4 w) {
     const Limbs x = limbs(a.x), y = limbs(a.y);
@@ -302,11 +279,6 @@ __device__ __forceinline__ Z* run_plan(Z* a, Z* b, const int4* tab, const FftPla
     return a;
 }
 
-// Scale of a column from the high word of its largest magnitude: |x| < 2^scale.
-__device__ __forceinline__ int column_scale(unsigned hi) { return max(int(hi >> 20), 64) - 1022; }
-__device__ __forceinline__ bool not_finite(unsigned hi) { return hi >= 0x7FF00000u; }
-__device__ __forceinline__ double nan64() { return __longlong_as_double(0x7FF8000000000000ll); }
-
 // x(b, i, col) = x + b*xb + i*si + col*sc ; lon_fast: i is the contiguous axis.
 // F: `ms` orders per item, of which m < nm are written.
 template <int NC>
@@ -345,7 +317,7 @@ __global__ void __launch_bounds__(256) fixed_fwd_kernel(const __grid_constant__ 
         if (mx) atomicMax(&top[cl], mx);
         __syncthreads();
         const unsigned h = top[cl];
-        const int c = 1074 + column_scale(h) - hb;
+        const int c = 1074 + fixed_scale(h) - hb;
         const bool bad = not_finite(h);
 #pragma unroll 4
         for (int i = i0; i < N; i += rs) {
@@ -368,7 +340,7 @@ __global__ void __launch_bounds__(256) fixed_fwd_kernel(const __grid_constant__ 
         __syncthreads();
         for (int cl = 0; cl < W; ++cl) {
             const unsigned h = top[cl];
-            const int c = 1074 + column_scale(h) - hb;
+            const int c = 1074 + fixed_scale(h) - hb;
             const bool bad = not_finite(h);
             for (int i = threadIdx.x; i < N; i += blockDim.x) {
                 long long* q = Al + plan.in_row[i] * W + cl;
@@ -381,7 +353,7 @@ __global__ void __launch_bounds__(256) fixed_fwd_kernel(const __grid_constant__ 
     // separate the two real spectra and store conj(X_m), m < nm (twice them: hb + 1)
     const int cp = threadIdx.x & (NC - 1), col = col0 + 2 * cp;
     const unsigned ha = top[2 * cp], hc = top[2 * cp + 1];
-    const int sa = column_scale(ha) - hb - 1, sb = column_scale(hc) - hb - 1;
+    const int sa = fixed_scale(ha) - hb - 1, sb = fixed_scale(hc) - hb - 1;
     const bool bad_a = not_finite(ha), bad_b = not_finite(hc);
     const int m0 = threadIdx.x / NC, dm = blockDim.x / NC;
     double2* out = reinterpret_cast<double2*>(F) + ((long long)b * ms + m0) * C + col;
@@ -470,7 +442,7 @@ __global__ void __launch_bounds__(256) fixed_inv_kernel(const __grid_constant__ 
     {
         // Hermitian completion of the packed spectra F_a + i F_b, conjugated
         const unsigned ha = top[2 * cp], hc = top[2 * cp + 1];
-        const int ca = 1074 + column_scale(ha) - hb, cb = 1074 + column_scale(hc) - hb;
+        const int ca = 1074 + fixed_scale(ha) - hb, cb = 1074 + fixed_scale(hc) - hb;
         const bool bad_a = not_finite(ha), bad_b = not_finite(hc);
         auto fix = [](double v, int c, bool bad) { return bad ? 0ll : to_fixed_c(v, c); };
 #pragma unroll 2
@@ -496,7 +468,7 @@ __global__ void __launch_bounds__(256) fixed_inv_kernel(const __grid_constant__ 
     // the second column of a pair is the imaginary part, conjugated
     auto value = [&](int i, int cl, unsigned h) {
         const long long v = Zl[plan.out_row[i] * W + cl];
-        return not_finite(h) ? nan64() : i64_ldexp((cl & 1) ? -v : v, column_scale(h) - hb);
+        return not_finite(h) ? nan64() : i64_ldexp((cl & 1) ? -v : v, fixed_scale(h) - hb);
     };
     if (!lon_fast) {
         const int cl = threadIdx.x & (W - 1), i0 = threadIdx.x / W, rs = blockDim.x / W;

@@ -133,6 +133,15 @@ int launch_rotate_euler_grad(cudaStream_t s, int kind, int L, int batch, const d
 int launch_rotate_ragged(cudaStream_t s, int Lmax, int items, double* coeffs, const long long* coff, const int4* vecs,
                          const std::vector<long long>& voff, const long long* voff_dev, const double* wigner,
                          const double* euler, int type, double* phase_scratch);
+// The same rotations in 64-bit fixed point (rotate_fixed.cu), orders up to 256,
+// with the d(pi/2) table as limbs (launch_fixed_wigner).
+constexpr int kFixedRotateOrder = 256;
+int launch_fixed_wigner(cudaStream_t s, int L, const double* wigner, int2* out);
+int launch_rotate_fixed(cudaStream_t s, int kind, int L, int batch, double* coeffs, long long cstride,
+                        const int2* wigner, const double* euler, int type, double* phase_scratch);
+int launch_rotate_fixed_ragged(cudaStream_t s, int Lmax, int items, double* coeffs, const long long* coff,
+                               const int4* vecs, const std::vector<long long>& voff, const long long* voff_dev,
+                               const int2* wigner, const double* euler, int type, double* phase_scratch);
 // The phase tables e^{-i m angle} [item][alpha', beta', gamma'][m < Lmax] of a
 // ragged rotation (double2 entries in phase_scratch).
 int launch_phases(cudaStream_t s, int Lmax, int items, const double* euler, int type, double* phase_scratch);

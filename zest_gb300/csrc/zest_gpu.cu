@@ -535,6 +535,21 @@ static int get_wigner(zest_gpu_context* ctx, int L, const double** out) {
     return ZEST_GPU_OK;
 }
 
+// the same table as limbs, for the fixed-point rotations
+static int get_wigner_fixed(zest_gpu_context* ctx, int L, const int2** out) {
+    auto it = ctx->wigner_fixed.find(L);
+    if (it == ctx->wigner_fixed.end()) {
+        const double* wig;
+        ZG_TRY(get_wigner(ctx, L, &wig));
+        auto b = std::make_unique<DevBuf>();
+        ZG_TRY(b->ensure((size_t)wig_off(L) * sizeof(int2)));
+        ZG_TRY(launch_fixed_wigner(ctx->stream, L, wig, b->as<int2>()));
+        it = ctx->wigner_fixed.emplace(L, std::move(b)).first;
+    }
+    *out = it->second->as<int2>();
+    return ZEST_GPU_OK;
+}
+
 // coefficient pairs of one expansion of order L: Zernike, SH triangle, or the
 // row-skipping triangle of one parity ((L + 1)^2 / 4, include/layout.hpp:356-362)
 static long long coeff_pairs(int kind, long long L) {
@@ -565,56 +580,21 @@ static int get_vectors(zest_gpu_context* ctx, int kind, int L, const int2** out,
     return ZEST_GPU_OK;
 }
 
-// The rotated vectors of `batch` expansions of one order, sorted by l, for
-// the split-precision rotation (cached per kind, order and batch).
-static int get_uniform_rotation(zest_gpu_context* ctx, int kind, int L, int batch, UniformRotation** out) {
-    auto key = std::make_tuple(kind, L, batch);
-    auto it = ctx->uniform_rot.find(key);
-    if (it == ctx->uniform_rot.end()) {
-        auto u = std::make_unique<UniformRotation>();
-        std::vector<int4> v;
-        u->voff.assign((size_t)L + 1, 0);
-        for (int l = 0; l < L; ++l) {
-            for (int b = 0; b < batch; ++b) {
-                if (kind == 0) {
-                    for (int n = (l == 0 ? 2 : l); n < L; n += 2) v.push_back(make_int4(b, n, l, int(zidx(n, l, 0))));
-                } else if (kind == 2) {
-                    if ((l & 1) == ((L - 1) & 1)) v.push_back(make_int4(b, L - 1, l, int(((long long)l * l) >> 2)));
-                } else if (l >= 1) {
-                    v.push_back(make_int4(b, l, l, int(tri_idx(l, 0))));
-                }
-            }
-            u->voff[(size_t)l + 1] = (long long)v.size();
-        }
-        std::vector<long long> coff((size_t)batch);
-        for (int b = 0; b < batch; ++b) coff[(size_t)b] = (long long)b * 2 * coeff_pairs(kind, L);
-        u->nvec = (long long)v.size();
-        ZG_TRY(upload(u->vecs, v, ctx->stream));
-        ZG_TRY(upload(u->coff, coff, ctx->stream));
-        it = ctx->uniform_rot.emplace(key, std::move(u)).first;
-    }
-    *out = it->second.get();
-    return ZEST_GPU_OK;
-}
-
 int rotate_dev(zest_gpu_context* ctx, int kind, int L, int batch, double* coeffs, const double* euler, int type) {
     // a whole expansion of order 1 has nothing to rotate; the row span of
     // order 1 (n = 0) still rotates its l = 0 vector, as the reference does
     if (batch == 0 || L < 1 || (L == 1 && kind != 2)) return ZEST_GPU_OK;
     const double* wig;
     ZG_TRY(get_wigner(ctx, L, &wig));
-    if (ctx->precision == ZEST_PRECISION_SPLIT && L <= 256 && L >= 2) {
-        // the X(+-pi/2) products of all vectors of one l as split GEMMs
-        UniformRotation* u;
-        ZG_TRY(get_uniform_rotation(ctx, kind, L, batch, &u));
-        ZG_TRY(ctx->phase.ensure((size_t)batch * 6 * L * sizeof(double)));
-        ZG_TRY(split_rotate_ragged(ctx, L, batch, u->nvec, u->vecs.as<int4>(), u->voff, u->coff.as<long long>(),
-                                   coeffs, wig, euler, type, ctx->phase.as<double>()));
-        return split_finish(ctx);
-    }
     ZG_TRY(ctx->phase.ensure((size_t)batch * 6 * L * sizeof(double)));
     const long long cstride = 2 * coeff_pairs(kind, L);
+    const int2* wigf = nullptr;
+    const bool fixed = ctx->precision == ZEST_PRECISION_SPLIT && L <= kFixedRotateOrder && L >= 2;
+    if (fixed) ZG_TRY(get_wigner_fixed(ctx, L, &wigf));
     StageScope sc(ctx, ST_ROTATE);
+    if (fixed)
+        return launch_rotate_fixed(ctx->stream, kind, L, batch, coeffs, cstride, wigf, euler, type,
+                                   ctx->phase.as<double>());
     return launch_rotate_vectors(ctx->stream, kind, L, batch, coeffs, cstride, wig, euler, type,
                                  ctx->phase.as<double>());
 }
@@ -788,10 +768,13 @@ static int ragged_sequence(zest_gpu_context* ctx, RaggedPlan& P, double* coeffs,
                            double* grids) {
     const double* wig;
     ZG_TRY(get_wigner(ctx, P.Lmax, &wig));
-    if (P.precision == ZEST_PRECISION_SPLIT && P.Lmax <= 256) {
-        // the X(+-pi/2) products of all vectors of one l as split GEMMs
-        ZG_TRY(split_rotate_ragged(ctx, P.Lmax, int(P.orders.size()), P.nwork, P.vecl.as<int4>(), P.voff, P.coff.as<long long>(),
-                                   coeffs, wig, euler, P.type, ctx->phase.as<double>()));
+    if (P.precision == ZEST_PRECISION_SPLIT && P.Lmax <= kFixedRotateOrder) {
+        const int2* wigf;
+        ZG_TRY(get_wigner_fixed(ctx, P.Lmax, &wigf));
+        StageScope sc(ctx, ST_ROTATE);
+        ZG_TRY(launch_rotate_fixed_ragged(ctx->stream, P.Lmax, int(P.orders.size()), coeffs, P.coff.as<long long>(),
+                                          P.vecl.as<int4>(), P.voff, P.voff_dev.as<long long>(), wigf, euler, P.type,
+                                          ctx->phase.as<double>()));
     } else {
         StageScope sc(ctx, ST_ROTATE);
         ZG_TRY(launch_rotate_ragged(ctx->stream, P.Lmax, int(P.orders.size()), coeffs, P.coff.as<long long>(),
@@ -878,7 +861,6 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
     }
     np->coff_h[n] = co;
     np->goff_h[n] = go;
-    np->nwork = (long long)work.size();
     ZG_TRY(upload(np->coff, np->coff_h, ctx->stream));
     {
         // the same vectors grouped by l (stable: item, then n, within a group)
@@ -1125,6 +1107,7 @@ int zest_gpu_trim(zest_gpu_context* ctx) {
     ctx->st_plans.clear();
     ctx->ffts.clear();
     ctx->wigner.clear();
+    ctx->wigner_fixed.clear();
     ctx->vec_lists.clear();
     ctx->tiles.clear();
     ctx->s0.release();
