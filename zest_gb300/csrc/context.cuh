@@ -109,14 +109,24 @@ struct StPlan {
     LegTables leg;
 };
 
+// The buffers and conventions of a call on a batch of uneven order.
+struct RaggedCall {
+    double* coeffs = nullptr;
+    const double* euler = nullptr;
+    double* grids = nullptr;
+    int zn = 0, sn = 0, sp = 0, type = 0, precision = 0, slices = 0;
+    bool operator==(const RaggedCall& o) const {
+        return coeffs == o.coeffs && euler == o.euler && grids == o.grids && zn == o.zn && sn == o.sn && sp == o.sp &&
+               type == o.type && precision == o.precision && slices == o.slices;
+    }
+};
+
 // A batch of expansions of different orders (rotate, then backward
-// transform), its device work lists and the CUDA graph that replays it.
+// transform): its device work lists, the last call, and the CUDA graph that
+// replays that call once it has been repeated.
 struct RaggedPlan {
     std::vector<int> orders;
-    const void* coeffs = nullptr;
-    const void* euler = nullptr;
-    const void* grids = nullptr;
-    int zn = 0, sn = 0, sp = 0, type = 0, precision = 0, slices = 0;
+    RaggedCall call;
     int Lmax = 0;
     DevBuf coff;                                               // per-item coefficient offsets
     DevBuf vecl;                                               // the {item, n, l, first pair} vectors sorted by l
@@ -126,11 +136,14 @@ struct RaggedPlan {
     std::vector<std::tuple<int, int, int>> buckets;            // {order, first item, count}
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    unsigned long long epoch = 0;  // alloc_epoch() when the graph was recorded
-    ~RaggedPlan() {
+    unsigned long long epoch = ~0ull;  // alloc_epoch() after the last call's eager run
+    void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
+        exec = nullptr;
+        graph = nullptr;
     }
+    ~RaggedPlan() { drop_graph(); }
 };
 
 struct TileEntry {
@@ -181,6 +194,7 @@ struct zest_gpu_context {
     std::map<std::tuple<int, int>, std::pair<std::unique_ptr<DevBuf>, int>> vec_lists;
     std::map<std::tuple<int, int, int, int, int, int>, std::unique_ptr<TileEntry>> tiles;
     bool autotune = true;                                     // time the tile shapes on first use
+    bool defer_finish = false;                                // split calls leave the wait flag to their caller
     size_t host_chunk_bytes = size_t(1) << 28;                // pipelined host calls: input bytes per chunk
     std::unique_ptr<RaggedPlan> ragged;                       // last batch of uneven orders, with its graph
     cudaStream_t graph_stream = nullptr;                      // own stream for graph capture and replay

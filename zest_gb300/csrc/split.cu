@@ -2210,8 +2210,10 @@ int build_st_tables(zest_gpu_context* ctx, SplitState* st, StPlan& plan, int S, 
 // Split-precision Zernike transforms
 // ===========================================================================
 // End of a split-path call: check the bounded-wait flag, unless the stream is
-// being captured into a graph (whose caller checks it after each replay).
+// being captured into a graph (whose caller checks it after each replay) or the
+// caller runs several and checks once.
 int split_finish(zest_gpu_context* ctx) {
+    if (ctx->defer_finish) return ZEST_GPU_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     ZG_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &cap));
     if (cap != cudaStreamCaptureStatusNone) return ZEST_GPU_OK;

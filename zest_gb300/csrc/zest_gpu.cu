@@ -759,31 +759,32 @@ int rotate_vjp_dev(zest_gpu_context* ctx, int kind, int L, int batch, const doub
 // ---------------------------------------------------------------------------
 // Batches of expansions of different orders: rotate every expansion (one
 // launch over a ragged work list), then backward-transform each group of equal
-// order as one batch.  The first call for a given (orders, buffers,
-// conventions, precision) runs eagerly -- building tables, work lists and
-// scratch, and autotuning tile shapes -- and then records the same sequence
-// into a CUDA graph; later identical calls replay the graph (a single launch
-// from the host).
-static int ragged_sequence(zest_gpu_context* ctx, RaggedPlan& P, double* coeffs, const double* euler,
-                           double* grids) {
+// order as one batch.  The offsets and the rotation's work list belong to the
+// orders and are kept for the last ones; a call with other buffers (or conventions)
+// runs eagerly -- the first one builds tables and scratch and autotunes tile
+// shapes -- and a call that repeats the last one is recorded into a CUDA graph and
+// replayed from then on (a single launch from the host).  Rebuilding lists and
+// graph for every change of buffers took 8 ms of 51 for 1,024 items.
+static int ragged_sequence(zest_gpu_context* ctx, RaggedPlan& P) {
+    const RaggedCall& c = P.call;
     const double* wig;
     ZG_TRY(get_wigner(ctx, P.Lmax, &wig));
-    if (P.precision == ZEST_PRECISION_SPLIT && P.Lmax <= kFixedRotateOrder) {
+    if (c.precision == ZEST_PRECISION_SPLIT && P.Lmax <= kFixedRotateOrder) {
         const int2* wigf;
         ZG_TRY(get_wigner_fixed(ctx, P.Lmax, &wigf));
         StageScope sc(ctx, ST_ROTATE);
-        ZG_TRY(launch_rotate_fixed_ragged(ctx->stream, P.Lmax, int(P.orders.size()), coeffs, P.coff.as<long long>(),
-                                          P.vecl.as<int4>(), P.voff, P.voff_dev.as<long long>(), wigf, euler, P.type,
+        ZG_TRY(launch_rotate_fixed_ragged(ctx->stream, P.Lmax, int(P.orders.size()), c.coeffs, P.coff.as<long long>(),
+                                          P.vecl.as<int4>(), P.voff, P.voff_dev.as<long long>(), wigf, c.euler, c.type,
                                           ctx->phase.as<double>()));
     } else {
         StageScope sc(ctx, ST_ROTATE);
-        ZG_TRY(launch_rotate_ragged(ctx->stream, P.Lmax, int(P.orders.size()), coeffs, P.coff.as<long long>(),
-                                    P.vecl.as<int4>(), P.voff, P.voff_dev.as<long long>(), wig, euler, P.type,
+        ZG_TRY(launch_rotate_ragged(ctx->stream, P.Lmax, int(P.orders.size()), c.coeffs, P.coff.as<long long>(),
+                                    P.vecl.as<int4>(), P.voff, P.voff_dev.as<long long>(), wig, c.euler, c.type,
                                     ctx->phase.as<double>()));
     }
     for (const auto& bk : P.buckets) {
         const int L = std::get<0>(bk), first = std::get<1>(bk), count = std::get<2>(bk);
-        ZG_TRY(zt_backward_dev(ctx, P.zn, P.sn, P.sp, L, L, count, coeffs + P.coff_h[first], grids + P.goff_h[first]));
+        ZG_TRY(zt_backward_dev(ctx, c.zn, c.sn, c.sp, L, L, count, c.coeffs + P.coff_h[first], c.grids + P.goff_h[first]));
     }
     return ZEST_GPU_OK;
 }
@@ -812,6 +813,45 @@ static int on_graph_stream(zest_gpu_context* ctx, F&& body) {
 static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp, const std::vector<int>& orders,
                                   double* coeffs, const double* euler, int type, double* grids);
 
+// Runs the sequence of `call` and remembers it: every table, list and buffer that
+// a graph of it needs then exists.  The split GEMMs' wait flag is checked once, at
+// the end, not after every group.
+static int ragged_eager(zest_gpu_context* ctx, RaggedPlan& P, const RaggedCall& call) {
+    if (P.exec) ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // its last replay may still run
+    P.drop_graph();
+    P.call = call;
+    P.epoch = ~0ull;  // no graph of a call that failed
+    ZG_TRY(ctx->phase.ensure((size_t)P.orders.size() * 6 * std::max(P.Lmax, 1) * sizeof(double)));
+    ctx->defer_finish = true;
+    int rc = ragged_sequence(ctx, P);
+    ctx->defer_finish = false;
+    if (call.precision == ZEST_PRECISION_SPLIT) {
+        const int late = split_check_flag(ctx);
+        if (rc == ZEST_GPU_OK) rc = late;
+    }
+    if (rc == ZEST_GPU_OK) P.epoch = alloc_epoch().load(std::memory_order_relaxed);
+    return rc;
+}
+
+// Records the sequence of the plan's last call into a graph (nothing executes).
+static int ragged_record(zest_gpu_context* ctx, RaggedPlan& P) {
+    const bool prof = ctx->prof.on;
+    ctx->prof.on = false;
+    ZG_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
+    const int rc = ragged_sequence(ctx, P);
+    cudaGraph_t g = nullptr;
+    const cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
+    ctx->prof.on = prof;
+    if (rc != ZEST_GPU_OK) {
+        if (g) cudaGraphDestroy(g);
+        return rc;
+    }
+    if (ec != cudaSuccess) return fail(ZEST_GPU_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ec));
+    P.graph = g;
+    ZG_CUDA_TRY(cudaGraphInstantiate(&P.exec, g, 0));
+    return ZEST_GPU_OK;
+}
+
 int zt_rotate_backward_ragged_dev(zest_gpu_context* ctx, int zn, int sn, int sp, const std::vector<int>& orders,
                                   double* coeffs, const double* euler, int type, double* grids) {
     return on_graph_stream(ctx, [&] { return ragged_on_graph_stream(ctx, zn, sn, sp, orders, coeffs, euler, type, grids); });
@@ -819,29 +859,22 @@ int zt_rotate_backward_ragged_dev(zest_gpu_context* ctx, int zn, int sn, int sp,
 
 static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp, const std::vector<int>& orders,
                                   double* coeffs, const double* euler, int type, double* grids) {
+    RaggedCall call{coeffs, euler, grids, zn, sn, sp, type, ctx->precision, ctx->slices};
     RaggedPlan* P = ctx->ragged.get();
-    const bool same = P && P->orders == orders && P->coeffs == coeffs && P->euler == euler && P->grids == grids &&
-                      P->zn == zn && P->sn == sn && P->sp == sp && P->type == type &&
-                      P->precision == ctx->precision && P->slices == ctx->slices;
-    // the graph's kernels hold pointers to scratch, tables and work lists: a
-    // buffer freed or reallocated since it was recorded means recording anew
-    if (same && P->exec && P->epoch == alloc_epoch().load(std::memory_order_relaxed)) {
-        ZG_CUDA_TRY(cudaGraphLaunch(P->exec, ctx->stream));
-        if (P->precision == ZEST_PRECISION_SPLIT) ZG_TRY(split_check_flag(ctx));
-        return ZEST_GPU_OK;
+    if (P && P->orders == orders) {
+        // the graph's kernels hold pointers to scratch, tables and work lists: a
+        // buffer freed or reallocated since the last run means running eagerly anew
+        const bool again = P->call == call && P->epoch == alloc_epoch().load(std::memory_order_relaxed);
+        if (again && !P->exec) ZG_TRY(ragged_record(ctx, *P));
+        if (again) {
+            ZG_CUDA_TRY(cudaGraphLaunch(P->exec, ctx->stream));
+            return call.precision == ZEST_PRECISION_SPLIT ? split_check_flag(ctx) : ZEST_GPU_OK;
+        }
+        return ragged_eager(ctx, *P, call);
     }
-    // new plan: offsets, buckets and the rotation work list
+    // new orders: offsets, buckets and the rotation work list
     auto np = std::make_unique<RaggedPlan>();
     np->orders = orders;
-    np->coeffs = coeffs;
-    np->euler = euler;
-    np->grids = grids;
-    np->zn = zn;
-    np->sn = sn;
-    np->sp = sp;
-    np->type = type;
-    np->precision = ctx->precision;
-    np->slices = ctx->slices;
     const int n = int(orders.size());
     np->coff_h.resize(n + 1);
     np->goff_h.resize(n + 1);
@@ -873,29 +906,9 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
         ZG_TRY(upload(np->vecl, byl, ctx->stream));
         ZG_TRY(upload(np->voff_dev, np->voff, ctx->stream));
     }
-    ZG_TRY(ctx->phase.ensure((size_t)n * 6 * std::max(np->Lmax, 1) * sizeof(double)));
+    if (P && P->exec) ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     ctx->ragged = std::move(np);
-    P = ctx->ragged.get();
-    // eager run: the result of this call, and every table, list and buffer the graph needs
-    ZG_TRY(ragged_sequence(ctx, *P, coeffs, euler, grids));
-    ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    // record the same sequence (nothing executes during capture)
-    const bool prof = ctx->prof.on;
-    ctx->prof.on = false;
-    ZG_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
-    const int rc = ragged_sequence(ctx, *P, coeffs, euler, grids);
-    cudaGraph_t g = nullptr;
-    const cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
-    ctx->prof.on = prof;
-    if (rc != ZEST_GPU_OK) {
-        if (g) cudaGraphDestroy(g);
-        return rc;
-    }
-    if (ec != cudaSuccess) return fail(ZEST_GPU_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ec));
-    P->graph = g;
-    ZG_CUDA_TRY(cudaGraphInstantiate(&P->exec, g, 0));
-    P->epoch = alloc_epoch().load(std::memory_order_relaxed);
-    return ZEST_GPU_OK;
+    return ragged_eager(ctx, *ctx->ragged, call);
 }
 
 }  // namespace zgpu
