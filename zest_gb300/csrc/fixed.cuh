@@ -42,14 +42,15 @@ __device__ __forceinline__ double i64_ldexp(long long T, int E) {
 // Cr - E(x) is at least 5 for every element of a row (the row exponent keeps
 // a bit of headroom); PTX shifts of 64 or more give 0, so a zero or an element
 // far below the row's largest rounds to 0 without a branch.
-__device__ __forceinline__ long long to_fixed_c(double x, int Cr) {
+// A bias is added with the rounding one.
+__device__ __forceinline__ long long to_fixed_c(double x, int Cr, long long bias = 0) {
     const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
     const unsigned E = unsigned(bits >> 52) & 0x7FFu;
     const unsigned long long M = (bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
     unsigned long long q;
     asm("shr.b64 %0, %1, %2;" : "=l"(q) : "l"(M), "r"(unsigned(Cr) - E));
     const long long sg = (long long)bits >> 63;  // 0 or -1
-    return (((long long)q ^ sg) + 1) >> 1;
+    return (((long long)q ^ sg) + (1 + 2 * bias)) >> 1;
 }
 
 // A fixed-point value as h 2^31 + l with a balanced low limb, |l| <= 2^30.

@@ -38,7 +38,7 @@
 // Every wait is bounded (about 2 s); on timeout the kernel records an error
 // code and winds down instead of hanging.
 #include <cuda.h>
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <mutex>
@@ -66,7 +66,7 @@ constexpr int SP_EPI_WARPS = 16;                  // epilogue warps: four per TM
 constexpr int SP_THREADS = 32 * (2 + SP_EPI_WARPS);  // + TMA producer + MMA issuer
 constexpr int SP_M = 128;
 constexpr int SP_MIXED = 1;      // narrow threshold value that selects mixed 80/32-column launches
-constexpr int SP_KB = 16;        // K elements per pipeline stage (32 bytes of bf16)
+constexpr int SP_KB = 16;        // K elements per pipeline stage (32 bytes of FP16)
 constexpr long long SP_TIMEOUT_NS = 2000000000LL;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -144,7 +144,7 @@ __device__ __forceinline__ void tmem_relinquish() {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void umma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+__device__ __forceinline__ void umma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
@@ -186,10 +186,10 @@ __device__ __forceinline__ uint64_t desc_sw32(uint32_t saddr) {
     d |= (uint64_t)6 << 61;                    // SWIZZLE_32B
     return d;
 }
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
+__host__ __device__ constexpr uint32_t idesc_f16_f32(int M, int N) {
     return (1u << 4)                       // D format F32
-           | (1u << 7)                     // A format BF16
-           | (1u << 10)                    // B format BF16
+           | (0u << 7)                     // A format F16
+           | (0u << 10)                    // B format F16
            | ((uint32_t)(N >> 3) << 17)    // N / 8
            | ((uint32_t)(M >> 4) << 24);   // M / 16
 }
@@ -466,8 +466,8 @@ struct SliceJob {
     int Ks;           // shared-memory row stride in doubles (padded layout, below)
     int S, bits, R, lr;  // lr = log2(R)
     int K0, Kp0, K1, Kp1;
-    __nv_bfloat16* out0;
-    __nv_bfloat16* out1;
+    __half* out0;
+    __half* out1;
     long long stride0, stride1;  // elements between slices
     int* ex0;
     int* ex1;
@@ -504,43 +504,49 @@ inline int sl_row_stride(int KS) {
     return p + ((6 - p % 4) % 4);
 }
 
-// Balanced 8-bit digits of 8 neighbouring elements (slice 0 most
-// significant), written as 8 BF16 per slice with one 16-byte store.  Adding
-// 128 sum_{i<S-1} 256^i turns the lower balanced digits into the plain bytes
-// of the sum (digit = byte - 128) and leaves the leading digit as the sum
-// shifted down.  A lower digit's float is built by one byte permute,
-// 0x4B4000bb = 2^23 + 2^22 + byte, and one subtraction of 2^23 + 2^22 + 128;
-// the float is exact with at most 8 significant bits, so its upper half is the
-// BF16.
+// 128 in each of the S digit bytes of a biased fixed-point value: byte b of
+// w + digit_bias<S>() is 128 + the balanced digit of weight 256^b, and the
+// leading digit's field (0..256) keeps its ninth bit.
 template <int S>
-__device__ __forceinline__ void store_digits8(const long long (&w)[8], __nv_bfloat16* out, long long stride) {
-    constexpr long long OFF = (long long)((0x8080808080808080ull) >> (8 * (9 - S)));  // 128 per lower byte
-    uint32_t lo[8], hi[8];
+__device__ __forceinline__ constexpr long long digit_bias() {
+    return (long long)(0x8080808080808080ull >> (8 * (8 - S)));
+}
+
+// Balanced 8-bit digits of 8 neighbouring biased elements (slice 0 most
+// significant), written as 8 FP16 per slice with one 16-byte store.  The FP16
+// pattern 0x6400 | byte is 1024 + byte, so a pair of digits is two bytes under
+// that mask and one packed subtraction of 1152; one byte permute brings two
+// digits of two elements together.  5 integer operations an element (9 when
+// each digit was built as a float), which are what the slicing spends its time
+// on: at order 200 x 64 forward + backward SLICE_FIG.
+template <int S>
+__device__ __forceinline__ void store_digits8(const unsigned long long (&u)[8], __half* out, long long stride) {
+    constexpr uint32_t MAGIC = 0x64006400u;
+    const __half2 off = __half2half2(__ushort_as_half(0x6480));  // 1152
+    uint32_t d[S][4];  // [digit byte][pair]
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const unsigned long long u = (unsigned long long)(w[q] + OFF);
-        lo[q] = uint32_t(u);
-        hi[q] = uint32_t(u >> 32);
+    for (int p = 0; p < 4; ++p) {
+        const uint32_t lo0 = uint32_t(u[2 * p]), lo1 = uint32_t(u[2 * p + 1]);
+        const uint32_t hi0 = uint32_t(u[2 * p] >> 32), hi1 = uint32_t(u[2 * p + 1] >> 32);
+        if constexpr (S == 4) {  // the leading field straddles the words
+            d[3][p] = __byte_perm(__funnelshift_r(lo0, hi0, 24), __funnelshift_r(lo1, hi1, 24), 0x5410) | MAGIC;
+        } else {
+            d[S - 1][p] = __byte_perm(hi0, hi1, S == 6 ? 0x6521 : 0x5410) | MAGIC;
+        }
+#pragma unroll
+        for (int b = 0; b < S - 1; b += 2) {
+            const uint32_t t = __byte_perm(b < 4 ? lo0 : hi0, b < 4 ? lo1 : hi1, (b & 2) ? 0x7632 : 0x5410);
+            d[b][p] = (t & 0x00FF00FFu) | MAGIC;
+            if (b + 1 < S - 1) d[b + 1][p] = __byte_perm(t, 0x64646464u, 0x4341);
+        }
     }
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         uint32_t o[4];
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-            float f[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int q = 2 * p + h;
-                if (s == 0) {
-                    const long long u = (long long)(((unsigned long long)hi[q] << 32) | lo[q]);
-                    f[h] = __int_as_float(0x4B400000 + int(u >> (8 * (S - 1)))) - 12582912.0f;
-                } else {
-                    const int b = S - 1 - s;  // byte of the sum holding digit s
-                    f[h] = __int_as_float(int(__byte_perm(b < 4 ? lo[q] : hi[q], 0x4B400000u, 0x7650u | (b & 3)))) -
-                           12583040.0f;
-                }
-            }
-            o[p] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);
+            const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&d[S - 1 - s][p]), off);
+            o[p] = *reinterpret_cast<const uint32_t*>(&v);
         }
         *reinterpret_cast<uint4*>(out + s * stride) = make_uint4(o[0], o[1], o[2], o[3]);
     }
@@ -679,18 +685,18 @@ __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
             constexpr int NJ = 8 + SHIFT;
             auto at = [&](int a, int j) { return base[a * astride + j + (j >> 3)]; };
             if constexpr (MODE == SL_ONE) {
-                long long w[8];
+                unsigned long long w[8];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(0, q), Cr);
+                for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(0, q), Cr, digit_bias<S>());
                 store_digits8<S>(w, J.out0 + row * J.Kp0 + 8 * c, J.stride0);
             } else if constexpr (MODE == SL_FOLD) {
                 long long fu[NJ], fd[NJ];
 #pragma unroll
                 for (int j = 0; j < NJ; ++j) {
-                    fu[j] = to_fixed_c(at(0, j), Cr);
+                    fu[j] = to_fixed_c(at(0, j), Cr, digit_bias<S>());
                     fd[j] = to_fixed_c(at(1, j), Cr);
                 }
-                long long w[8];
+                unsigned long long w[8];
                 if (c < nch0) {
 #pragma unroll
                     for (int q = 0; q < 8; ++q) w[q] = fu[q] + fd[q];
@@ -703,15 +709,15 @@ __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
                 }
             } else {
                 // SL_PAIR: up | dn
-                long long w[8];
+                unsigned long long w[8];
                 if (c < nch0) {
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(0, q), Cr);
+                    for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(0, q), Cr, digit_bias<S>());
                     store_digits8<S>(w, J.out0 + row * J.Kp0 + 8 * c, J.stride0);
                 }
                 if (c < nch1) {
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(1, q + SHIFT), Cr);
+                    for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(1, q + SHIFT), Cr, digit_bias<S>());
                     store_digits8<S>(w, J.out1 + row * J.Kp1 + 8 * c, J.stride1);
                 }
             }
@@ -1138,7 +1144,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                 const SplitUnit u = P.units[ui];
                 // narrow units: one MMA per product, N = valid rows rounded up to 16
                 const bool narrow = u.n <= P.narrow && NT > 32;
-                const uint32_t idesc1 = idesc_bf16_f32(SP_M, narrow ? ((u.n + 15) & ~15) : NT);
+                const uint32_t idesc1 = idesc_f16_f32(SP_M, narrow ? ((u.n + 15) & ~15) : NT);
                 // accumulator set of this unit: the k-th use of set b is unit tile = k NBUF + b
                 const int buf = NBUF == 2 ? (tile & 1) : 0;
                 const uint32_t tacc = tmem + (uint32_t)(buf * 256);
@@ -1165,14 +1171,14 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                         if (narrow) {
 #pragma unroll
                             for (int t = 0; t < S - s; ++t)
-                                umma_bf16(tacc + (uint32_t)((s + t) * NT), as, db + (uint64_t)((t * B_TILE) >> 4),
+                                umma_f16(tacc + (uint32_t)((s + t) * NT), as, db + (uint64_t)((t * B_TILE) >> 4),
                                           idesc1, acc);
                         } else {
 #pragma unroll
                             for (int t = 0; t < S - s; t += GMAX) {
                                 const int g = (S - s - t) < GMAX ? (S - s - t) : GMAX;
-                                umma_bf16(tacc + (uint32_t)((s + t) * NT), as, db + (uint64_t)((t * B_TILE) >> 4),
-                                          idesc_bf16_f32(SP_M, g * NT), acc);
+                                umma_f16(tacc + (uint32_t)((s + t) * NT), as, db + (uint64_t)((t * B_TILE) >> 4),
+                                          idesc_f16_f32(SP_M, g * NT), acc);
                             }
                         }
                     }
@@ -1427,7 +1433,7 @@ int make_map(CUtensorMap* map, const void* base, long long rows, int Kp, int S, 
     cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)rows * Kp * 2};
     cuuint32_t box[3] = {16, (cuuint32_t)box_rows, (cuuint32_t)S};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ZEST_GPU_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(int(r)) + ")");
@@ -1460,7 +1466,7 @@ struct SliceArray {
         ZG_TRY(ex.ensure((size_t)r * 4 + 16));
         return ZEST_GPU_OK;
     }
-    __nv_bfloat16* ptr() const { return data.as<__nv_bfloat16>(); }
+    __half* ptr() const { return data.as<__half>(); }
 };
 
 // Sliced tables of one Zernike plan for one slice count.
