@@ -6,11 +6,11 @@
 // longer ones and the SH transforms take the FFT of fixed_fft.cu), the folded
 // Legendre sums and the radial sums -- is evaluated as
 //     C[r, n] = sum_k A[r, k] B[n, k]
-// with FP64 operands represented in BF16 fixed-point slices:
+// with FP64 operands represented in FP16 fixed-point slices:
 //   * each operand row gets an exponent e (|x| < 2^(e-1) over the row) and
 //     its values are rounded to v = round(x 2^{8S - e}) (ties away from zero);
 //   * v is cut into S balanced base-256 digits d_s in [-128, 127] (the
-//     leading one in [-128, 128]), each exact in BF16;
+//     leading one in [-128, 128]), each exact in FP16;
 //   * the products d_s(A) d_t(B) with s + t = level <= S - 1 (21 products at
 //     S = 6) accumulate in FP32 TMEM accumulators, one per level.  A product
 //     is at most 2^14, so a level with p products is exact while
@@ -28,13 +28,14 @@
 // loads (SWIZZLE_32B, one 16-wide K block of the S slices of both operands
 // per pipeline stage, the B slices back to back), warp 1 issues tcgen05.mma
 // (M = 128 operand rows; the products of one A slice with consecutive B
-// slices go to consecutive accumulators, so up to 256 / NT of them form one
-// MMA of N = g NT: 9 MMAs per K block at NT = 80), warps 2..17 read the
-// accumulators back (tcgen05.ld, four warps per TMEM lane quarter),
-// recombine and store through a stage-specific epilogue.  Six accumulators
-// of NT = 80 columns fill the 512 TMEM columns; with NT = 32 (or 16) two sets
-// fit, so that the next tile's MMAs overlap the drain.  For the SH sums the
-// table is the 128-row operand and the 2 x batch data rows are the columns.
+// slices go to consecutive accumulators, so up to 256 / W of them form one
+// MMA of N = g W, W the unit's table rows: 9 MMAs per K block at W = 80),
+// warps 2..17 read the accumulators back (tcgen05.ld, four warps per TMEM lane
+// quarter), recombine and store through a stage-specific epilogue.  Six
+// accumulators of 80 columns fill the 512 TMEM columns; those of two
+// consecutive narrower units fit together, and the MMAs of one then overlap
+// the drain of the other.  For the SH sums the table is the 128-row operand
+// and the 2 x batch data rows are the columns.
 // Every wait is bounded (about 2 s); on timeout the kernel records an error
 // code and winds down instead of hanging.
 #include <cuda.h>
@@ -65,7 +66,6 @@ namespace {
 constexpr int SP_EPI_WARPS = 16;                  // epilogue warps: four per TMEM lane quarter
 constexpr int SP_THREADS = 32 * (2 + SP_EPI_WARPS);  // + TMA producer + MMA issuer
 constexpr int SP_M = 128;
-constexpr int SP_MIXED = 1;      // narrow threshold value that selects mixed 80/32-column launches
 constexpr int SP_KB = 16;        // K elements per pipeline stage (32 bytes of FP16)
 constexpr long long SP_TIMEOUT_NS = 2000000000LL;
 
@@ -197,7 +197,7 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32(int M, int N) {
 }  // namespace
 
 // ===========================================================================
-// Slicing kernel: FP64 operand rows -> S BF16 digit slices + row exponents
+// Slicing kernel: FP64 operand rows -> S FP16 digit slices + row exponents
 // ===========================================================================
 namespace {
 
@@ -518,7 +518,8 @@ __device__ __forceinline__ constexpr long long digit_bias() {
 // that mask and one packed subtraction of 1152; one byte permute brings two
 // digits of two elements together.  5 integer operations an element (9 when
 // each digit was built as a float), which are what the slicing spends its time
-// on: at order 200 x 64 forward + backward SLICE_FIG.
+// on: at order 200 x 64 forward + backward 17.6 -> 17.2 ms,
+// most of which is now the memory's.
 template <int S>
 __device__ __forceinline__ void store_digits8(const unsigned long long (&u)[8], __half* out, long long stride) {
     constexpr uint32_t MAGIC = 0x64006400u;
@@ -568,7 +569,7 @@ __device__ __forceinline__ void load_staged(const Loader& ld, const typename Loa
 // one chunk of one row at a time: the chunk's values (and, for a shifted
 // second array, the next one) are rounded to the row's fixed-point grid once,
 // folded exactly in integers where requested, split into balanced 8-bit
-// digits and written as S BF16 slices, 16 bytes per slice and array.
+// digits and written as S FP16 slices, 16 bytes per slice and array.
 template <class Loader, int S>
 __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
     constexpr int MODE = Loader::MODE, SHIFT = Loader::SHIFT, NA = staged_arrays<Loader>();
@@ -740,7 +741,7 @@ struct SplitUnit {
     int a_row0;   // first operand row of the tile (row index inside the slice array)
     int a_rows;   // valid rows (<= 128)
     int b_row0;   // first table row
-    int n;        // valid table rows (<= NT)
+    int n;        // valid table rows (at most the tile width)
     int ksteps;   // 16-wide K blocks
     int flags;    // bit 0: A map, bit 1: B map, bit 2: parity / RMW
     int g;        // group (m or l)
@@ -1015,7 +1016,7 @@ struct SplitParams {
     int nunits;
     const int* ea[2];
     const int* eb[2];
-    int narrow;               // units of at most this many valid table rows run one MMA per product
+    int nst, stage;           // pipeline stages and their size in bytes
     int* err;
     int* host_err;            // mapped host word: each CTA copies a set flag there as it exits
     unsigned long long* dbg;  // optional cycle counters (null in normal use)
@@ -1031,11 +1032,18 @@ struct SplitParams {
 //
 // The products of one A slice s with the B slices t, t + 1, .. go to the
 // accumulators s + t, s + t + 1, ..: with the B slices of a stage stored one
-// after the other (NT rows each) and the accumulators NT columns apart, up to
-// 256 / NT of them are one MMA of N = g NT (9 MMAs per K block at S = 6,
-// NT = 80, instead of 21 of N = NT).  Each MMA reads its A tile once for g
+// after the other (W rows each) and the accumulators W columns apart, up to
+// 256 / W of them are one MMA of N = g W (9 MMAs per K block at S = 6,
+// W = 80, instead of 21 of N = W).  Each MMA reads its A tile once for g
 // products, which is what keeps the shared-memory reads per MAC low enough
 // for the tensor pipe.
+//
+// W is the unit's own width, its valid table rows rounded up to 16 (the least
+// step of N): the last tile of a sum, and the short sums of the triangular
+// stages, load, multiply and drain only the rows they have.  With every tile
+// 80 wide the 200 columns of an order-200 DFT cost 240; with this the GEMMs of
+// the transforms at order 200 x 64 take 30.0 ms instead of 31.4, and 1,024
+// transforms of orders 8 to 64 36.8 ms instead of 40.4.
 template <int S>
 struct Sched {
     static constexpr int NACC = S;                      // accumulators: levels 0..S-1
@@ -1044,43 +1052,46 @@ struct Sched {
 };
 static_assert(Sched<6>::PRODUCTS == 21 && Sched<4>::PRODUCTS == 10, "schedules");
 
-template <int S, int BITS, int NT>
-__host__ __device__ constexpr int stage_count() {
-    constexpr int st = S * 128 * 32 + Sched<S>::NB * NT * 32;
-    constexpr int n = (220 * 1024) / st;
-    return n > 6 ? 6 : n;
+// Widest tile: S accumulators of that many columns within the 512 of TMEM (two
+// sets of 64 for four slices).
+template <int S>
+__host__ __device__ constexpr int max_tile() {
+    return S == 6 ? 80 : S == 5 ? 96 : 64;
 }
+constexpr int SP_MAXW = 96;
+constexpr int SP_MAXST = 8;  // pipeline stages at most
+__host__ __device__ inline int tile_width(int n) { return (n + 15) & ~15; }
 
-template <int S, int BITS, int NT, class Epi>  // S slices of BITS-bit digits, NT table rows per tile
+// Tensor maps of one launch: the operand arrays (boxes of 128 rows) and the
+// table arrays, by box height: b[i][W / 16 - 1] brings W rows.
+struct SplitMaps {
+    CUtensorMap a[2];
+    CUtensorMap b[2][SP_MAXW / 16];
+};
+
+template <int S, class Epi>  // S slices of 8-bit digits
 __global__ void __launch_bounds__(SP_THREADS, 1)
-    split_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1,
-                      const __grid_constant__ CUtensorMap mapB0, const __grid_constant__ CUtensorMap mapB1,
-                      const SplitParams P, const Epi epi) {
+    split_gemm_kernel(const __grid_constant__ SplitMaps maps, const SplitParams P, const Epi epi) {
     using SC = Sched<S>;
-    static_assert(BITS == 8, "8-bit digits");
-    constexpr int NST = stage_count<S, BITS, NT>();
     constexpr int A_TILE = SP_M * 32;  // one slice, 16 K elements
-    constexpr int B_TILE = NT * 32;    // one slice of NT table rows: the B slices are contiguous
-    constexpr int STAGE = S * A_TILE + SC::NB * B_TILE;
-    constexpr uint32_t TX = S * (SP_M * 32) + SC::NB * (NT * 32);
-    constexpr int GMAX = 256 / NT;     // products of one A slice per MMA (N = g NT <= 256)
-    // every B tile is loaded whole; a unit of at most 32 valid table rows runs
-    // its 21 products as MMAs of N = its rows rounded up to 16, the others as
-    // grouped MMAs of full tiles
+    constexpr int NT = max_tile<S>();
     static_assert(SC::NACC * NT <= 512, "accumulators must fit in TMEM");
-    static_assert(NT % 16 == 0 && NT >= 16 && NT <= 128, "the MMA's N and the epilogue's 4-column loads");
-    static_assert(STAGE % 1024 == 0 && B_TILE % 256 == 0, "stage and tile alignment of the 32-byte swizzle");
-    // Two accumulator sets when they fit in TMEM (NT = 48): the MMAs of the
-    // next unit then run while the epilogue drains the previous one.
-    constexpr int NBUF = 2 * SC::NACC * NT <= 512 ? 2 : 1;
+    static_assert(NT % 16 == 0 && NT <= SP_MAXW, "tile widths are multiples of 16");
+    const int NST = P.nst, STAGE = P.stage;
 
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + NST * STAGE);
     uint64_t* empty = full + NST;
-    uint64_t* tfull = empty + NST;  // [NBUF]
-    uint64_t* tempty = tfull + 2;   // [NBUF]
+    uint64_t* tfull = empty + NST;  // [2]
+    uint64_t* tempty = tfull + 2;   // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    // Accumulators of this CTA's units alternate between the two ends of TMEM:
+    // unit i takes S W columns from the left (i even) or up to the right edge,
+    // and starts when unit i - 2 is drained, and also unit i - 1 where the two
+    // would overlap.  So the MMAs of narrow units (two of up to 42 columns
+    // together 85, at S = 6) run while the one before is drained.
+    auto acc_column = [](int tile, int W) { return (tile & 1) ? 512 - SC::NACC * W : 0; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long t_start = clock64();
@@ -1089,7 +1100,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        for (int b = 0; b < NBUF; ++b) {
+        for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
             mbar_init(&tempty[b], SP_EPI_WARPS);
         }
@@ -1107,24 +1118,29 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
-            int it = 0;
+            int it = 0, st = 0;  // copies issued; the next one's stage
+            uint32_t ph = 0;     // and the parity of its round through the stages
             bool ok = true;
             for (int ui = blockIdx.x; ui < P.nunits && ok; ui += gridDim.x) {
                 const SplitUnit u = P.units[ui];
-                const CUtensorMap* ma = (u.flags & 1) ? &mapA1 : &mapA0;
-                const CUtensorMap* mb = (u.flags & 2) ? &mapB1 : &mapB0;
+                const int W = tile_width(u.n);
+                const CUtensorMap* ma = &maps.a[u.flags & 1];
+                const CUtensorMap* mb = &maps.b[(u.flags >> 1) & 1][W / 16 - 1];
+                const uint32_t tx = (uint32_t)(S * (SP_M + W) * 32);
                 for (int kb = 0; kb < u.ksteps; ++kb, ++it) {
-                    const int st = it % NST;
-                    const uint32_t ph = (it / NST) & 1;
                     const long long w0 = clock64();
                     if (!mbar_wait(&empty[st], ph ^ 1, P.err, 1)) { ok = false; break; }
                     if (P.dbg) atomicAdd(&P.dbg[0], (unsigned long long)(clock64() - w0));
-                    mbar_expect_tx(&full[st], TX);
+                    mbar_expect_tx(&full[st], tx);
                     unsigned char* sa = smem + st * STAGE;
                     unsigned char* sb = sa + S * A_TILE;
-                    // one box per operand: the S slices of 128 rows (A) and of NT rows (B)
+                    // one box per operand: the S slices of 128 rows (A) and of W rows (B)
                     tma_load_3d(sa, ma, &full[st], (u.k0 + kb) * SP_KB, u.a_row0, 0);
                     tma_load_3d(sb, mb, &full[st], (u.k0 + kb) * SP_KB, u.b_row0, 0);
+                    if (++st == NST) {
+                        st = 0;
+                        ph ^= 1;
+                    }
                 }
             }
             // drain: wait (bounded) for the copies this thread issued
@@ -1138,66 +1154,80 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            int it = 0, tile = 0;
+            int tile = 0, st = 0, Wp = 0;  // Wp: width of the unit before
+            uint32_t ph = 0;
             bool ok = true;
             for (int ui = blockIdx.x; ui < P.nunits && ok; ui += gridDim.x, ++tile) {
                 const SplitUnit u = P.units[ui];
-                // narrow units: one MMA per product, N = valid rows rounded up to 16
-                const bool narrow = u.n <= P.narrow && NT > 32;
-                const uint32_t idesc1 = idesc_f16_f32(SP_M, narrow ? ((u.n + 15) & ~15) : NT);
-                // accumulator set of this unit: the k-th use of set b is unit tile = k NBUF + b
-                const int buf = NBUF == 2 ? (tile & 1) : 0;
-                const uint32_t tacc = tmem + (uint32_t)(buf * 256);
+                const int W = tile_width(u.n);
+                const int side = tile & 1;
+                const uint32_t tacc = tmem + (uint32_t)acc_column(tile, W);
                 const long long w0 = clock64();
-                if (!mbar_wait(&tempty[buf], ((tile / NBUF) & 1) ^ 1, P.err, 2)) { ok = false; break; }
+                // the k-th use of a side is unit 2 k + side
+                if (!mbar_wait(&tempty[side], ((tile >> 1) & 1) ^ 1, P.err, 2)) { ok = false; break; }
+                if (tile > 0 && SC::NACC * (W + Wp) > 512 &&
+                    !mbar_wait(&tempty[side ^ 1], ((tile - 1) >> 1) & 1, P.err, 2)) { ok = false; break; }
+                Wp = W;
                 if (P.dbg) atomicAdd(&P.dbg[1], (unsigned long long)(clock64() - w0));
                 tc_fence_after();
-                for (int kb = 0; kb < u.ksteps; ++kb, ++it) {
-                    const int st = it % NST;
-                    const uint32_t ph = (it / NST) & 1;
-                    const long long w1 = clock64();
-                    if (!mbar_wait(&full[st], ph, P.err, 3)) { ok = false; break; }
-                    if (P.dbg) atomicAdd(&P.dbg[2], (unsigned long long)(clock64() - w1));
-                    tc_fence_after();
-                    // descriptors differ only in the start-address field (address >> 4)
-                    const uint64_t da = desc_sw32(smem_u32(smem + st * STAGE));
-                    const uint64_t db = da + (uint64_t)((S * A_TILE) >> 4);
-                    // A slice 0 comes first: its products start every accumulator
-                    // (levels 0..S-1) in the first K block, all later ones add
+                // all K blocks of a unit, for its width as a constant: one thread
+                // issues, and the MMAs wait for it where it has more to compute
+                // than the precomputed steps of an unrolled list
+                auto issue = [&](auto width) {
+                    constexpr int CWD = decltype(width)::value;
+                    constexpr int G = 256 / CWD;  // products of one A slice per MMA (N = g W <= 256)
+                    for (int kb = 0; kb < u.ksteps; ++kb) {
+                        const long long w1 = P.dbg ? clock64() : 0;
+                        if (!mbar_wait(&full[st], ph, P.err, 3)) { ok = false; break; }
+                        if (P.dbg) atomicAdd(&P.dbg[2], (unsigned long long)(clock64() - w1));
+                        tc_fence_after();
+                        // descriptors differ only in the start-address field (address >> 4)
+                        const uint64_t da = desc_sw32(smem_u32(smem + st * STAGE));
+                        const uint64_t db = da + (uint64_t)((S * A_TILE) >> 4);
+                        // A slice 0 comes first: its products start every accumulator
+                        // (levels 0..S-1) in the first K block, all later ones add
 #pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        const uint32_t acc = (kb > 0 || s > 0) ? 1u : 0u;
-                        const uint64_t as = da + (uint64_t)((s * A_TILE) >> 4);
-                        if (narrow) {
+                        for (int s = 0; s < S; ++s) {
+                            const uint32_t acc = (kb > 0 || s > 0) ? 1u : 0u;
+                            const uint64_t as = da + (uint64_t)((s * A_TILE) >> 4);
 #pragma unroll
-                            for (int t = 0; t < S - s; ++t)
-                                umma_f16(tacc + (uint32_t)((s + t) * NT), as, db + (uint64_t)((t * B_TILE) >> 4),
-                                          idesc1, acc);
-                        } else {
-#pragma unroll
-                            for (int t = 0; t < S - s; t += GMAX) {
-                                const int g = (S - s - t) < GMAX ? (S - s - t) : GMAX;
-                                umma_f16(tacc + (uint32_t)((s + t) * NT), as, db + (uint64_t)((t * B_TILE) >> 4),
-                                          idesc_f16_f32(SP_M, g * NT), acc);
+                            for (int t = 0; t < S - s; t += G) {
+                                const int g = (S - s - t) < G ? (S - s - t) : G;
+                                umma_f16(tacc + (uint32_t)((s + t) * CWD), as, db + (uint64_t)((t * CWD * 32) >> 4),
+                                         idesc_f16_f32(SP_M, g * CWD), acc);
                             }
                         }
+                        umma_commit(&empty[st]);
+                        if (++st == NST) {
+                            st = 0;
+                            ph ^= 1;
+                        }
                     }
-                    umma_commit(&empty[st]);
+                };
+                switch (W) {
+                case 16: issue(std::integral_constant<int, 16>{}); break;
+                case 32: issue(std::integral_constant<int, 32>{}); break;
+                case 48: issue(std::integral_constant<int, 48>{}); break;
+                case 64: issue(std::integral_constant<int, 64>{}); break;
+                case 80: if constexpr (NT >= 80) issue(std::integral_constant<int, 80>{}); break;
+                case 96: if constexpr (NT >= 96) issue(std::integral_constant<int, 96>{}); break;
                 }
-                if (ok) umma_commit(&tfull[buf]);
+                if (ok) umma_commit(&tfull[side]);
             }
         }
         __syncwarp();
     } else {
         // ---------------- epilogue ----------------
         const int q = warp & 3;              // TMEM lane quarter of this warp
-        constexpr int CW = NT / (SP_EPI_WARPS / 4);  // columns per epilogue warp
-        static_assert(CW % 4 == 0 && CW <= 64, "epilogue column split");
+        constexpr int CW = NT / (SP_EPI_WARPS / 4);  // columns per epilogue warp, at most
+        static_assert(SP_EPI_WARPS == 16 && CW % 4 == 0 && CW <= 32, "epilogue column split");
         const int part = (warp - 2) >> 2;    // which column part
-        const int col0 = part * CW;
         int tile = 0;
         for (int ui = blockIdx.x; ui < P.nunits; ui += gridDim.x, ++tile) {
             const SplitUnit u = P.units[ui];
+            const int W = tile_width(u.n);
+            const int cw = W >> 2;           // columns of each part (a multiple of 4)
+            const int col0 = part * cw;
             const int r = 32 * q + lane;
             const bool rv = r < u.a_rows;
             const int row = u.a_row0 + (rv ? r : 0);
@@ -1206,15 +1236,12 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             const int* __restrict__ eav = amap ? P.ea[1] : P.ea[0];
             const int* __restrict__ ebv = bmap ? P.eb[1] : P.eb[0];
             const int ea = eav[row];
-            // NT/2 <= 64 columns per warp: lane l holds the exponents of columns col0 + l and col0 + 32 + l
-            const int ca = col0 + lane, cb = col0 + 32 + lane;
-            const int eb_a = (ca < col0 + CW && ca < u.n) ? ebv[u.b_row0 + ca] : 0;
-            const int eb_b = (CW > 32 && cb < col0 + CW && cb < u.n) ? ebv[u.b_row0 + cb] : 0;
+            const int eb_a = (lane < cw && col0 + lane < u.n) ? ebv[u.b_row0 + col0 + lane] : 0;
             const typename Epi::Row R = epi.row(u, row);
-            const int buf = NBUF == 2 ? (tile & 1) : 0;
-            const uint32_t tacc = tmem + (uint32_t)(buf * 256);
+            const int side = tile & 1;
+            const uint32_t tacc = tmem + (uint32_t)acc_column(tile, W);
             const long long w0 = clock64();
-            const bool got = mbar_wait(&tfull[buf], (tile / NBUF) & 1, P.err, 4);
+            const bool got = mbar_wait(&tfull[side], (tile >> 1) & 1, P.err, 4);
             const long long w1 = clock64();
             if (!__all_sync(0xffffffffu, got)) break;
             tc_fence_after();
@@ -1234,10 +1261,11 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             if (active) {
 #pragma unroll
             for (int c = 0; c < CW / 4; ++c) {
+                if (4 * c >= cw) break;
                 uint32_t v[SC::NACC][4];
 #pragma unroll
                 for (int a = 0; a < SC::NACC; ++a)
-                    tmem_ld4(tacc + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * NT + col0 + 4 * c), v[a]);
+                    tmem_ld4(tacc + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * W + col0 + 4 * c), v[a]);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -1267,12 +1295,13 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             tc_fence_before();
             __syncwarp();
             const long long w2 = clock64();
-            if (lane == 0) mbar_arrive(&tempty[buf]);
+            if (lane == 0) mbar_arrive(&tempty[side]);
             // phase 2 (overlaps the next tile's MMAs): FP64 results and stores
             if constexpr (raw_epi<Epi>::value) {
             if (active) {
 #pragma unroll
             for (int c = 0; c < CW / 4; ++c) {
+                if (4 * c >= cw) break;
                 long long oldr[4] = {0, 0, 0, 0};
                 if constexpr (Epi::RMW) {
                     if (rv) {
@@ -1285,14 +1314,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                 for (int j = 0; j < 4; ++j) {
                     const int n = col0 + 4 * c + j;
                     const int idx = 4 * c + j;
-                    int eb;
-                    if constexpr (CW <= 32) {
-                        eb = __shfl_sync(0xffffffffu, eb_a, idx);
-                    } else {
-                        const int e1 = __shfl_sync(0xffffffffu, eb_a, idx & 31);
-                        const int e2 = __shfl_sync(0xffffffffu, eb_b, idx & 31);
-                        eb = idx < 32 ? e1 : e2;
-                    }
+                    const int eb = __shfl_sync(0xffffffffu, eb_a, idx);
                     if (rv && n < u.n) epi.store_raw(R, u, n, T[4 * c + j], ea + eb + TEXP, oldr[j]);
                 }
             }
@@ -1301,6 +1323,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             if (active) {
 #pragma unroll
             for (int c = 0; c < CW / 4; ++c) {
+                if (4 * c >= cw) break;
                 double old[4][2];
                 double vv[4];  // pair-row epilogues: this row's values of the four columns
                 if constexpr (Epi::RMW) {
@@ -1314,14 +1337,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                 for (int j = 0; j < 4; ++j) {
                     const int n = col0 + 4 * c + j;
                     const int idx = 4 * c + j;
-                    int eb;
-                    if constexpr (CW <= 32) {
-                        eb = __shfl_sync(0xffffffffu, eb_a, idx);
-                    } else {
-                        const int e1 = __shfl_sync(0xffffffffu, eb_a, idx & 31);
-                        const int e2 = __shfl_sync(0xffffffffu, eb_b, idx & 31);
-                        eb = idx < 32 ? e1 : e2;
-                    }
+                    const int eb = __shfl_sync(0xffffffffu, eb_a, idx);
                     if constexpr (pair_rows_epi<Epi>::value) {
                         // rows 2i and 2i + 1 are the two halves of one 16-byte
                         // pair at every column: neighbouring lanes swap one
@@ -1388,11 +1404,7 @@ __global__ void wait_expiry_kernel(int* err, int* host_err, long long limit_ns) 
     }
 }
 
-template <int S, int BITS, int NT>
-constexpr size_t split_smem_bytes() {
-    constexpr int NST = stage_count<S, BITS, NT>();
-    return (size_t)NST * (S * SP_M * 32 + Sched<S>::NB * NT * 32) + 1024 + 256;
-}
+constexpr int SP_SMEM = 220 * 1024;  // stages; beside them alignment and barriers
 
 }  // namespace
 
@@ -1422,7 +1434,7 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// [S][rows][Kp] bf16 slice array -> 3D map (Kp, rows, S), box (16, box_rows,
+// [S][rows][Kp] FP16 slice array -> 3D map (Kp, rows, S), box (16, box_rows,
 // S), 32B swizzle: one copy brings a tile of every slice, the slices one
 // after the other in shared memory (rows past the array's end read as 0)
 int make_map(CUtensorMap* map, const void* base, long long rows, int Kp, int S, int box_rows) {
@@ -1442,13 +1454,12 @@ int make_map(CUtensorMap* map, const void* base, long long rows, int Kp, int S, 
 
 inline int r16(int k) { return (k + 15) & ~15; }
 
-// table rows per tile: S accumulators of NT columns within the 512 TMEM columns
-// (6 x 80, 5 x 96, 4 x 64 with two accumulator sets)
-int n_tile(int S) { return S == 6 ? 80 : S == 5 ? 96 : 64; }
+// table rows per tile at most
+int n_tile(int S) { return S == 6 ? max_tile<6>() : S == 5 ? max_tile<5>() : max_tile<4>(); }
 
 }  // namespace
 
-// Slice arrays of one operand: [copies * S][rows][Kp] bf16 + per-row exponents
+// Slice arrays of one operand: [copies * S][rows][Kp] FP16 + per-row exponents
 // (the GEMMs read one copy: every level has its own accumulator).
 struct SliceArray {
     DevBuf data, ex;
@@ -1501,12 +1512,10 @@ struct StSplitTables {
 struct UnitList {
     std::vector<SplitUnit> v;
     int max_ksteps = 0;   // longest sum of a unit, in 16-wide K blocks
+    unsigned widths = 0;  // tile widths W of the units: bit W / 16 - 1
     double useful = 0.0;  // 2 * rows * table rows * K * products, valid tiles only
-    double issued = 0.0;  // the same for full 128 x NT x 16k tiles
+    double issued = 0.0;  // the same for full 128 x W x 16k tiles
     DevBuf dev;
-    // mixed launches: the units of more than 32 valid table rows (80-column
-    // tiles) and the others (32-column tiles), split on first use
-    std::unique_ptr<UnitList> wide, narrow;
 };
 
 struct SplitState {
@@ -1524,9 +1533,7 @@ struct SplitState {
     DevBuf tmp;                 // FP64 staging of generated tables
     DevBuf cycles;              // role wait counters, kept when ZEST_GPU_SPLIT_CYCLES is set
     bool cycles_on = false;
-    int narrow = 32;            // widest unit (valid table rows) run as one MMA per product
-    bool narrow_fixed = false;  // set by the tuning override: the autotuner keeps it
-    // timed choice per (stage, Lg, Lm, batch): column tile | narrow threshold << 8
+    // timed choice per (stage, Lg, Lm, batch): column tile
     std::map<std::tuple<int, int, int, int>, int> tuned;
     int nt[16];                 // column tile of each work-list stage: 0 = chosen per launch, or 32 / 80
     SplitState();
@@ -1649,20 +1656,6 @@ int get_state(zest_gpu_context* ctx, SplitState** out) {
     if (!ctx->split) {
         ctx->split.reset(new SplitState());
         ctx->split->cycles_on = std::getenv("ZEST_GPU_SPLIT_CYCLES") != nullptr;
-        // tuning override: units of at most this many valid table rows (16..64)
-        // issue one MMA per product instead of grouped full-width MMAs
-        if (const char* e = std::getenv("ZEST_GPU_SPLIT_NARROW")) {
-            // "mixed": units of up to 32 rows in a second launch of 32-column tiles
-            const int v = std::string(e) == "mixed" ? SP_MIXED : std::atoi(e);
-            if (v == SP_MIXED) {
-                ctx->split->narrow = SP_MIXED;
-                ctx->split->narrow_fixed = true;
-            }
-            if (v >= 16 && v <= 64) {
-                ctx->split->narrow = v;
-                ctx->split->narrow_fixed = true;
-            }
-        }
         // tuning override of the column tiles, "stage=nt,..." with stage one of
         // dft_f leg_f rad_f rad_b leg_b dft_b and nt 32 or 80
         if (const char* e = std::getenv("ZEST_GPU_SPLIT_NT")) {
@@ -1861,7 +1854,7 @@ int build_zt_tables(zest_gpu_context* ctx, SplitState* st, ZtPlan& plan, int S, 
     return ZEST_GPU_OK;
 }
 
-template <int S, int BITS, int NT, class Epi>
+template <int S, class Epi>
 int run_gemm_t(zest_gpu_context* ctx, UnitList& ul, const SliceArray& A0, const SliceArray& A1, const SliceArray& B0,
                const SliceArray& B1, const Epi& epi) {
     const std::vector<SplitUnit>& units = ul.v;
@@ -1869,18 +1862,28 @@ int run_gemm_t(zest_gpu_context* ctx, UnitList& ul, const SliceArray& A0, const 
     SplitState* st;
     ZG_TRY(get_state(ctx, &st));
     cudaStream_t s = ctx->stream;
-    CUtensorMap ma0, ma1, mb0, mb1;
     if (A0.copies != 1 || A1.copies != 1 || B0.copies != 1 || B1.copies != 1)
         return fail(ZEST_GPU_ERR_INVALID, "split GEMM: operands must hold one copy of their slices");
-    // the FP32 level sums stay exact only up to these lengths
-    if (ul.max_ksteps * SP_KB > (BITS == 8 ? SL_K8MAX : SL_KMAX))
+    if (A0.bits != 8 || A1.bits != 8 || B0.bits != 8 || B1.bits != 8)
+        return fail(ZEST_GPU_ERR_INVALID, "split GEMM: operands need 8-bit digits");
+    // the FP32 level sums stay exact only up to this length
+    if (ul.max_ksteps * SP_KB > SL_K8MAX)
         return fail(ZEST_GPU_ERR_INVALID, "split GEMM: sum too long for exact level sums");
     if (A0.S != S || A1.S != S || B0.S != S || B1.S != S)
         return fail(ZEST_GPU_ERR_INVALID, "split GEMM: operands sliced with another slice count");
-    ZG_TRY(make_map(&ma0, A0.ptr(), A0.rows, A0.Kp, S, SP_M));
-    ZG_TRY(make_map(&ma1, A1.ptr(), A1.rows, A1.Kp, S, SP_M));
-    ZG_TRY(make_map(&mb0, B0.ptr(), B0.rows, B0.Kp, S, NT));
-    ZG_TRY(make_map(&mb1, B1.ptr(), B1.rows, B1.Kp, S, NT));
+    SplitMaps maps = {};
+    ZG_TRY(make_map(&maps.a[0], A0.ptr(), A0.rows, A0.Kp, S, SP_M));
+    if (&A1 == &A0) maps.a[1] = maps.a[0];
+    else ZG_TRY(make_map(&maps.a[1], A1.ptr(), A1.rows, A1.Kp, S, SP_M));
+    int maxw = 0;
+    for (int w = 0; w < SP_MAXW / 16; ++w) {
+        if (!(ul.widths >> w & 1)) continue;
+        maxw = 16 * (w + 1);
+        ZG_TRY(make_map(&maps.b[0][w], B0.ptr(), B0.rows, B0.Kp, S, maxw));
+        if (&B1 == &B0) maps.b[1][w] = maps.b[0][w];
+        else ZG_TRY(make_map(&maps.b[1][w], B1.ptr(), B1.rows, B1.Kp, S, maxw));
+    }
+    if (maxw > max_tile<S>()) return fail(ZEST_GPU_ERR_INVALID, "split GEMM: tile too wide");
     if (!ul.dev.p) {  // work lists are uploaded once and cached with their key
         ZG_TRY(ul.dev.ensure(units.size() * sizeof(SplitUnit)));
         ZG_CUDA_TRY(cudaMemcpyAsync(ul.dev.p, units.data(), units.size() * sizeof(SplitUnit),
@@ -1899,16 +1902,17 @@ int run_gemm_t(zest_gpu_context* ctx, UnitList& ul, const SliceArray& A0, const 
     P.eb[1] = B1.ex.as<int>();
     P.err = st->err.as<int>();
     P.host_err = st->host_err_dev;
-    P.narrow = st->narrow;
+    P.stage = (S * (SP_M + maxw) * 32 + 1023) & ~1023;
+    P.nst = std::min(SP_MAXST, SP_SMEM / P.stage);
     P.dbg = nullptr;
     if (st->cycles_on) {
         ZG_TRY(st->cycles.ensure(8 * sizeof(unsigned long long)));
         ZG_CUDA_TRY(cudaMemsetAsync(st->cycles.p, 0, 8 * sizeof(unsigned long long), s));
         P.dbg = st->cycles.as<unsigned long long>();
     }
-    const size_t smem = split_smem_bytes<S, BITS, NT>();
-    ZG_TRY(set_attributes_once(split_gemm_kernel<S, BITS, NT, Epi>, [smem](auto k) -> int {
-        ZG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = (size_t)P.nst * P.stage + 1024 + 256;
+    ZG_TRY(set_attributes_once(split_gemm_kernel<S, Epi>, [](auto k) -> int {
+        ZG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM + 1024 + 256));
         return ZEST_GPU_OK;
     }));
     int nsm = 0;
@@ -1916,7 +1920,7 @@ int run_gemm_t(zest_gpu_context* ctx, UnitList& ul, const SliceArray& A0, const 
     const int grid = std::min<int>(int(units.size()), nsm);
     {
         StageScope sc(ctx, ST_SPLIT_GEMM);
-        split_gemm_kernel<S, BITS, NT, Epi><<<grid, SP_THREADS, smem, s>>>(ma0, ma1, mb0, mb1, P, epi);
+        split_gemm_kernel<S, Epi><<<grid, SP_THREADS, smem, s>>>(maps, P, epi);
         ZG_TRY(launch_check("split_gemm_kernel"));
     }
     // A bounded-wait timeout reaches the caller through split_finish at the end
@@ -1929,9 +1933,9 @@ int run_gemm_t(zest_gpu_context* ctx, UnitList& ul, const SliceArray& A0, const 
         const char* fn = __PRETTY_FUNCTION__;
         const char* tag = std::strstr(fn, "Epi = ");
         std::fprintf(stderr,
-                     "split_gemm S=%d NT=%d %.40s units=%zu grid=%d: total %.0f | producer waits %.0f | mma waits "
+                     "split_gemm S=%d W<=%d %.40s units=%zu grid=%d: total %.0f | producer waits %.0f | mma waits "
                      "tmem %.0f, smem %.0f | epilogue waits %.0f, drains %.0f, stores %.0f (cycles per CTA)\n",
-                     S, NT, tag ? tag + 6 : "", units.size(), grid, double(c[5]) / grid, double(c[0]) / grid,
+                     S, maxw, tag ? tag + 6 : "", units.size(), grid, double(c[5]) / grid, double(c[0]) / grid,
                      double(c[1]) / grid,
                      double(c[2]) / grid, double(c[3]) / grid, double(c[4]) / grid, double(c[6]) / grid);
     }
@@ -1962,44 +1966,16 @@ int get_units(zest_gpu_context* ctx, std::tuple<int, int, int, int, int, int> ke
     return ZEST_GPU_OK;
 }
 
-// The split GEMM of a work list, its column tile NT chosen at run time: with
-// six slices 80 (one accumulator set) or 32 (two sets, so that the next
-// unit's MMAs overlap the epilogue's drain); five slices use 96 and four 64.
-// Later K-chunks of long sums need six slices.
+// The split GEMM of a work list.  Later K-chunks of long sums need six slices.
 template <class Epi>
-int run_gemm_nt(zest_gpu_context* ctx, int nt, int S, UnitList& ul, const SliceArray& A0, const SliceArray& A1,
-                const SliceArray& B0, const SliceArray& B1, const Epi& epi) {
-    const int bits = A0.bits;
-    if (A1.bits != bits || B0.bits != bits || B1.bits != bits)
-        return fail(ZEST_GPU_ERR_INVALID, "split GEMM: operands sliced with different digit widths");
-    if (bits != 8) return fail(ZEST_GPU_ERR_INVALID, "split GEMM: operands need 8-bit digits");
+int run_gemm(zest_gpu_context* ctx, int S, UnitList& ul, const SliceArray& A0, const SliceArray& A1,
+             const SliceArray& B0, const SliceArray& B1, const Epi& epi) {
     if (Epi::CHUNK && S != 6)
         return fail(ZEST_GPU_ERR_UNSUPPORTED, "split path: sums longer than 256 terms need 6 slices");
-    SplitState* st;
-    ZG_TRY(get_state(ctx, &st));
-    if (S == 6 && nt == 80 && st->narrow == SP_MIXED) {
-        // mixed: units of at most 32 valid table rows run in a second launch of
-        // 32-column tiles (one MMA per A slice over all levels), the others in
-        // 80-column tiles; the two launches write disjoint outputs
-        if (!ul.wide) {
-            ul.wide.reset(new UnitList());
-            ul.narrow.reset(new UnitList());
-            for (const SplitUnit& u : ul.v) (u.n <= 32 ? ul.narrow : ul.wide)->v.push_back(u);
-            ul.wide->max_ksteps = ul.narrow->max_ksteps = ul.max_ksteps;
-        }
-        if (ctx->prof.on) {  // the halves carry no flop counts of their own
-            st->useful_flops += ul.useful;
-            st->issued_flops += ul.issued;
-        }
-        const int rc = run_gemm_t<6, 8, 80>(ctx, *ul.wide, A0, A1, B0, B1, epi);
-        if (rc != ZEST_GPU_OK) return rc;
-        return run_gemm_t<6, 8, 32>(ctx, *ul.narrow, A0, A1, B0, B1, epi);
-    }
     switch (S) {
-    case 6: return nt == 32 ? run_gemm_t<6, 8, 32>(ctx, ul, A0, A1, B0, B1, epi)
-                            : run_gemm_t<6, 8, 80>(ctx, ul, A0, A1, B0, B1, epi);
-    case 5: return run_gemm_t<5, 8, 96>(ctx, ul, A0, A1, B0, B1, epi);
-    case 4: return run_gemm_t<4, 8, 64>(ctx, ul, A0, A1, B0, B1, epi);
+    case 6: return run_gemm_t<6>(ctx, ul, A0, A1, B0, B1, epi);
+    case 5: return run_gemm_t<5>(ctx, ul, A0, A1, B0, B1, epi);
+    case 4: return run_gemm_t<4>(ctx, ul, A0, A1, B0, B1, epi);
     }
     return fail(ZEST_GPU_ERR_UNSUPPORTED, "split path supports 4..6 slices");
 }
@@ -2019,60 +1995,48 @@ void add_units(UnitList& ul, int S, int bits, long long a0, long long arows, int
             u.b_row0 = b0 + c;
             u.n = std::min(NT, nrows - c);
             u.ksteps = ksteps;
-            // a unit of at most 32 valid rows runs N = its rows rounded up to 16
-            const int ncols = (u.n <= 32 && NT > 32) ? r16(u.n) : NT;
+            const int W = tile_width(u.n);
+            ul.widths |= 1u << (W / 16 - 1);
             u.flags = flags;
             u.g = g;
             u.aux = c;
             u.k0 = k0 / 16;
             ul.v.push_back(u);
             ul.useful += 2.0 * u.a_rows * u.n * kk * P;
-            ul.issued += 2.0 * SP_M * ncols * 16.0 * ksteps * P;
+            ul.issued += 2.0 * SP_M * W * 16.0 * ksteps * P;
         }
 }
 
 
-// Column tile of a stage's launches with six slices, also part of the
-// work-list key; ncols = the most table rows a group of the stage has.
+// Widest column tile of a stage's launches, also part of the work-list key;
+// ncols = the most table rows a group of the stage has.
 //   * 32 where no group has more than 32 columns (the small orders of a
-//     ragged batch): two accumulator sets, and an 80-wide tile would be at
-//     least 60% empty;
-//   * 80 otherwise: one set of six 80-column accumulators, MMAs of up to
-//     three products (N = 240).
+//     ragged batch);
+//   * as wide as TMEM takes otherwise: the fewest reads of the operand rows.
 // A tuning override (ZEST_GPU_SPLIT_NT) can pin a stage to 32 or 80.
 inline int stage_nt(const SplitState* st, int wk, int S, int ncols) {
     if (S != 6) return n_tile(S);
     if (st->nt[wk]) return st->nt[wk];
     return ncols <= 32 ? 32 : 80;
 }
-inline int nt_pass(int nt) { return nt == 32 ? 1 << 16 : 0; }
+inline int nt_pass(int nt) { return nt << 16; }
 
-// Runs one split GEMM stage, `launch(nt)`, with its column tile and narrow
-// threshold: a tuning override (ZEST_GPU_SPLIT_NT) if set; else, with the
-// context's autotuner on, outside graph capture and for a stage whose
-// launches overwrite their outputs (single sums), the fastest of the
-// candidates (80 columns with units of up to 32, 48 or 64 valid table rows
-// issued as one MMA per product; 80 columns with the units of up to 32 rows
-// in a second launch of 32-column tiles; or 32 columns), timed with CUDA events on
-// the context stream at the stage's first run at this size (each candidate
-// once untimed, then once timed; neither choice changes a result); else the
-// rule of stage_nt.
+// Runs one split GEMM stage, `launch(nt)`, with its column tile: a tuning
+// override (ZEST_GPU_SPLIT_NT) if set; else, with the context's autotuner on,
+// outside graph capture and for a stage whose launches overwrite their outputs
+// (single sums), the fastest of the candidates (narrower tiles overlap more of
+// the drain of the one before, wider ones read the operand rows less often),
+// timed with CUDA events on the context stream at the stage's first run at
+// this size (each candidate once untimed, then once timed; no choice changes a
+// result); else the rule of stage_nt.
 template <class Launch>
 int tuned_stage(zest_gpu_context* ctx, SplitState* st, int wk, int S, int Lg, int Lm, int batch, int ncols,
                 bool idempotent, Launch&& launch) {
-    int nt = stage_nt(st, wk, S, ncols);
+    const int nt = stage_nt(st, wk, S, ncols);
     if (S != 6 || st->nt[wk] || !ctx->autotune || !idempotent) return launch(nt);
-    const int narrow0 = st->narrow;
-    // runs candidate (t, w): tile t, narrow threshold w
-    auto run = [&](int t, int w) -> int {
-        st->narrow = w;
-        const int rc = launch(t);
-        st->narrow = narrow0;
-        return rc;
-    };
     const auto key = std::make_tuple(wk, Lg, Lm, batch);
     auto it = st->tuned.find(key);
-    if (it != st->tuned.end()) return run(it->second & 0xFF, it->second >> 8);
+    if (it != st->tuned.end()) return launch(it->second);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     ZG_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &cap));
     if (cap != cudaStreamCaptureStatusNone) return launch(nt);
@@ -2081,25 +2045,23 @@ int tuned_stage(zest_gpu_context* ctx, SplitState* st, int wk, int S, int Lg, in
     ZG_CUDA_TRY(cudaEventCreate(&e1));
     const bool prof = ctx->prof.on;  // the timing runs stay out of the stage profile
     ctx->prof.on = false;
-    const int cand[5][2] = {{80, 32}, {80, 48}, {80, 64}, {80, SP_MIXED}, {32, 32}};
     float best = 0.0f;
-    int choice = nt | (narrow0 << 8);
+    int choice = nt;
     int rc = ZEST_GPU_OK;
-    for (int i = 0; i < 5 && rc == ZEST_GPU_OK; ++i) {
-        // one tile of at most 32 columns: the thresholds agree; a fixed threshold is kept
-        if (i > 0 && i < 4 && (ncols <= 32 || st->narrow_fixed)) continue;
-        const int w = st->narrow_fixed ? narrow0 : cand[i][1];
-        rc = run(cand[i][0], w);
+    for (int t : {80, 64, 48, 32}) {
+        if (tile_width(ncols) < t && t > 32) continue;  // the same units as a narrower candidate's
+        rc = launch(t);
         if (rc == ZEST_GPU_OK && cudaEventRecord(e0, ctx->stream) != cudaSuccess) rc = fail(ZEST_GPU_ERR_CUDA, "event");
-        if (rc == ZEST_GPU_OK) rc = run(cand[i][0], w);
+        if (rc == ZEST_GPU_OK) rc = launch(t);
         if (rc == ZEST_GPU_OK && cudaEventRecord(e1, ctx->stream) != cudaSuccess) rc = fail(ZEST_GPU_ERR_CUDA, "event");
         float ms = 0.0f;
         if (rc == ZEST_GPU_OK &&
             (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess))
             rc = fail(ZEST_GPU_ERR_CUDA, "split tile autotuner: timing failed");
-        if (rc == ZEST_GPU_OK && (i == 0 || ms < best)) {
+        if (rc != ZEST_GPU_OK) break;
+        if (best == 0.0f || ms < best) {
             best = ms;
-            choice = cand[i][0] | (w << 8);
+            choice = t;
         }
     }
     ctx->prof.on = prof;
@@ -2107,7 +2069,7 @@ int tuned_stage(zest_gpu_context* ctx, SplitState* st, int wk, int S, int Lg, in
     cudaEventDestroy(e1);
     if (rc != ZEST_GPU_OK) return rc;
     st->tuned.emplace(key, choice);
-    return run(choice & 0xFF, choice >> 8);
+    return launch(choice);
 }
 
 // Longitude DFT of `batch` grids x[b][lon][col] (C columns, item stride gsz) of
@@ -2134,7 +2096,7 @@ int dft_forward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t,
                 if (Lm > 1) add_units(ul, S, bits, r, rr, 0, Lm - 1, NT, Lg - 1, 1 | 2, 0);
             }
         }, &u));
-        return run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], t.cos_f, t.sin_f, EpiDftFwd{G, C, Lg});
+        return run_gemm(ctx, S, *u, st->op[0], st->op[1], t.cos_f, t.sin_f, EpiDftFwd{G, C, Lg});
     });
 }
 
@@ -2161,7 +2123,7 @@ int dft_backward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t
             for (long long r = 0; r < rows; r += SP_M)
                 add_units(ul, S, bits, r, std::min<long long>(SP_M, rows - r), 0, Lg, NT, Lg, 0, 0, 0);
         }, &u));
-        ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], t.cos_bj, t.sin_bj,
+        ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[1], t.cos_bj, t.sin_bj,
                            EpiDftBwdCosRaw{grids, Ts, C, N, Lg, gsz}));
         UnitList* v;
         ZG_TRY(get_units(ctx, std::make_tuple(int(WK_DFT_B), Lg, Lm, batch, S, 5 + nt_pass(NT)), [&](UnitList& ul) {
@@ -2169,7 +2131,7 @@ int dft_backward_stage(zest_gpu_context* ctx, SplitState* st, const DftTables& t
                 add_units(ul, S, bits, r, std::min<long long>(SP_M, rows - r), 1, Lg - 1, NT, Lg - 1, 1 | 2 | 4, 0,
                           0);
         }, &v));
-        return run_gemm_nt(ctx, NT, S, *v, st->op[0], st->op[1], t.cos_bj, t.sin_bj,
+        return run_gemm(ctx, S, *v, st->op[0], st->op[1], t.cos_bj, t.sin_bj,
                            EpiDftBwdSinRaw{grids, Ts, C, N, Lg, gsz});
     });
 }
@@ -2291,9 +2253,9 @@ int split_zt_forward(zest_gpu_context* ctx, ZtPlan& plan, int Lg, int Le, int Lm
                     }
             }, &u));
             if (ch == 0)
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], tb->leg_f, tb->leg_f, EpiLegFwd<false>{flm, batch, nr2}));
+                ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[1], tb->leg_f, tb->leg_f, EpiLegFwd<false>{flm, batch, nr2}));
             else
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], tb->leg_f, tb->leg_f, EpiLegFwd<true>{flm, batch, nr2}));
+                ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[1], tb->leg_f, tb->leg_f, EpiLegFwd<true>{flm, batch, nr2}));
         }
         return ZEST_GPU_OK;
         }));
@@ -2317,9 +2279,9 @@ int split_zt_forward(zest_gpu_context* ctx, ZtPlan& plan, int Lg, int Le, int Lm
                               int(plan.rad.off_h[l]), (Lm - l + 1) / 2, NT, std::min(KCHUNK, nr - k0), 0, l, k0);
             }, &u));
             if (ch == 0)
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[0], tb->rad_f, tb->rad_f, EpiRadFwd<false>{coeffs, batch, csz}));
+                ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[0], tb->rad_f, tb->rad_f, EpiRadFwd<false>{coeffs, batch, csz}));
             else
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[0], tb->rad_f, tb->rad_f, EpiRadFwd<true>{coeffs, batch, csz}));
+                ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[0], tb->rad_f, tb->rad_f, EpiRadFwd<true>{coeffs, batch, csz}));
         }
         return ZEST_GPU_OK;
         }));
@@ -2369,9 +2331,9 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
                               std::min(KCHUNK, (Lm - l + 1) / 2 - k0), 0, l, k0);
             }, &u));
             if (ch == 0)
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[0], tb->rad_bT, tb->rad_bT, EpiRadBwd<false>{flm, nr, batch}));
+                ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[0], tb->rad_bT, tb->rad_bT, EpiRadBwd<false>{flm, nr, batch}));
             else
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[0], tb->rad_bT, tb->rad_bT, EpiRadBwd<true>{flm, nr, batch}));
+                ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[0], tb->rad_bT, tb->rad_bT, EpiRadBwd<true>{flm, nr, batch}));
         }
         return ZEST_GPU_OK;
         }));
@@ -2403,7 +2365,7 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
                 // spare the inverse DFT's input a second array
                 ul.useful *= 0.5;
             }, &u));
-            return run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[0], tb->leg_bU, tb->leg_bU,
+            return run_gemm(ctx, S, *u, st->op[0], st->op[0], tb->leg_bU, tb->leg_bU,
                                EpiLegBwdU<false>{E, batch, Lg, nlat, nr2});
         }));
         // ---- longitude: inverse real DFT of the spectra at every latitude ----
@@ -2438,10 +2400,10 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
                 }
             }, &u));
             if (ch == 0)
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], tb->leg_bT, tb->leg_bT,
+                ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[1], tb->leg_bT, tb->leg_bT,
                                 EpiLegBwdE<false>{E, batch, Lg, kh, nr2}));
             else
-                ZG_TRY(run_gemm_nt(ctx, NT, S, *u, st->op[0], st->op[1], tb->leg_bT, tb->leg_bT,
+                ZG_TRY(run_gemm(ctx, S, *u, st->op[0], st->op[1], tb->leg_bT, tb->leg_bT,
                                 EpiLegBwdE<true>{E, batch, Lg, kh, nr2}));
         }
         return ZEST_GPU_OK;
@@ -2462,26 +2424,13 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
 // Split-precision SH Legendre sums.  The table is the 128-row operand: with
 // 2 x batch data rows per order m the data could not fill a row tile.  The
 // data (the folded spectra, or the coefficients) is the scaled-copy operand,
-// sliced per call; its 2 x batch rows are the columns, in tiles of 16 (batches
-// up to 8: a tile loads no unused data rows), 32 (up to 16) or 80.
+// sliced per call; its 2 x batch rows are the columns.
 // ===========================================================================
 namespace {
-template <class F>
-int st_with_nt(int batch, F&& f) {
-    if (2 * batch <= 16) return f(std::integral_constant<int, 16>{});
-    return 2 * batch <= 32 ? f(std::integral_constant<int, 32>{}) : f(std::integral_constant<int, 80>{});
-}
 // SH sums always use 8-bit digits and 6 slices; sums longer than 256 run as
 // K-chunks of at most 256 whose FP64 results are added (the later chunks
 // through the read-modify-write epilogues).
 constexpr int ST_KCHUNK = SL_K8MAX;
-template <int NT, class Epi>
-int run_gemm_st(zest_gpu_context* ctx, UnitList& ul, const SliceArray& A, const SliceArray& B0, const SliceArray& B1,
-                const Epi& epi) {
-    if (A.bits != 8 || B0.bits != 8 || B1.bits != 8)
-        return fail(ZEST_GPU_ERR_INVALID, "split SH sums: operands must have 8-bit digits");
-    return run_gemm_t<6, 8, NT>(ctx, ul, A, A, B0, B1, epi);
-}
 }  // namespace
 
 int split_st_forward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int batch, const double* X, double* coeffs,
@@ -2507,25 +2456,23 @@ int split_st_forward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int ba
     const int nchunk = (kh + ST_KCHUNK - 1) / ST_KCHUNK;
     for (int ch = 0; ch < nchunk; ++ch) {
         const int k0 = ch * ST_KCHUNK, kk = std::min(ST_KCHUNK, kh - k0);
-        ZG_TRY(st_with_nt(batch, [&](auto nt) -> int {
-            constexpr int NT = decltype(nt)::value;
-            UnitList* u;
-            ZG_TRY(get_units(ctx, std::make_tuple(int(WK_ST_LEG_F), Lg, Lm, batch, S, int(plan.sh.latlon) + 2 * ch),
-                             [&](UnitList& ul) {
-                                 for (int m = 0; m < Lm; ++m)
-                                     for (int p = 0; p < 2; ++p) {
-                                         const int cnt = (Lm - m - p > 0) ? (Lm - m - p + 1) / 2 : 0;
-                                         add_units(ul, S, bits, plan.leg.off_h[2 * m + p], cnt, int(m * per_m),
-                                                   int(per_m), NT, kk, (p << 1) | (p << 2), m, k0);
-                                     }
-                             },
-                             &u));
-            if (ch == 0)
-                return run_gemm_st<NT>(ctx, *u, tb->leg_f, st->op[0], st->op[1],
-                                       EpiStLegFwd<false>{coeffs, csz, plan.leg.L});
-            return run_gemm_st<NT>(ctx, *u, tb->leg_f, st->op[0], st->op[1],
-                                   EpiStLegFwd<true>{coeffs, csz, plan.leg.L});
-        }));
+        UnitList* u;
+        ZG_TRY(get_units(ctx, std::make_tuple(int(WK_ST_LEG_F), Lg, Lm, batch, S, int(plan.sh.latlon) + 2 * ch),
+                         [&](UnitList& ul) {
+                             for (int m = 0; m < Lm; ++m)
+                                 for (int p = 0; p < 2; ++p) {
+                                     const int cnt = (Lm - m - p > 0) ? (Lm - m - p + 1) / 2 : 0;
+                                     add_units(ul, S, bits, plan.leg.off_h[2 * m + p], cnt, int(m * per_m),
+                                               int(per_m), n_tile(S), kk, (p << 1) | (p << 2), m, k0);
+                                 }
+                         },
+                         &u));
+        if (ch == 0)
+            ZG_TRY(run_gemm_t<6>(ctx, *u, tb->leg_f, tb->leg_f, st->op[0], st->op[1],
+                            EpiStLegFwd<false>{coeffs, csz, plan.leg.L}));
+        else
+            ZG_TRY(run_gemm_t<6>(ctx, *u, tb->leg_f, tb->leg_f, st->op[0], st->op[1],
+                            EpiStLegFwd<true>{coeffs, csz, plan.leg.L}));
     }
     return split_finish(ctx);
 }
@@ -2558,27 +2505,25 @@ int split_st_backward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int b
     const int nchunk = ((Lm + 1) / 2 + ST_KCHUNK - 1) / ST_KCHUNK;
     for (int ch = 0; ch < nchunk; ++ch) {
         const int k0 = ch * ST_KCHUNK;
-        ZG_TRY(st_with_nt(batch, [&](auto nt) -> int {
-            constexpr int NT = decltype(nt)::value;
-            UnitList* u;
-            ZG_TRY(get_units(ctx, std::make_tuple(int(WK_ST_LEG_B), Lg, Lm, batch, S, int(plan.sh.latlon) + 2 * ch),
-                             [&](UnitList& ul) {
-                                 for (int m = 0; m < Lm; ++m)
-                                     for (int p = 0; p < 2; ++p) {
-                                         const int cnt = (Lm - m - p > 0) ? (Lm - m - p + 1) / 2 : 0;
-                                         // the degrees of this chunk: i in [k0, min(cnt, k0 + 256))
-                                         const int kk = std::min(cnt - k0, ST_KCHUNK);
-                                         add_units(ul, S, bits, (long long)(2 * m + p) * kh, kh, int(m * per_m),
-                                                   int(per_m), NT, kk, (p << 1) | (p << 2), m, k0);
-                                     }
-                             },
-                             &u));
-            if (ch == 0)
-                return run_gemm_st<NT>(ctx, *u, tb->leg_bT, st->op[0], st->op[1],
-                                       EpiStLegBwdE<false>{E, batch, Lg, kh});
-            return run_gemm_st<NT>(ctx, *u, tb->leg_bT, st->op[0], st->op[1],
-                                   EpiStLegBwdE<true>{E, batch, Lg, kh});
-        }));
+        UnitList* u;
+        ZG_TRY(get_units(ctx, std::make_tuple(int(WK_ST_LEG_B), Lg, Lm, batch, S, int(plan.sh.latlon) + 2 * ch),
+                         [&](UnitList& ul) {
+                             for (int m = 0; m < Lm; ++m)
+                                 for (int p = 0; p < 2; ++p) {
+                                     const int cnt = (Lm - m - p > 0) ? (Lm - m - p + 1) / 2 : 0;
+                                     // the degrees of this chunk: i in [k0, min(cnt, k0 + 256))
+                                     const int kk = std::min(cnt - k0, ST_KCHUNK);
+                                     add_units(ul, S, bits, (long long)(2 * m + p) * kh, kh, int(m * per_m),
+                                               int(per_m), n_tile(S), kk, (p << 1) | (p << 2), m, k0);
+                                 }
+                         },
+                         &u));
+        if (ch == 0)
+            ZG_TRY(run_gemm_t<6>(ctx, *u, tb->leg_bT, tb->leg_bT, st->op[0], st->op[1],
+                            EpiStLegBwdE<false>{E, batch, Lg, kh}));
+        else
+            ZG_TRY(run_gemm_t<6>(ctx, *u, tb->leg_bT, tb->leg_bT, st->op[0], st->op[1],
+                            EpiStLegBwdE<true>{E, batch, Lg, kh}));
     }
     *Eout = E;
     return ZEST_GPU_OK;
@@ -2602,8 +2547,8 @@ int split_dense_gemm(zest_gpu_context* ctx, int M, int N, int K, const double* A
         const int k0 = ch * KCHUNK;
         UnitList u;
         add_units(u, S, bits, 0, M, 0, N, NT, std::min(KCHUNK, K - k0), 0, 0, k0);
-        if (ch == 0) ZG_TRY(run_gemm_nt(ctx, NT, S, u, a, a, b, b, EpiDense<false>{C, N}));
-        else ZG_TRY(run_gemm_nt(ctx, NT, S, u, a, a, b, b, EpiDense<true>{C, N}));
+        if (ch == 0) ZG_TRY(run_gemm(ctx, S, u, a, a, b, b, EpiDense<false>{C, N}));
+        else ZG_TRY(run_gemm(ctx, S, u, a, a, b, b, EpiDense<true>{C, N}));
         ZG_TRY(split_finish(ctx));  // the local work list must outlive its launch
     }
     return ZEST_GPU_OK;  // the local operands outlive the launches (split_finish synchronizes)
