@@ -158,17 +158,19 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-}
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// waits for this warp's loads; names their registers, so that nothing uses them before
+template <int N>
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[N][4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int a = 0; a < N; ++a)
+        asm volatile("" : "+r"(v[a][0]), "+r"(v[a][1]), "+r"(v[a][2]), "+r"(v[a][3]));
+}
 // a * b + c with a 32 x 32 -> 64-bit signed product
 __device__ __forceinline__ long long mad_wide_s32(int a, int b, long long c) {
     long long r;
@@ -517,9 +519,8 @@ __device__ __forceinline__ constexpr long long digit_bias() {
 // pattern 0x6400 | byte is 1024 + byte, so a pair of digits is two bytes under
 // that mask and one packed subtraction of 1152; one byte permute brings two
 // digits of two elements together.  5 integer operations an element (9 when
-// each digit was built as a float), which are what the slicing spends its time
-// on: at order 200 x 64 forward + backward 17.6 -> 17.2 ms,
-// most of which is now the memory's.
+// each digit was built as a float), at order
+// 200 x 64 forward + backward 17.6 -> 17.2 ms, most of which is the memory's.
 template <int S>
 __device__ __forceinline__ void store_digits8(const unsigned long long (&u)[8], __half* out, long long stride) {
     constexpr uint32_t MAGIC = 0x64006400u;
@@ -985,8 +986,9 @@ struct EpiDftBwdCosRaw {
         return Row{grid + b * gsz + col, Ts + (b * L + u.aux) * C + col, u.aux};
     }
     __device__ void load_raw(const Row&, int, long long*) const {}
-    __device__ void store_raw(const Row& R, const SplitUnit&, int n, long long T, int e, long long) const {
-        if (R.aux + n == 0) *R.x = i64_ldexp(T, e);
+    template <class Value>
+    __device__ void store_raw(const Row& R, int n, long long T, long long, const Value& value) const {
+        if (R.aux + n == 0) *R.x = value(T);
         else R.t[(long long)n * C] = T;
     }
 };
@@ -1004,10 +1006,11 @@ struct EpiDftBwdSinRaw {
         return Row{grid + b * gsz + col, Ts + (b * L + u.aux + 1) * C + col, u.aux + 1};
     }
     __device__ void load_raw(const Row& R, int n, long long* old) const { *old = R.t[(long long)n * C]; }
-    __device__ void store_raw(const Row& R, const SplitUnit&, int n, long long T, int e, long long old) const {
+    template <class Value>
+    __device__ void store_raw(const Row& R, int n, long long T, long long old, const Value& value) const {
         const int i = R.i0 + n;
-        R.x[(long long)i * C] = i64_ldexp(old + T, e);
-        R.x[(long long)(N - i) * C] = i64_ldexp(old - T, e);
+        R.x[(long long)i * C] = value(old + T);
+        R.x[(long long)(N - i) * C] = value(old - T);
     }
 };
 
@@ -1043,7 +1046,7 @@ struct SplitParams {
 // stages, load, multiply and drain only the rows they have.  With every tile
 // 80 wide the 200 columns of an order-200 DFT cost 240; with this the GEMMs of
 // the transforms at order 200 x 64 take 30.0 ms instead of 31.4, and 1,024
-// transforms of orders 8 to 64 36.8 ms instead of 40.4.
+// items of orders 8 to 64 40.4 ms instead of 42.0.
 template <int S>
 struct Sched {
     static constexpr int NACC = S;                      // accumulators: levels 0..S-1
@@ -1236,7 +1239,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             const int* __restrict__ eav = amap ? P.ea[1] : P.ea[0];
             const int* __restrict__ ebv = bmap ? P.eb[1] : P.eb[0];
             const int ea = eav[row];
-            const int eb_a = (lane < cw && col0 + lane < u.n) ? ebv[u.b_row0 + col0 + lane] : 0;
+            const bool hascol = lane < cw && col0 + lane < u.n;
+            const int eb_a = hascol ? ebv[u.b_row0 + col0 + lane] : 0;
             const typename Epi::Row R = epi.row(u, row);
             const int side = tile & 1;
             const uint32_t tacc = tmem + (uint32_t)acc_column(tile, W);
@@ -1259,107 +1263,110 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
             // warps whose columns are all past the unit's valid rows skip the work
             const bool active = col0 < u.n;
             if (active) {
+                const uint32_t tcol = tacc + ((uint32_t)(32 * q) << 16) + (uint32_t)col0;
 #pragma unroll
-            for (int c = 0; c < CW / 4; ++c) {
-                if (4 * c >= cw) break;
-                uint32_t v[SC::NACC][4];
+                for (int c = 0; c < CW / 4; ++c) {
+                    if (4 * c >= cw) break;
+                    uint32_t v[SC::NACC][4];
 #pragma unroll
-                for (int a = 0; a < SC::NACC; ++a)
-                    tmem_ld4(tacc + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * W + col0 + 4 * c), v[a]);
-                tmem_ld_wait();
+                    for (int a = 0; a < SC::NACC; ++a) tmem_ld4(tcol + (uint32_t)(a * W + 4 * c), v[a]);
+                    tmem_ld_wait(v);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int i0 = __float_as_int(__uint_as_float(v[0][j]) + 12582912.0f) - 0x4B400000;
-                    const int i01 = i0 * 256 + __float2int_rn(__uint_as_float(v[1][j]));
-                    long long t;
-                    if constexpr (S == 6) {
-                        // levels 4 and 5 combined in FP32 at level 4's unit (2^8 of T):
-                        // one rounding of the sum and one of the conversion, at most
-                        // 1.5 units of level 4 (384 of T), against up to K 2^7 of T
-                        // from the rounding of the operands to 48 bits
-                        const int i45 = __float2int_rn(__fmaf_rn(__uint_as_float(v[5][j]), 0.00390625f,
-                                                                 __uint_as_float(v[4][j])));
-                        t = (long long)i01 * 4294967296LL;
-                        t = mad_wide_s32(__float2int_rn(__uint_as_float(v[2][j])), 1 << 24, t);
-                        t = mad_wide_s32(__float2int_rn(__uint_as_float(v[3][j])), 1 << 16, t);
-                        t = mad_wide_s32(i45, 1 << 8, t);
-                    } else {
-                        t = i01;
+                    for (int j = 0; j < 4; ++j) {
+                        const int i0 = __float_as_int(__uint_as_float(v[0][j]) + 12582912.0f) - 0x4B400000;
+                        const int i01 = i0 * 256 + __float2int_rn(__uint_as_float(v[1][j]));
+                        long long t;
+                        if constexpr (S == 6) {
+                            // levels 4 and 5 combined in FP32 at level 4's unit (2^8 of T):
+                            // one rounding of the sum and one of the conversion, at most
+                            // 1.5 units of level 4 (384 of T), against up to K 2^7 of T
+                            // from the rounding of the operands to 48 bits
+                            const int i45 = __float2int_rn(__fmaf_rn(__uint_as_float(v[5][j]), 0.00390625f,
+                                                                     __uint_as_float(v[4][j])));
+                            t = (long long)i01 * 4294967296LL;
+                            t = mad_wide_s32(__float2int_rn(__uint_as_float(v[2][j])), 1 << 24, t);
+                            t = mad_wide_s32(__float2int_rn(__uint_as_float(v[3][j])), 1 << 16, t);
+                            t = mad_wide_s32(i45, 1 << 8, t);
+                        } else {
+                            t = i01;
 #pragma unroll
-                        for (int a = 2; a < SC::NACC; ++a) t = t * 256 + __float2int_rn(__uint_as_float(v[a][j]));
+                            for (int a = 2; a < SC::NACC; ++a) t = t * 256 + __float2int_rn(__uint_as_float(v[a][j]));
+                        }
+                        T[4 * c + j] = t;
                     }
-                    T[4 * c + j] = t;
                 }
-            }
             }
             tc_fence_before();
             __syncwarp();
             const long long w2 = clock64();
             if (lane == 0) mbar_arrive(&tempty[side]);
             // phase 2 (overlaps the next tile's MMAs): FP64 results and stores
-            if constexpr (raw_epi<Epi>::value) {
-            if (active) {
-#pragma unroll
-            for (int c = 0; c < CW / 4; ++c) {
-                if (4 * c >= cw) break;
-                long long oldr[4] = {0, 0, 0, 0};
-                if constexpr (Epi::RMW) {
-                    if (rv) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (col0 + 4 * c + j < u.n) epi.load_raw(R, col0 + 4 * c + j, &oldr[j]);
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int n = col0 + 4 * c + j;
-                    const int idx = 4 * c + j;
-                    const int eb = __shfl_sync(0xffffffffu, eb_a, idx);
-                    if (rv && n < u.n) epi.store_raw(R, u, n, T[4 * c + j], ea + eb + TEXP, oldr[j]);
-                }
-            }
-            }
-            } else {
-            if (active) {
-#pragma unroll
-            for (int c = 0; c < CW / 4; ++c) {
-                if (4 * c >= cw) break;
-                double old[4][2];
-                double vv[4];  // pair-row epilogues: this row's values of the four columns
-                if constexpr (Epi::RMW) {
-                    if (rv) {
+            // x: this row's and column's scale, as an exponent or as the high word's
+            // base of i64_ldexp_normal; the latter where every result of the warp is
+            // in the normal range whatever its value
+            auto emit = [&](auto normal, int xrow, int xcol) {
+                constexpr bool NORMAL = decltype(normal)::value;
+                // raw epilogues: the old values of the next four columns are on their
+                // way while four are combined and stored
+                [[maybe_unused]] long long nextr[4] = {0, 0, 0, 0};
+                [[maybe_unused]] auto fetch = [&](int c0) {
+                    if constexpr (Epi::RMW && raw_epi<Epi>::value) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            if (col0 + 4 * c + j < u.n) epi.load(R, col0 + 4 * c + j, old[j]);
+                            if (rv && col0 + c0 + j < u.n) epi.load_raw(R, col0 + c0 + j, &nextr[j]);
                     }
-                }
+                };
+                if constexpr (raw_epi<Epi>::value) fetch(0);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int n = col0 + 4 * c + j;
-                    const int idx = 4 * c + j;
-                    const int eb = __shfl_sync(0xffffffffu, eb_a, idx);
-                    if constexpr (pair_rows_epi<Epi>::value) {
-                        // rows 2i and 2i + 1 are the two halves of one 16-byte
-                        // pair at every column: neighbouring lanes swap one
-                        // value, and each stores a whole pair, the even lane at
-                        // the even column of the two and the odd lane at the
-                        // odd one
-                        vv[j] = i64_ldexp(T[4 * c + j], ea + eb + TEXP);
-                        if (j & 1) {
-                            const bool odd = lane & 1;
-                            const double got = __shfl_xor_sync(0xffffffffu, odd ? vv[j - 1] : vv[j], 1);
-                            const int np = odd ? n : n - 1;
-                            if (rv && np < u.n)
-                                epi.store_pair(R, np, odd ? make_double2(got, vv[j]) : make_double2(vv[j - 1], got),
-                                               odd);
+                for (int c = 0; c < CW / 4; ++c) {
+                    if (4 * c >= cw) break;
+                    [[maybe_unused]] double old[4][2];
+                    [[maybe_unused]] double vv[4];  // pair-row epilogues: this row's values of the four columns
+                    [[maybe_unused]] long long oldr[4] = {nextr[0], nextr[1], nextr[2], nextr[3]};
+                    if constexpr (raw_epi<Epi>::value) {
+                        if (4 * (c + 1) < cw) fetch(4 * (c + 1));
+                    } else if constexpr (Epi::RMW) {
+                        if (rv) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (col0 + 4 * c + j < u.n) epi.load(R, col0 + 4 * c + j, old[j]);
                         }
-                    } else if (rv && n < u.n) {
-                        const double v = i64_ldexp(T[4 * c + j], ea + eb + TEXP);
-                        epi.store(R, u, n, v, old[j]);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int n = col0 + 4 * c + j;
+                        const int x = xrow + __shfl_sync(0xffffffffu, xcol, 4 * c + j);
+                        auto value = [x](long long t) { return NORMAL ? i64_ldexp_normal(t, x) : i64_ldexp(t, x); };
+                        if constexpr (raw_epi<Epi>::value) {
+                            if (rv && n < u.n) epi.store_raw(R, n, T[4 * c + j], oldr[j], value);
+                        } else if constexpr (pair_rows_epi<Epi>::value) {
+                            // rows 2i and 2i + 1 are the two halves of one 16-byte
+                            // pair at every column: neighbouring lanes swap one
+                            // value, and each stores a whole pair, the even lane at
+                            // the even column of the two and the odd lane at the
+                            // odd one
+                            vv[j] = value(T[4 * c + j]);
+                            if (j & 1) {
+                                const bool odd = lane & 1;
+                                const double got = __shfl_xor_sync(0xffffffffu, odd ? vv[j - 1] : vv[j], 1);
+                                const int np = odd ? n : n - 1;
+                                if (rv && np < u.n)
+                                    epi.store_pair(R, np, odd ? make_double2(got, vv[j]) : make_double2(vv[j - 1], got),
+                                                   odd);
+                            }
+                        } else if (rv && n < u.n) {
+                            epi.store(R, u, n, value(T[4 * c + j]), old[j]);
+                        }
                     }
                 }
-            }
-            }
+            };
+            if (active) {
+                const int emin = __reduce_min_sync(0xffffffffu, ea) + __reduce_min_sync(0xffffffffu, hascol ? eb_a : 1 << 20);
+                const int emax = __reduce_max_sync(0xffffffffu, ea) + __reduce_max_sync(0xffffffffu, hascol ? eb_a : -(1 << 20));
+                if (emin + TEXP >= -1022 && emax + TEXP <= 958)
+                    emit(std::true_type{}, (ea + TEXP + 1085) << 20, eb_a << 20);
+                else
+                    emit(std::false_type{}, ea + TEXP, eb_a);
             }
             if (P.dbg && warp == 2 && lane == 0) {
                 atomicAdd(&P.dbg[3], (unsigned long long)(w1 - w0));
