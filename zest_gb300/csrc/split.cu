@@ -25,7 +25,7 @@
 // Only the tables (P_lm, R_nl, cos/sin) are prepared in FP64.
 //
 // Kernel: warp-specialised, persistent, one CTA per SM.  Warp 0 issues TMA
-// loads (SWIZZLE_32B, one 16-wide K block of the S slices of both operands
+// loads (no swizzle, one 16-wide K block of the S slices of both operands
 // per pipeline stage, the B slices back to back), warp 1 issues tcgen05.mma
 // (M = 128 operand rows; the products of one A slice with consecutive B
 // slices go to consecutive accumulators, so up to 256 / W of them form one
@@ -178,14 +178,15 @@ __device__ __forceinline__ long long mad_wide_s32(int a, int b, long long c) {
     return r;
 }
 
-// K-major operand tile, SWIZZLE_32B: rows of 32 bytes, 8-row groups 256 bytes apart.
-__device__ __forceinline__ uint64_t desc_sw32(uint32_t saddr) {
+// K-major operand tile of 8 x 16-byte core matrices, no swizzle: the rows of one
+// group of 8 K elements are contiguous (16 bytes each, 8-row groups 128 bytes
+// apart), the next group is kstride bytes further.
+__device__ __forceinline__ uint64_t desc_rows16(uint32_t saddr, uint32_t kstride) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address
-    d |= (uint64_t)(16u >> 4) << 16;           // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(256u >> 4) << 32;          // stride byte offset: 8 rows x 32 B
+    d |= (uint64_t)(kstride >> 4) << 16;       // leading byte offset: along K
+    d |= (uint64_t)(128u >> 4) << 32;          // stride byte offset: 8 rows
     d |= (uint64_t)1 << 46;                    // descriptor version for tcgen05
-    d |= (uint64_t)6 << 61;                    // SWIZZLE_32B
     return d;
 }
 __host__ __device__ constexpr uint32_t idesc_f16_f32(int M, int N) {
@@ -498,12 +499,12 @@ struct ragged_loader<L, std::void_t<decltype(std::declval<const L&>().kvalid(std
 // each at neighbouring chunks (stride 9 doubles) hit distinct banks.
 __device__ __forceinline__ int sl_pos(int k) { return k + (k >> 3); }
 
-// Row stride of the staged rows: room for KS padded elements, and 2 mod 4
-// doubles, so that the row-fast staging (16 rows x 2 k per warp) stores
-// conflict-free.
-inline int sl_row_stride(int KS) {
-    const int p = KS + (KS >> 3) + 1;
-    return p + ((6 - p % 4) % 4);
+// Row stride of the staged rows: room for KS padded elements, and 16 / R
+// doubles (one from 16 rows on) past a multiple of twice that, so that a half
+// warp on R rows at 16 / R neighbouring elements or chunks is conflict-free.
+inline int sl_row_stride(int KS, int R) {
+    const int step = R < 16 ? 16 / R : 1, need = KS + (KS >> 3) + 1;
+    return (need + step - 1) / (2 * step) * (2 * step) + step;
 }
 
 // 128 in each of the S digit bytes of a biased fixed-point value: byte b of
@@ -676,13 +677,13 @@ __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
     const int nch0 = min(J.Kp0, KS) >> 3, nch1 = NA > 1 ? min(J.Kp1, KS) >> 3 : 0;
     const int nch = max(nch0, nch1);
     if (nch == 0) return;  // a ragged block of rows with no valid k: exponents only
-    const int items = R * nch;
-    int r = threadIdx.x / nch, c = threadIdx.x - r * nch;
-    const int dr = blockDim.x / nch, dc = blockDim.x - dr * nch;
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-        const long long row = row0 + r;
-        if (row < J.rows) {
-            const int Cr = 1074 + (max(int(emax[r] >> 20), 64) - 1022 + 1 + fold_bit) - nbits;
+    // every thread stays on one row; neighbouring threads have neighbouring rows,
+    // whose digits of one chunk are neighbours in the slice arrays
+    const int r = threadIdx.x & (R - 1);
+    const long long row = row0 + r;
+    if (row < J.rows) {
+        const int Cr = 1074 + (max(int(emax[r] >> 20), 64) - 1022 + 1 + fold_bit) - nbits;
+        for (int c = threadIdx.x >> lr; c < nch; c += (int)blockDim.x >> lr) {
             const double* base = sl_smem + r * Ks + 9 * c;  // element 8c
             constexpr int NJ = 8 + SHIFT;
             auto at = [&](int a, int j) { return base[a * astride + j + (j >> 3)]; };
@@ -690,7 +691,7 @@ __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
                 unsigned long long w[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(0, q), Cr, digit_bias<S>());
-                store_digits8<S>(w, J.out0 + row * J.Kp0 + 8 * c, J.stride0);
+                store_digits8<S>(w, J.out0 + c * S * J.stride0 + row * 8, J.stride0);
             } else if constexpr (MODE == SL_FOLD) {
                 long long fu[NJ], fd[NJ];
 #pragma unroll
@@ -702,12 +703,12 @@ __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
                 if (c < nch0) {
 #pragma unroll
                     for (int q = 0; q < 8; ++q) w[q] = fu[q] + fd[q];
-                    store_digits8<S>(w, J.out0 + row * J.Kp0 + 8 * c, J.stride0);
+                    store_digits8<S>(w, J.out0 + c * S * J.stride0 + row * 8, J.stride0);
                 }
                 if (c < nch1) {
 #pragma unroll
                     for (int q = 0; q < 8; ++q) w[q] = fu[q + SHIFT] - fd[q + SHIFT];
-                    store_digits8<S>(w, J.out1 + row * J.Kp1 + 8 * c, J.stride1);
+                    store_digits8<S>(w, J.out1 + c * S * J.stride1 + row * 8, J.stride1);
                 }
             } else {
                 // SL_PAIR: up | dn
@@ -715,20 +716,14 @@ __global__ void __launch_bounds__(256) slice_kernel(Loader ld, SliceJob J) {
                 if (c < nch0) {
 #pragma unroll
                     for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(0, q), Cr, digit_bias<S>());
-                    store_digits8<S>(w, J.out0 + row * J.Kp0 + 8 * c, J.stride0);
+                    store_digits8<S>(w, J.out0 + c * S * J.stride0 + row * 8, J.stride0);
                 }
                 if (c < nch1) {
 #pragma unroll
                     for (int q = 0; q < 8; ++q) w[q] = to_fixed_c(at(1, q + SHIFT), Cr, digit_bias<S>());
-                    store_digits8<S>(w, J.out1 + row * J.Kp1 + 8 * c, J.stride1);
+                    store_digits8<S>(w, J.out1 + c * S * J.stride1 + row * 8, J.stride1);
                 }
             }
-        }
-        c += dc;
-        r += dr;
-        if (c >= nch) {
-            c -= nch;
-            ++r;
         }
     }
 }
@@ -1046,7 +1041,7 @@ struct SplitParams {
 // stages, load, multiply and drain only the rows they have.  With every tile
 // 80 wide the 200 columns of an order-200 DFT cost 240; with this the GEMMs of
 // the transforms at order 200 x 64 take 30.0 ms instead of 31.4, and 1,024
-// items of orders 8 to 64 40.4 ms instead of 42.0.
+// items of orders 8 to 128 40.4 ms instead of 42.0.
 template <int S>
 struct Sched {
     static constexpr int NACC = S;                      // accumulators: levels 0..S-1
@@ -1138,8 +1133,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                     unsigned char* sa = smem + st * STAGE;
                     unsigned char* sb = sa + S * A_TILE;
                     // one box per operand: the S slices of 128 rows (A) and of W rows (B)
-                    tma_load_3d(sa, ma, &full[st], (u.k0 + kb) * SP_KB, u.a_row0, 0);
-                    tma_load_3d(sb, mb, &full[st], (u.k0 + kb) * SP_KB, u.b_row0, 0);
+                    tma_load_3d(sa, ma, &full[st], 2 * u.a_row0, 0, 2 * (u.k0 + kb));
+                    tma_load_3d(sb, mb, &full[st], 2 * u.b_row0, 0, 2 * (u.k0 + kb));
                     if (++st == NST) {
                         st = 0;
                         ph ^= 1;
@@ -1185,18 +1180,19 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                         if (P.dbg) atomicAdd(&P.dbg[2], (unsigned long long)(clock64() - w1));
                         tc_fence_after();
                         // descriptors differ only in the start-address field (address >> 4)
-                        const uint64_t da = desc_sw32(smem_u32(smem + st * STAGE));
-                        const uint64_t db = da + (uint64_t)((S * A_TILE) >> 4);
+                        const uint32_t sa = smem_u32(smem + st * STAGE);
+                        const uint64_t da = desc_rows16(sa, S * SP_M * 16);
+                        const uint64_t db = desc_rows16(sa + S * A_TILE, S * CWD * 16);
                         // A slice 0 comes first: its products start every accumulator
                         // (levels 0..S-1) in the first K block, all later ones add
 #pragma unroll
                         for (int s = 0; s < S; ++s) {
                             const uint32_t acc = (kb > 0 || s > 0) ? 1u : 0u;
-                            const uint64_t as = da + (uint64_t)((s * A_TILE) >> 4);
+                            const uint64_t as = da + (uint64_t)(s * SP_M);
 #pragma unroll
                             for (int t = 0; t < S - s; t += G) {
                                 const int g = (S - s - t) < G ? (S - s - t) : G;
-                                umma_f16(tacc + (uint32_t)((s + t) * CWD), as, db + (uint64_t)((t * CWD * 32) >> 4),
+                                umma_f16(tacc + (uint32_t)((s + t) * CWD), as, db + (uint64_t)(t * CWD),
                                          idesc_f16_f32(SP_M, g * CWD), acc);
                             }
                         }
@@ -1441,19 +1437,22 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// [S][rows][Kp] FP16 slice array -> 3D map (Kp, rows, S), box (16, box_rows,
-// S), 32B swizzle: one copy brings a tile of every slice, the slices one
-// after the other in shared memory (rows past the array's end read as 0)
+// [Kp / 8][S][rows][8] FP16 slice array -> 3D map of 8-byte words (2 rows, S,
+// Kp / 8), box (2 box_rows, S, 2): one copy brings one 16-wide K block of a tile of
+// every slice in runs of 16 box_rows bytes (rows past the array's end read as 0).
+// The copy engine moves about one run a cycle, whatever its length: as [row][K]
+// with 32-byte runs (1,248 a K block at 80 columns) it bounded every GEMM, 29.3 ms
+// of them at order 200 x 64 where the 24 long runs take 26.4.
 int make_map(CUtensorMap* map, const void* base, long long rows, int Kp, int S, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(ZEST_GPU_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
-    if (rows >= (1ll << 31)) return fail(ZEST_GPU_ERR_UNSUPPORTED, "slice array too tall for TMA");
-    cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, (cuuint64_t)S};
-    cuuint64_t strides[2] = {(cuuint64_t)Kp * 2, (cuuint64_t)rows * Kp * 2};
-    cuuint32_t box[3] = {16, (cuuint32_t)box_rows, (cuuint32_t)S};
+    if (rows >= (1ll << 30)) return fail(ZEST_GPU_ERR_UNSUPPORTED, "slice array too tall for TMA");
+    cuuint64_t dims[3] = {(cuuint64_t)rows * 2, (cuuint64_t)S, (cuuint64_t)Kp / 8};
+    cuuint64_t strides[2] = {(cuuint64_t)rows * 16, (cuuint64_t)rows * 16 * S};
+    cuuint32_t box[3] = {2 * (cuuint32_t)box_rows, (cuuint32_t)S, 2};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ZEST_GPU_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(int(r)) + ")");
     return ZEST_GPU_OK;
@@ -1466,7 +1465,7 @@ int n_tile(int S) { return S == 6 ? max_tile<6>() : S == 5 ? max_tile<5>() : max
 
 }  // namespace
 
-// Slice arrays of one operand: [copies * S][rows][Kp] FP16 + per-row exponents
+// Slice arrays of one operand: [Kp / 8][S][rows][8] FP16 + per-row exponents
 // (the GEMMs read one copy: every level has its own accumulator).
 struct SliceArray {
     DevBuf data, ex;
@@ -1585,8 +1584,8 @@ int run_slice(cudaStream_t s, const Loader& ld, SliceJob J) {
     if (std::max(J.Kp0, NA > 1 ? J.Kp1 : 0) == 0) return ZEST_GPU_OK;  // nothing to write
     J.KS = std::max(J.Kp0, NA > 1 ? J.Kp1 : 0) + Loader::SHIFT;
     if (J.K > J.KS) return fail(ZEST_GPU_ERR_INVALID, "split path: staged range");
-    J.Ks = sl_row_stride(J.KS);
-    J.R = slice_rows_per_block(NA * J.Ks * (int)sizeof(double));
+    J.R = slice_rows_per_block(NA * sl_row_stride(J.KS, 4) * (int)sizeof(double));
+    J.Ks = sl_row_stride(J.KS, J.R);
     J.lr = 0;
     while ((1 << J.lr) < J.R) ++J.lr;
     const size_t smem = (size_t)NA * J.R * J.Ks * sizeof(double);
@@ -1623,7 +1622,7 @@ int launch_slice(cudaStream_t s, const Loader& ld, long long rows, int K, int S,
     J.S = S;
     J.bits = bits;
     J.out0 = out.ptr();
-    J.stride0 = out.rows * out.Kp;
+    J.stride0 = out.rows * 8;
     J.ex0 = out.ex.as<int>();
     return run_slice(s, ld, J);
 }
@@ -1652,8 +1651,8 @@ int launch_slice2(cudaStream_t s, const Loader& ld, long long rows, int K0, int 
     J.bits = bits;
     J.out0 = out0.ptr();
     J.out1 = out1.ptr();
-    J.stride0 = out0.rows * out0.Kp;
-    J.stride1 = out1.rows * out1.Kp;
+    J.stride0 = out0.rows * 8;
+    J.stride1 = out1.rows * 8;
     J.ex0 = out0.ex.as<int>();
     J.ex1 = out1.ex.as<int>();
     return run_slice(s, ld, J);
@@ -2031,11 +2030,13 @@ inline int nt_pass(int nt) { return nt << 16; }
 // Runs one split GEMM stage, `launch(nt)`, with its column tile: a tuning
 // override (ZEST_GPU_SPLIT_NT) if set; else, with the context's autotuner on,
 // outside graph capture and for a stage whose launches overwrite their outputs
-// (single sums), the fastest of the candidates (narrower tiles overlap more of
-// the drain of the one before, wider ones read the operand rows less often),
-// timed with CUDA events on the context stream at the stage's first run at
-// this size (each candidate once untimed, then once timed; no choice changes a
-// result); else the rule of stage_nt.
+// (single sums), the fastest of four widths, timed with CUDA events on the
+// context stream at the stage's first run at this size (each candidate once
+// untimed, then once timed; no choice changes a result); else the rule of
+// stage_nt.  Wide tiles read the operand rows less often, narrow ones overlap
+// the drain of the one before and split few units evenly: at order 200 x 64
+// the forward DFT takes 7.3 ms at 80 and 10.9 at 32; 1,024 items of orders 8 to
+// 128 take 37.0 ms with all four and 39.1 with 80 and 32 alone.
 template <class Launch>
 int tuned_stage(zest_gpu_context* ctx, SplitState* st, int wk, int S, int Lg, int Lm, int batch, int ncols,
                 bool idempotent, Launch&& launch) {
