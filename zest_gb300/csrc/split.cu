@@ -333,9 +333,9 @@ __device__ __forceinline__ RadRow rad_row(long long r, int B) {
 }
 // the same decoding for a row of the known group l
 __device__ __forceinline__ RadRow rad_row_of(long long r, int l, int B) {
-    const long long local = (r >> 1) - (long long)l * (l + 1) / 2 * B;
-    const int b = int(local / (l + 1));
-    return RadRow{l, b, int(local - (long long)b * (l + 1)), int(r & 1)};
+    const unsigned local = unsigned((r >> 1) - (long long)l * (l + 1) / 2 * B);  // rows of a group are below 2^30
+    const unsigned b = local / unsigned(l + 1);
+    return RadRow{l, int(b), int(local - b * unsigned(l + 1)), int(r & 1)};
 }
 
 struct RadFwdLoader {  // rows (l, b, m, c) as rad_row; k = radial node: flm[(tri(l,m) B + b)][k][c]
@@ -771,18 +771,18 @@ struct EpiDftFwd {  // rows (b, col): conj X_m -> G[b][m][col][re, im]
     static constexpr bool CHUNK = false;
     double* G;
     int C, L;
-    struct Row { double* p; };  // &G[b][m0][col][re or im]
+    struct Row { double* p; bool first; };  // &G[b][m0][col][re or im]; first: Re F_0 is column 0
     __device__ Row row(const SplitUnit& u, int r) const {
         const int b = r / C, col = r - b * C;
         const int sin = (u.flags >> 1) & 1;
         const int m0 = u.aux + sin;
-        return Row{G + (((long long)b * L + m0) * C + col) * 2 + sin};
+        return Row{G + (((long long)b * L + m0) * C + col) * 2 + sin, m0 == 0};
     }
     __device__ void load(const Row&, int, double*) const {}
-    __device__ void store(const Row& R, const SplitUnit& u, int n, double v, const double*) const {
-        double* g = R.p + (long long)n * C * 2;
+    __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double*) const {
+        double* g = R.p + 2 * ((long long)n * C);
         g[0] = v;
-        if (((u.flags >> 1) & 1) == 0 && u.aux + n == 0) g[1] = 0.0;  // Im X_0 = 0
+        if (R.first && n == 0) g[1] = 0.0;  // Im X_0 = 0
     }
 };
 template <bool ACC = false>
@@ -798,9 +798,10 @@ struct EpiLegFwd {  // rows (m, b, kc) -> flm[tri(l,m)][b][kc], l = m + p + 2 (a
         const int l0 = m + p + 2 * u.aux;
         return Row{flm + (tri_idx(l0, m) * B) * nr2 + local, l0};
     }
-    // tri(l0 + 2n, m) - tri(l0, m) = n (2 l0 + 2 n + 1)
+    // tri(l0 + 2n, m) - tri(l0, m) = n (2 l0 + 2 n + 1), below 2^24; the B nr2 rows
+    // of one (l, m) are below 2^30
     __device__ double* at(const Row& R, int n) const {
-        return R.p + (long long)n * (2LL * R.l0 + 2 * n + 1) * B * nr2;
+        return R.p + (long long)(n * (2 * R.l0 + 2 * n + 1)) * (B * nr2);
     }
     __device__ void load(const Row& R, int n, double* old) const { old[0] = *at(R, n); }
     __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double* old) const {
@@ -814,15 +815,17 @@ struct EpiRadFwd {  // rows (l, b, m, c) as rad_row -> coeffs[b][zidx(n,l,m)][c]
     double* coeffs;
     int B;
     long long cs;
-    struct Row { double* p; long long zl0; int l; };
+    struct Row { double* p; unsigned n0; };
     __device__ Row row(const SplitUnit& u, int r) const {
         const RadRow w = rad_row_of(r, u.g, B);
-        const long long n0 = w.l + 2 * u.aux;
-        return Row{coeffs + w.b * cs + 2 * w.m + w.c, n0, w.l};
+        return Row{coeffs + w.b * cs + 2 * (w.m + ((w.l * w.l) >> 2)) + w.c, unsigned(w.l + 2 * u.aux)};
     }
+    // (n + 1) (n + 3) (2 n + 1) / 24, the product below 2^35: its eighth and the
+    // third of that are 32-bit numbers
     __device__ double* at(const Row& R, int n) const {
-        const long long nn = R.zl0 + 2 * n;
-        return R.p + 2 * ((nn + 1) * (nn + 3) * (2 * nn + 1) / 24 + ((R.l * R.l) >> 2));
+        const unsigned nn = R.n0 + 2 * n;
+        const unsigned long long v = (unsigned long long)((nn + 1) * (nn + 3)) * (2 * nn + 1);
+        return R.p + 2 * (unsigned long long)(unsigned(v >> 3) / 3u);
     }
     __device__ void load(const Row& R, int n, double* old) const { old[0] = *at(R, n); }
     __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double* old) const {
@@ -860,18 +863,18 @@ struct EpiLegBwdE {
     static constexpr bool CHUNK = ACC;
     double* E;
     int B, L, kh, nr2;
-    struct Row { double* p; unsigned long long sgn; };  // sgn: the sign bit flipped for imaginary parts
+    struct Row { double* p; int sgn; };  // sgn: the sign bit flipped for imaginary parts
     __device__ Row row(const SplitUnit& u, int r) const {
         const int m = u.g, par = (u.flags >> 2) & 1;
-        const long long local = r - (long long)m * B * nr2;
-        const int b = int(local / nr2), kc = int(local - (long long)b * nr2);
+        const unsigned local = unsigned(r - (long long)m * B * nr2);  // rows of a group are below 2^30
+        const int b = int(local / unsigned(nr2)), kc = int(local - unsigned(b) * unsigned(nr2));
         return Row{E + ((((long long)par * B + b) * L + m) * kh + u.aux) * nr2 + kc,
-                   (kc & 1) ? (1ull << 63) : 0ull};
+                   int(unsigned(kc) << 31)};
     }
     __device__ void load(const Row& R, int n, double* old) const { old[0] = R.p[(long long)n * nr2]; }
     __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double* old) const {
         // the conjugate by a sign-bit flip (an integer operation, not an FP64 multiply)
-        const double w = __longlong_as_double(__double_as_longlong(v) ^ (long long)R.sgn);
+        const double w = __hiloint2double(__double2hiint(v) ^ R.sgn, __double2loint(v));
         R.p[(long long)n * nr2] = ACC ? old[0] + w : w;
     }
 };
@@ -884,16 +887,16 @@ struct EpiLegBwdU {
     static constexpr bool CHUNK = ACC;
     double* E;
     int B, L, nlat, nr2;
-    struct Row { double* p; unsigned long long sgn; };
+    struct Row { double* p; int sgn; };
     __device__ Row row(const SplitUnit& u, int r) const {
         const int m = u.g;
-        const long long local = r - (long long)m * B * nr2;
-        const int b = int(local / nr2), kc = int(local - (long long)b * nr2);
-        return Row{E + (((long long)b * L + m) * nlat + u.aux) * nr2 + kc, (kc & 1) ? (1ull << 63) : 0ull};
+        const unsigned local = unsigned(r - (long long)m * B * nr2);  // rows of a group are below 2^30
+        const int b = int(local / unsigned(nr2)), kc = int(local - unsigned(b) * unsigned(nr2));
+        return Row{E + (((long long)b * L + m) * nlat + u.aux) * nr2 + kc, int(unsigned(kc) << 31)};
     }
     __device__ void load(const Row& R, int n, double* old) const { old[0] = R.p[(long long)n * nr2]; }
     __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double* old) const {
-        const double w = __longlong_as_double(__double_as_longlong(v) ^ (long long)R.sgn);
+        const double w = __hiloint2double(__double2hiint(v) ^ R.sgn, __double2loint(v));
         R.p[(long long)n * nr2] = ACC ? old[0] + w : w;
     }
 };
@@ -942,7 +945,7 @@ struct EpiStLegBwdE {
         old[0] = R.p[(long long)(n >> 1) * L * kh * 2 + (n & 1)];
     }
     __device__ void store(const Row& R, const SplitUnit&, int n, double v, const double* old) const {
-        const double w = __longlong_as_double(__double_as_longlong(v) ^ (long long)((n & 1) ? 1ull << 63 : 0ull));
+        const double w = __hiloint2double(__double2hiint(v) ^ int(unsigned(n) << 31), __double2loint(v));
         R.p[(long long)(n >> 1) * L * kh * 2 + (n & 1)] = ACC ? old[0] + w : w;
     }
 };
