@@ -1,6 +1,6 @@
 """Benchmark of the headline workload: Zernike GLQ forward + backward
 transforms at order 200 on a batch of 64 functions (the reference's
-zt::GLQTransformerGeo), in the split-precision form (BF16 fixed-point slices
+zt::GLQTransformerGeo), in the split-precision form (FP16 fixed-point slices
 on tcgen05) and in the plain FP64 form on the same GPU.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
@@ -38,10 +38,10 @@ METRIC = "Zernike fwd+bwd transforms/s, order 200x64: split-prec vs FP64 GPU at 
 # DRAM read + write bytes of one forward+backward step per function at order
 # 200, from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of
 # the launches of a step at batch 4, which grow in proportion to the batch:
-# the seven split GEMM launches (6.464 GB) and the six slicing launches
-# (5.376 GB)
-GEMM_DRAM_BYTES_PER_FUNCTION_ORDER200 = 6.464e9 / 4
-SLICE_DRAM_BYTES_PER_FUNCTION_ORDER200 = 5.376e9 / 4
+# the seven split GEMM launches (6.437 GB) and the six slicing launches
+# (5.306 GB)
+GEMM_DRAM_BYTES_PER_FUNCTION_ORDER200 = 6.437e9 / 4
+SLICE_DRAM_BYTES_PER_FUNCTION_ORDER200 = 5.306e9 / 4
 # the least a forward+backward transform can move at order 200: the grid read
 # and written once, the coefficients written and read once
 MIN_BYTES_PER_FUNCTION_ORDER200 = 288.7e6
@@ -287,7 +287,7 @@ def run_sh(args, rank: int, world: int, barrier) -> None:
         peak = peaks["bf16_tflops_sustained"] or peaks["bf16_tflops"]
         roofline = {"bound": "tensor", "kernel": "split_gemm_kernel (all launches of a step)", "achieved": achieved,
                     "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
-                    "algorithmic": "BF16 MMA flops of the slice products on valid rows",
+                    "algorithmic": "FP16 MMA flops of the slice products on valid rows",
                     "useful_tflop_per_step": useful / 1e12, "issued_tflop_per_step": issued / 1e12,
                     "peak_source": peaks["source"] + " bf16 sustained"}
     # CPU baseline: the compiled reference, one transformer per item and thread
@@ -312,7 +312,7 @@ def run_sh(args, rank: int, world: int, barrier) -> None:
                                                                              if split else ", FP64"),
             "value": world * B / (ms * 1e-3), "unit": "transforms/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "bf16 digit slices, fp64 recombination" if split else "f64",
+            "vs_baseline": None, "dtype": "fp16 digit slices and 64-bit fixed point, fp64 recombination" if split else "f64",
             "data": "synthetic", "config": {"workload": "sh_glq_bwd_fwd", "order": 1024, "batch": B,
                                             "layout": "LonLat", "conventions": "GLQTransformerGeo",
                                             "precision": "split" if split else "fp64"},
@@ -560,7 +560,7 @@ def run_rotate(args, rank: int, world: int, barrier) -> None:
             "metric": "Zernike rotations per second, order 64 x 256 (Rotor::rotate)",
             "value": world * B / (out["split"]["ms"] * 1e-3), "unit": "rotations/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": out["split"]["ms"], "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "bf16 digit slices, fp64 recombination",
+            "scaling": "weak", "vs_baseline": None, "dtype": "64-bit fixed point",
             "data": "synthetic", "config": {"workload": "zernike_rotate", "order": L, "batch": B},
             "fp64_gpu": {"value": world * B / (out["fp64"]["ms"] * 1e-3), "ms_per_step": out["fp64"]["ms"]},
             "split_vs_fp64": out["fp64"]["ms"] / out["split"]["ms"],
@@ -702,7 +702,7 @@ def run_batching(args, rank: int, world: int, barrier) -> None:
             "metric": "Zernike rotate + backward expansions/s, 4096 orders U{8..128}",
             "value": world * n / (ms * 1e-3), "unit": "expansions/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "f64" if precision == "fp64" else "bf16-slices + f64",
+            "vs_baseline": None, "dtype": "f64" if precision == "fp64" else "fp16-slices + 64-bit fixed point",
             "data": "synthetic", "config": {"workload": "zernike_ragged_rotate_backward", "items": n,
                                             "orders": "U{8..128} sorted", "precision": precision,
                                             "graph": "CUDA graph replay", "autotune": True},
@@ -862,7 +862,7 @@ def main():
         del g64
         errors = {"forward_coeffs": err_c, "backward_grid": err_g, "roundtrip_grid": err_rt,
                   "measure": "max over the batch of max|x - x_fp64| / max|x_fp64| per function"}
-        dtype = "bf16 digit slices (8-bit fixed point, 6 per operand), fp32 exact level sums, fp64 recombination"
+        dtype = "fp16 digit slices (8-bit fixed point, 6 per operand), fp32 exact level sums, fp64 recombination"
     else:
         ms, prof, launches, clocks, tflops = ms64, prof64, launches64, clocks64, (0.0, 0.0)
         dtype = "f64"
@@ -886,7 +886,7 @@ def main():
                     "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak if achieved else None,
                     "traffic": traffic, "traffic_unit": "bytes per launch (ncu dram read + write)",
                     "peak_source": peaks["source"] + " bf16 sustained",
-                    "algorithmic": "BF16 MMA flops of the slice products on valid rows",
+                    "algorithmic": "FP16 MMA flops of the slice products on valid rows",
                     "useful_tflop_per_step": useful / 1e12, "issued_tflop_per_step": issued / 1e12,
                     "issued_rate": issued / (gemm_ms * 1e-3) / 1e12 if achieved else None,
                     "dram_rate_tbs": (traffic * launches_per_step / (gemm_ms * 1e-3) / 1e12

@@ -69,7 +69,7 @@ extern "C" {
 #define ZEST_EXPANSION_ZERNIKE_ROW 2 /* zt::ZernikeSHSpan: RowSkippingTriangleLayout, layout.hpp:334-371 */
 /* arithmetic of the contractions */
 #define ZEST_PRECISION_FP64 0  /* FP64 everywhere (plain form) */
-#define ZEST_PRECISION_SPLIT 1 /* BF16 fixed-point slices on tcgen05, exact FP32 partial sums, FP64 recombination */
+#define ZEST_PRECISION_SPLIT 1 /* FP16 fixed-point slices on tcgen05, exact FP32 partial sums, FP64 recombination */
 /* memory kinds of data pointers */
 #define ZEST_MEM_DEVICE 0
 #define ZEST_MEM_HOST 1
@@ -86,7 +86,7 @@ int zest_gpu_ctx_create(zest_gpu_context** ctx, int device, void* stream);
 int zest_gpu_ctx_destroy(zest_gpu_context* ctx);
 /* Message of the last failing call on this thread ("" if none). */
 const char* zest_gpu_last_error(void);
-/* Precision of the dense contractions; `slices` = number of BF16 digit
+/* Precision of the dense contractions; `slices` = number of FP16 digit
  * slices per operand for ZEST_PRECISION_SPLIT (4..6, 0 = default 6), 8-bit
  * digits, sums longer than 256 terms in chunks of at most 256. */
 int zest_gpu_set_precision(zest_gpu_context* ctx, int precision, int slices);
@@ -103,7 +103,7 @@ int zest_gpu_trim(zest_gpu_context* ctx);
 int zest_gpu_profile_enable(zest_gpu_context* ctx, int enable);
 int zest_gpu_profile_read(zest_gpu_context* ctx, int reset, double* ms, long long* count, int n);
 int zest_gpu_profile_stage_count(void);
-/* BF16 tensor-core flops of the split-precision products issued while
+/* FP16 tensor-core flops of the split-precision products issued while
  * profiling: `useful` counts valid rows x table rows x K x slice products,
  * `issued` the whole 128-row tiles as executed (reset != 0 clears them). */
 int zest_gpu_profile_flops(zest_gpu_context* ctx, int reset, double* useful, double* issued);
@@ -309,22 +309,23 @@ int zest_gpu_zt_rotate_noalloc(void* stream, size_t order, size_t batch, double*
  * Rotates expansion i by euler[3i..3i+2] (in place) and backward-transforms it
  * to a grid of its own order, for n_items expansions.  `orders` (host) must be
  * non-decreasing; `coeffs`, `euler` and `grids` are device buffers, expansions
- * and grids packed back to back in item order.  The first call for a given
- * (orders, buffers, conventions, precision) runs the work eagerly and records
- * it into a CUDA graph on the context; a later identical call replays the
- * graph (recorded anew if any of the context's device buffers was freed or
- * reallocated since, e.g. by zest_gpu_trim).  Results are those of
+ * and grids packed back to back in item order.  A call on buffers other than
+ * the last call's runs the work eagerly; the second call in a row for the same
+ * (orders, buffers, conventions, precision) records it into a CUDA graph on
+ * the context, and later ones replay the graph (recorded anew if any of the
+ * context's device buffers was freed or reallocated since, e.g. by
+ * zest_gpu_trim).  Results are those of
  * zest_gpu_zt_rotate + zest_gpu_zt_backward per item; in
- * ZEST_PRECISION_SPLIT (orders up to 256) the rotation's d(pi/2) products
- * also run in split precision on the tensor cores, within 1e-11 of FP64. */
+ * ZEST_PRECISION_SPLIT (orders up to 256) the rotation runs in 64-bit fixed
+ * point, within 1e-11 of FP64. */
 int zest_gpu_zt_rotate_backward_ragged(zest_gpu_context* ctx, int zernike_norm, int sh_norm, int sh_phase,
                                        size_t n_items, const int* orders, double* coeffs, const double* euler,
                                        int rotation_type, double* grids);
 /* Autotuning of the contraction tile shapes: when enabled (the default), the
  * first run of each Zernike stage at a new size times the candidate shapes on
  * the context stream and keeps the fastest (the FP64 tile shapes; in
- * ZEST_PRECISION_SPLIT the column tile, 80 or 32, of each single-sum tensor
- * core stage); disabled, a size rule picks them.  The shapes change only how
+ * ZEST_PRECISION_SPLIT the widest column tile, 32 to 80, of each single-sum
+ * tensor core stage); disabled, a size rule picks them.  The shapes change only how
  * the output is tiled, not any result. */
 int zest_gpu_set_autotune(zest_gpu_context* ctx, int enable);
 /* Pipelining of host-memory Zernike transforms (mem = ZEST_MEM_HOST): a
@@ -389,7 +390,7 @@ int zest_gpu_st_rotate_vjp(zest_gpu_context* ctx, size_t order, size_t batch, co
 /* ---- split-precision dense product (no reference counterpart) ----
  * C = A B^T for row-major FP64 A (M x K) and B (N x K), K <= 2048, evaluated
  * with the context's slice count on the tcgen05 path used by
- * ZEST_PRECISION_SPLIT (BF16 fixed-point slices, exact FP32 partial sums,
+ * ZEST_PRECISION_SPLIT (FP16 fixed-point slices, exact FP32 partial sums,
  * FP64 recombination).  Exposed to test and measure the emulation itself. */
 int zest_gpu_split_gemm(zest_gpu_context* ctx, size_t M, size_t N, size_t K, const double* A, const double* B,
                         double* C, int mem);

@@ -258,7 +258,7 @@ class Context:
         _check(self.lib.zest_gpu_profile_enable(self._h, int(enable)))
 
     def profile_flops(self, reset: bool = True):
-        """(useful, issued) BF16 tensor flops of the split products since the last reset."""
+        """(useful, issued) FP16 tensor flops of the split products since the last reset."""
         u = ctypes.c_double(0.0)
         i = ctypes.c_double(0.0)
         _check(self.lib.zest_gpu_profile_flops(self._h, int(reset), ctypes.byref(u), ctypes.byref(i)))

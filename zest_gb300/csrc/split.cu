@@ -1048,7 +1048,6 @@ struct SplitParams {
 template <int S>
 struct Sched {
     static constexpr int NACC = S;                      // accumulators: levels 0..S-1
-    static constexpr int NB = S;                        // B tiles per stage: the S slices
     static constexpr int PRODUCTS = S * (S + 1) / 2;    // slice products per K block
 };
 static_assert(Sched<6>::PRODUCTS == 21 && Sched<4>::PRODUCTS == 10, "schedules");

@@ -1,4 +1,4 @@
-// Split-precision (BF16 fixed-point slices on tcgen05) form of the Zernike
+// Split-precision (FP16 fixed-point slices on tcgen05) form of the Zernike
 // contractions and of the SH Legendre sums; see split.cu.
 #pragma once
 
@@ -32,7 +32,7 @@ int split_st_backward(zest_gpu_context* ctx, StPlan& plan, int Lg, int Lm, int b
                       long long csz, double** E);
 // C = A B^T (A: M x K, B: N x K, C: M x N, row-major FP64 device buffers)
 int split_dense_gemm(zest_gpu_context* ctx, int M, int N, int K, const double* A, const double* B, double* C);
-// BF16 tensor-core flops of the split GEMM launches since the last reset
+// FP16 tensor-core flops of the split GEMM launches since the last reset
 // (counted while profiling is enabled): useful = valid rows x table rows x K,
 // issued = whole 128-row tiles as executed.
 void split_flops(zest_gpu_context* ctx, bool reset, double* useful, double* issued);
