@@ -36,3 +36,27 @@ def test_tile_widths_are_exact(ctx, S, N):
     finally:
         ctx.set_precision(zest_gb300.PRECISION_FP64)
     assert np.array_equal(C, A @ B.T)
+
+
+@pytest.mark.parametrize("ka", [(0,), (-500, 0, 40), (-900, -500, -30, 0, 500, 900)])
+def test_row_scales_are_exact(ctx, ka):
+    # rows scaled by powers of two: warps whose results all stay in the normal
+    # range, and warps with some below it (which are 0) or above (infinite).
+    # The integer sums are exact as above, and so are the scaled ones.
+    import zest_gb300
+    M, N, K = 260, 50, 40
+    rng = np.random.default_rng(len(ka))
+    A = rng.integers(-(1 << 12) + 1, 1 << 12, size=(M, K)).astype(np.float64)
+    B = rng.integers(-(1 << 12) + 1, 1 << 12, size=(N, K)).astype(np.float64)
+    A[7] = 0.0
+    ea = np.array([ka[i % len(ka)] for i in range(M)])
+    eb = np.array([(0, 300, -450)[i % 3] if len(ka) > 1 else 0 for i in range(N)])
+    ctx.set_precision(zest_gb300.PRECISION_SPLIT, 6)
+    try:
+        C = ctx.split_gemm(np.ldexp(A, ea[:, None]), np.ldexp(B, eb[:, None]))
+    finally:
+        ctx.set_precision(zest_gb300.PRECISION_FP64)
+    with np.errstate(over="ignore"):
+        ref = np.ldexp(A @ B.T, ea[:, None] + eb[None, :])
+    ref[np.abs(ref) < 2.0 ** -1022] = 0.0
+    assert np.array_equal(C, ref)
