@@ -18,7 +18,8 @@
 // phases with CB fraction bits.  A sum folds its accumulators every CHUNK terms:
 // CHUNK 2^30 2^27 + 2^30 sum |xh| (Cauchy-Schwarz: 2^29.5 over a chunk) < 2^63.
 // A dropped low product is below 4 units of 2^-HB of the vector's largest
-// coefficient.  A vector with an infinity or a NaN becomes NaN.
+// coefficient.  A vector with an infinity or a NaN becomes NaN, and so does one
+// with an Euler angle whose multiples up to l are not all finite.
 //
 // Measured, order 64 x 256: 0.43 ms a call (0.40 the kernel); 0.80 as sliced
 // tensor products per degree, with an error of 2.8e-14 against 4.5e-15 now; about 1
@@ -50,7 +51,8 @@ __global__ void fixed_wigner_kernel(long long n, const double* __restrict__ d, i
         out[i] = constant(d[i]);
 }
 
-// phases[b][k][m] = e^{-i m angle_k} as limbs {re h, re l, im h, im l}
+// phases[b][k][m] = e^{-i m angle_k} as limbs {re h, re l, im h, im l}; limbs hold no
+// NaN, so the phase of a multiple that is not finite is zero
 __global__ void fixed_phase_kernel(int L, int batch, const double* __restrict__ euler, int type, int4* __restrict__ ph) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
@@ -58,12 +60,19 @@ __global__ void fixed_phase_kernel(int L, int batch, const double* __restrict__ 
     double ang[3];
     convert_angles(euler + 3 * b, type, ang[0], ang[1], ang[2]);
     for (int k = 0; k < 3; ++k) {
-        double s, c;
-        sincos(-double(m) * ang[k], &s, &c);
-        const int2 re = constant(c), im = constant(s);
-        ph[((long long)b * 3 + k) * L + m] = make_int4(re.x, re.y, im.x, im.y);
+        int4 w = make_int4(0, 0, 0, 0);
+        const double x = -double(m) * ang[k];
+        if (isfinite(x)) {
+            double s, c;
+            sincos(x, &s, &c);
+            const int2 re = constant(c), im = constant(s);
+            w = make_int4(re.x, re.y, im.x, im.y);
+        }
+        ph[((long long)b * 3 + k) * L + m] = w;
     }
 }
+// a phase has a part of at least 1 / sqrt(2), and with it a high limb
+__device__ __forceinline__ bool is_phase(int4 w) { return (w.x | w.z) != 0; }
 
 struct Z {
     long long x, y;
@@ -159,7 +168,7 @@ __global__ void __launch_bounds__(256, 4) rotate_fixed_kernel(RotSet S, int elem
     extern __shared__ __align__(16) int2 fbuf[];
     __shared__ long long off[128];
     __shared__ int item[128];
-    __shared__ unsigned top[128];  // high word of a vector's largest magnitude
+    __shared__ unsigned top[128];  // high word of a vector's largest magnitude; an infinity's: it becomes NaN
     const int l = S.L - 1 - int(blockIdx.y);
     const int V = rot_tile(l, elems, TV), VS = rot_stride(V);
     const long long cnt = S.count(l), first = (long long)blockIdx.x * V;
@@ -186,10 +195,12 @@ __global__ void __launch_bounds__(256, 4) rotate_fixed_kernel(RotSet S, int elem
         auto high = [](double x) { return unsigned(__double2hiint(x)) & 0x7FFFFFFFu; };
         unsigned mx = 0;
         for (int m = lane; m < ld; m += 32) mx = max(mx, m ? max(high(c[2 * m]), high(c[2 * m + 1])) : high(c[0]));
+        const int4* pa = ph + (long long)item[v] * 3 * L;
+        const int4* pg = pa + 2 * L;
+        if (lane < 3 && !is_phase(pa[lane * L + l])) mx = 0x7FF00000u;
         mx = __reduce_max_sync(0xffffffffu, mx);
         if (lane == 0) top[v] = mx;
         const int cr = 1074 + fixed_scale(mx) - HB + 1;  // one bit more of the operand, dropped by the shift below
-        const int4* pg = ph + ((long long)item[v] * 3 + 2) * L;
         for (int m = lane; m < ld; m += 32) {
             Z x{0, 0};
             if (!not_finite(mx)) {
