@@ -194,7 +194,11 @@ __global__ void __launch_bounds__(256, 4) rotate_fixed_kernel(RotSet S, int elem
         const double* c = coeffs + off[v];
         auto high = [](double x) { return unsigned(__double2hiint(x)) & 0x7FFFFFFFu; };
         unsigned mx = 0;
-        for (int m = lane; m < ld; m += 32) mx = max(mx, m ? max(high(c[2 * m]), high(c[2 * m + 1])) : high(c[0]));
+        for (int m = lane; m < ld; m += 32) {
+            // the sine part of m = 0 takes no part, unless it is not finite
+            const unsigned im = high(c[2 * m + 1]);
+            mx = max(mx, max(high(c[2 * m]), m || not_finite(im) ? im : 0u));
+        }
         const int4* pa = ph + (long long)item[v] * 3 * L;
         const int4* pg = pa + 2 * L;
         if (lane < 3 && !is_phase(pa[lane * L + l])) mx = 0x7FF00000u;
