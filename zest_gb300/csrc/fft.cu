@@ -46,6 +46,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "spectra.cuh"
 
 namespace zgpu {
 
@@ -317,10 +318,10 @@ __global__ void __launch_bounds__(256) rfft_fwd_kernel(const __grid_constant__ F
     }
 }
 
-__global__ void __launch_bounds__(256) rfft_inv_kernel(const __grid_constant__ FftPlan plan,
-                                                       const double* __restrict__ F, int C, int nm, int NC,
-                                                       int lon_fast, double* __restrict__ x, long long xb,
-                                                       long long si, long long sc) {
+template <class In>
+__global__ void __launch_bounds__(256) rfft_inv_kernel(const __grid_constant__ FftPlan plan, const In src, int C,
+                                                       int nm, int NC, int lon_fast, double* __restrict__ x,
+                                                       long long xb, long long si, long long sc) {
     extern __shared__ double2 smem[];
     const int N = plan.N;
     double2* tab = smem;
@@ -338,9 +339,8 @@ __global__ void __launch_bounds__(256) rfft_inv_kernel(const __grid_constant__ F
         const int cp = e % NC;
         const int m = e / NC;
         const int col = col0 + 2 * cp;
-        const double* in = F + (((long long)b * nm + m) * C + col) * 2;
-        const double2 fa = (col < C) ? make_double2(in[0], in[1]) : make_double2(0.0, 0.0);
-        const double2 fb = (col + 1 < C) ? make_double2(in[2], in[3]) : make_double2(0.0, 0.0);
+        const double2 fa = (col < C) ? src.get(b, m, col) : make_double2(0.0, 0.0);
+        const double2 fb = (col + 1 < C) ? src.get(b, m, col + 1) : make_double2(0.0, 0.0);
         if (m == 0) {
             A[plan.in_row[0] * NC + cp] = make_double2(fa.x, -fb.x);
         } else {
@@ -615,7 +615,8 @@ int set_smem_limit() {
     std::lock_guard<std::mutex> lock(mu);
     if (done.count(dev)) return ZEST_GPU_OK;
     ZG_CUDA_TRY(cudaFuncSetAttribute(rfft_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    ZG_CUDA_TRY(cudaFuncSetAttribute(rfft_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ZG_CUDA_TRY(cudaFuncSetAttribute(rfft_inv_kernel<SpectraIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ZG_CUDA_TRY(cudaFuncSetAttribute(rfft_inv_kernel<ParityIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     done.insert(dev);
     return ZEST_GPU_OK;
 }
@@ -633,15 +634,32 @@ int launch_rfft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, long l
     return launch_check("rfft_fwd_kernel");
 }
 
-int launch_rfft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int batch, int lon_fast,
-                    double* x, long long xb, long long si, long long sc) {
+namespace {
+
+template <class In>
+int launch_inv(cudaStream_t s, const FftPlan& plan, const In& src, int C, int nm, int batch, int lon_fast, double* x,
+               long long xb, long long si, long long sc) {
     if (batch <= 0 || C <= 0) return ZEST_GPU_OK;
     ZG_TRY(set_smem_limit());
     const int NC = choose_nc(plan, (long long)C * batch);
     const size_t smem = fft_smem_bytes(plan, NC);
     dim3 grid((C + 2 * NC - 1) / (2 * NC), batch);
-    rfft_inv_kernel<<<grid, threads_for(smem, (long long)grid.x * batch), smem, s>>>(plan, F, C, nm, NC, lon_fast, x, xb, si, sc);
+    rfft_inv_kernel<<<grid, threads_for(smem, (long long)grid.x * batch), smem, s>>>(plan, src, C, nm, NC, lon_fast, x, xb, si, sc);
     return launch_check("rfft_inv_kernel");
+}
+
+}  // namespace
+
+int launch_rfft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int batch, int lon_fast,
+                    double* x, long long xb, long long si, long long sc) {
+    return launch_inv(s, plan, SpectraIn{F, C, nm}, C, nm, batch, lon_fast, x, xb, si, sc);
+}
+
+int launch_rfft_inv_parity(cudaStream_t s, const FftPlan& plan, const double* E, int nlat, int nrad, int kh, int j0u,
+                           int j0d, int nm, int ms, int batch, int lon_fast, double* x, long long xb, long long si,
+                           long long sc) {
+    return launch_inv(s, plan, ParityIn{E, ms, nm, nrad, kh, j0u, j0d, batch}, nlat * nrad, nm, batch, lon_fast, x, xb,
+                      si, sc);
 }
 
 }  // namespace zgpu

@@ -1,6 +1,6 @@
 // Batched real DFT along the longitude axis in 64-bit fixed point: the longitude
-// transforms of the split-precision SH path, and of its Zernike path above order
-// 256.
+// transforms of the split-precision SH path on LonLat grids, and of its Zernike path
+// above order 256.  (LatLon grids keep the FP64 transform of fft.cu.)
 //
 // The FP64 pipe of GB300 retires two operations per clock and SM; the tensor
 // cores need the data cut into slices (20 bytes of traffic per value) and a dense
@@ -15,9 +15,11 @@
 // Numbers.  A column is held as round(x 2^{hb - e}), |x| < 2^e; the DFT of N
 // points grows by at most N sqrt(2) in either component of a packed pair of
 // columns (and every partial sum inside a stage, the Rader product included, by
-// Cauchy-Schwarz), so hb = 62 - ceil(log2(N sqrt 2)), at most 52: N = 399 keeps
-// 52 bits, N = 2047 50, against the 48 bits of the slices that the Legendre sums
-// read.  A value x = xh 2^31 + xl and a root c 2^60 = ch 2^31 + cl (xl, cl
+// Cauchy-Schwarz), so hb = 62 - ceil(log2(N sqrt 2)), at most 52, forward, and with
+// twice the growth for the inverse, whose packed spectra are twice as large: 52 bits
+// forward and 51 inverse at N = 399, 50 and 49 at N = 2047, 49 and 48 at N = 4093,
+// against the 48 bits less one or two of headroom of a tensor product's slices.  A
+// value x = xh 2^31 + xl and a root c 2^60 = ch 2^31 + cl (xl, cl
 // balanced) are multiplied as xh ch, xh cl + xl ch; the dropped xl cl is at most
 // one unit of the result.  Sums of products are kept in two 64-bit accumulators
 // (at most 10 terms each, bounded by 2^63) and shifted once.  Results become FP64
@@ -25,7 +27,7 @@
 // NaN.
 //
 // What bounds it: the integer pipes (multiply and ALU about 60% busy each).
-// Measured, SH order 1024 x 8 (N = 2047), one direction: 0.47 ms; 0.65 as
+// Measured, SH order 1024 x 8 (N = 2047), forward 0.45 ms, inverse 0.48; 0.65 as
 // K-chunked tensor products with their slicing, 1.3 in FP64.  At N = 399 (Zernike
 // order 200 x 64) it takes 16 ms against 13.4 of the tensor products, whose sums
 // are short there: orders up to 256 of the Zernike path stay on the tensor cores.
@@ -41,6 +43,7 @@
 #include "common.cuh"
 #include "fixed.cuh"
 #include "kernels.cuh"
+#include "spectra.cuh"
 
 namespace zgpu {
 
@@ -279,12 +282,12 @@ __device__ __forceinline__ Z* run_plan(Z* a, Z* b, const int4* tab, const FftPla
     return a;
 }
 
-// x(b, i, col) = x + b*xb + i*si + col*sc ; lon_fast: i is the contiguous axis.
+// x(b, i, col) = x + b*xb + i*si + col*sc.
 // F: `ms` orders per item, of which m < nm are written.
 template <int NC>
 __global__ void __launch_bounds__(256) fixed_fwd_kernel(const __grid_constant__ FftPlan plan, int hb,
                                                            const double* __restrict__ x, long long xb, long long si,
-                                                           long long sc, int C, int nm, int ms, int lon_fast,
+                                                           long long sc, int C, int nm, int ms,
                                                            double* __restrict__ F) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int W = 2 * NC;
@@ -301,14 +304,17 @@ __global__ void __launch_bounds__(256) fixed_fwd_kernel(const __grid_constant__ 
     const double* xbp = x + (long long)b * xb;
     long long* Al = reinterpret_cast<long long*>(A);
     auto high = [](double v) { return unsigned(__double2hiint(v)) & 0x7FFFFFFFu; };
-    if (!lon_fast) {
-        // a thread keeps one column: rows i0, i0 + rs, ..
-        const int cl = threadIdx.x & (W - 1), i0 = threadIdx.x / W, rs = blockDim.x / W;
-        const bool in = col0 + cl < C;
+    // a thread keeps one column: rows i0, i0 + rs, ..  Blocks with all their columns
+    // load without a check; with one loop for both the compiler needs registers that
+    // cost the third CTA per SM (SH order 1024 x 8 0.45 against 0.53 ms; 0.48 with the
+    // loads unrolled by 8 instead of 2)
+    auto load = [&](auto whole) {
+        const int cl = threadIdx.x & (W - 1), i0 = threadIdx.x / W, rs = 256 / W;
+        const bool in = decltype(whole)::value || col0 + cl < C;
         const double* p = xbp + (long long)(col0 + cl) * sc + (long long)i0 * si;
         const long long dp = (long long)rs * si;
         unsigned mx = 0;
-#pragma unroll 8
+#pragma unroll 2
         for (int i = i0; i < N; i += rs, p += dp) {
             const double v = in ? *p : 0.0;
             mx = max(mx, high(v));
@@ -324,30 +330,9 @@ __global__ void __launch_bounds__(256) fixed_fwd_kernel(const __grid_constant__ 
             long long* q = Al + plan.in_row[i] * W + cl;
             *q = bad ? 0 : to_fixed_c(__longlong_as_double(*q), c);
         }
-    } else {
-        for (int cl = 0; cl < W; ++cl) {
-            const bool in = col0 + cl < C;
-            const double* p = xbp + (long long)(col0 + cl) * sc;
-            unsigned mx = 0;
-#pragma unroll 4
-            for (int i = threadIdx.x; i < N; i += blockDim.x) {
-                const double v = in ? p[(long long)i * si] : 0.0;
-                mx = max(mx, high(v));
-                Al[plan.in_row[i] * W + cl] = __double_as_longlong(v);
-            }
-            if (mx) atomicMax(&top[cl], mx);
-        }
-        __syncthreads();
-        for (int cl = 0; cl < W; ++cl) {
-            const unsigned h = top[cl];
-            const int c = 1074 + fixed_scale(h) - hb;
-            const bool bad = not_finite(h);
-            for (int i = threadIdx.x; i < N; i += blockDim.x) {
-                long long* q = Al + plan.in_row[i] * W + cl;
-                *q = bad ? 0 : to_fixed_c(__longlong_as_double(*q), c);
-            }
-        }
-    }
+    };
+    if (col0 + W <= C) load(std::true_type{});
+    else load(std::false_type{});
     __syncthreads();
     const Z* Zr = run_plan<NC>(A, Bf, tab, plan);
     // separate the two real spectra and store conj(X_m), m < nm (twice them: hb + 1)
@@ -370,35 +355,9 @@ __global__ void __launch_bounds__(256) fixed_fwd_kernel(const __grid_constant__ 
     }
 }
 
-// Spectra F[b][m][col] as fft.cu lays them out (ms orders per item), or formed
-// from the parity sums E_p[b][m][j'][2 rad + {re, im}] of folded backward
-// Legendre sums (p, b: B items): E_0 + E_1 at the north node lat = j0u + j',
-// E_0 - E_1 at the south node lat = j0d - j' (the equator, j0u = j0d, is north).
-struct SpectraIn {
-    const double* F;
-    int C, ms;
-    __device__ double2 get(int b, int m, int col) const {
-        return *reinterpret_cast<const double2*>(F + (((long long)b * ms + m) * C + col) * 2);
-    }
-};
-struct ParityIn {
-    const double* E;
-    int ms, nm, nrad, kh, j0u, j0d, B;
-    __device__ double2 get(int b, int m, int col) const {
-        const int lat = col / nrad, rad = col - lat * nrad;
-        const bool north = lat >= j0u;
-        const int jf = north ? lat - j0u : j0d - lat;
-        const double* p = E + ((((long long)b * ms + m) * kh + jf) * nrad + rad) * 2;
-        const double2 e0 = *reinterpret_cast<const double2*>(p);
-        double2 e1 = make_double2(0.0, 0.0);  // the last order has no degree of the odd parity
-        if (m + 1 < nm) e1 = *reinterpret_cast<const double2*>(p + (long long)B * ms * kh * nrad * 2);
-        return north ? make_double2(e0.x + e1.x, e0.y + e1.y) : make_double2(e0.x - e1.x, e0.y - e1.y);
-    }
-};
-
 template <int NC, class In>
 __global__ void __launch_bounds__(256) fixed_inv_kernel(const __grid_constant__ FftPlan plan, int hb, const In src,
-                                                           int C, int nm, int lon_fast, double* __restrict__ x,
+                                                           int C, int nm, double* __restrict__ x,
                                                            long long xb, long long si, long long sc) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int W = 2 * NC;
@@ -470,21 +429,13 @@ __global__ void __launch_bounds__(256) fixed_inv_kernel(const __grid_constant__ 
         const long long v = Zl[plan.out_row[i] * W + cl];
         return not_finite(h) ? nan64() : i64_ldexp((cl & 1) ? -v : v, fixed_scale(h) - hb);
     };
-    if (!lon_fast) {
-        const int cl = threadIdx.x & (W - 1), i0 = threadIdx.x / W, rs = blockDim.x / W;
-        if (col0 + cl >= C) return;
-        const unsigned h = top[cl];
-        double* p = xbp + (long long)(col0 + cl) * sc + (long long)i0 * si;
-        const long long dp = (long long)rs * si;
+    const int cl = threadIdx.x & (W - 1), i0 = threadIdx.x / W, rs = blockDim.x / W;
+    if (col0 + cl >= C) return;
+    const unsigned h = top[cl];
+    double* p = xbp + (long long)(col0 + cl) * sc + (long long)i0 * si;
+    const long long dp = (long long)rs * si;
 #pragma unroll 2
-        for (int i = i0; i < N; i += rs, p += dp) *p = value(i, cl, h);
-    } else {
-        for (int cl = 0; cl < W && col0 + cl < C; ++cl) {
-            const unsigned h = top[cl];
-            double* p = xbp + (long long)(col0 + cl) * sc;
-            for (int i = threadIdx.x; i < N; i += blockDim.x) p[(long long)i * si] = value(i, cl, h);
-        }
-    }
+    for (int i = i0; i < N; i += rs, p += dp) *p = value(i, cl, h);
 }
 
 // bits of a column's largest value: the growth by N sqrt(2) (`wide`: twice that,
@@ -531,14 +482,13 @@ int with_nc(const FftPlan& plan, int C, int batch, Go&& go) {
 }
 
 template <class In>
-int launch_inv(cudaStream_t s, const FftPlan& plan, const In& src, int C, int nm, int batch, int lon_fast, double* x,
-               long long xb, long long si, long long sc) {
+int launch_inv(cudaStream_t s, const FftPlan& plan, const In& src, int C, int nm, int batch, double* x, long long xb,
+               long long si, long long sc) {
     if (batch <= 0 || C <= 0) return ZEST_GPU_OK;
     return with_nc(plan, C, batch, [&](auto nc, size_t smem, dim3 grid) -> int {
         constexpr int NC = decltype(nc)::value;
         ZG_TRY(allow_smem(fixed_inv_kernel<NC, In>));
-        fixed_inv_kernel<NC, In><<<grid, 256, smem, s>>>(plan, headroom_bits(plan.N, true), src, C, nm, lon_fast, x, xb,
-                                                         si, sc);
+        fixed_inv_kernel<NC, In><<<grid, 256, smem, s>>>(plan, headroom_bits(plan.N, true), src, C, nm, x, xb, si, sc);
         return launch_check("fixed_inv_kernel");
     });
 }
@@ -559,27 +509,25 @@ void fixed_fft_table(const std::vector<double>& tab, std::vector<int4>& itab) {
 }
 
 int launch_fixed_fft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, long long xb, long long si,
-                         long long sc, int C, int nm, int ms, int batch, int lon_fast, double* F) {
+                         long long sc, int C, int nm, int ms, int batch, double* F) {
     if (batch <= 0 || C <= 0 || nm <= 0) return ZEST_GPU_OK;
     return with_nc(plan, C, batch, [&](auto nc, size_t smem, dim3 grid) -> int {
         constexpr int NC = decltype(nc)::value;
         ZG_TRY(allow_smem(fixed_fwd_kernel<NC>));
-        fixed_fwd_kernel<NC><<<grid, 256, smem, s>>>(plan, headroom_bits(plan.N, false), x, xb, si, sc, C, nm, ms,
-                                                     lon_fast, F);
+        fixed_fwd_kernel<NC><<<grid, 256, smem, s>>>(plan, headroom_bits(plan.N, false), x, xb, si, sc, C, nm, ms, F);
         return launch_check("fixed_fwd_kernel");
     });
 }
 
 int launch_fixed_fft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int ms, int batch,
-                         int lon_fast, double* x, long long xb, long long si, long long sc) {
-    return launch_inv(s, plan, SpectraIn{F, C, ms}, C, nm, batch, lon_fast, x, xb, si, sc);
+                         double* x, long long xb, long long si, long long sc) {
+    return launch_inv(s, plan, SpectraIn{F, C, ms}, C, nm, batch, x, xb, si, sc);
 }
 
 int launch_fixed_fft_inv_parity(cudaStream_t s, const FftPlan& plan, const double* E, int nlat, int nrad, int kh,
-                                int j0u, int j0d, int nm, int ms, int batch, int lon_fast, double* x, long long xb,
-                                long long si, long long sc) {
-    return launch_inv(s, plan, ParityIn{E, ms, nm, nrad, kh, j0u, j0d, batch}, nlat * nrad, nm, batch, lon_fast, x, xb, si,
-                      sc);
+                                int j0u, int j0d, int nm, int ms, int batch, double* x, long long xb, long long si,
+                                long long sc) {
+    return launch_inv(s, plan, ParityIn{E, ms, nm, nrad, kh, j0u, j0d, batch}, nlat * nrad, nm, batch, x, xb, si, sc);
 }
 
 }  // namespace zgpu

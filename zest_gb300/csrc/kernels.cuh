@@ -42,19 +42,22 @@ int launch_rfft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, long l
 // inverse (Hermitian, factor 1): F as above -> x
 int launch_rfft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int batch, int lon_fast,
                     double* x, long long xb, long long si, long long sc);
+// the same from the parity sums E_p[b][m][j'][rad][2] of folded Legendre sums, of
+// which nm of ms orders count: E_0 +- E_1 at the nodes j0u + j' and j0d - j'
+int launch_rfft_inv_parity(cudaStream_t s, const FftPlan& plan, const double* E, int nlat, int nrad, int kh, int j0u,
+                           int j0d, int nm, int ms, int batch, int lon_fast, double* x, long long xb, long long si,
+                           long long sc);
 
 // The same transforms in 64-bit fixed point (fixed_fft.cu): F holds ms orders per
-// item, of which m < nm are written or read (the others count as zero).  The
-// parity form reads the sums E_p[b][m][j'][rad][2] of folded Legendre sums,
-// E_0 +- E_1 at the nodes j0u + j' and j0d - j'.
+// item, of which m < nm are written or read (the others count as zero).
 void fixed_fft_table(const std::vector<double>& tab, std::vector<int4>& itab);
 int launch_fixed_fft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, long long xb, long long si,
-                         long long sc, int C, int nm, int ms, int batch, int lon_fast, double* F);
+                         long long sc, int C, int nm, int ms, int batch, double* F);
 int launch_fixed_fft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int ms, int batch,
-                         int lon_fast, double* x, long long xb, long long si, long long sc);
+                         double* x, long long xb, long long si, long long sc);
 int launch_fixed_fft_inv_parity(cudaStream_t s, const FftPlan& plan, const double* E, int nlat, int nrad, int kh,
-                                int j0u, int j0d, int nm, int ms, int batch, int lon_fast, double* x, long long xb,
-                                long long si, long long sc);
+                                int j0u, int j0d, int nm, int ms, int batch, double* x, long long xb, long long si,
+                                long long sc);
 
 // ---- grouped FP64 contractions ------------------------------------------------
 // Per-call metadata of the folded Legendre / radial stages, all device pointers.

@@ -2236,7 +2236,7 @@ int split_zt_forward(zest_gpu_context* ctx, ZtPlan& plan, int Lg, int Le, int Lm
         const FftPlan* fft;
         ZG_TRY(get_fft(ctx, N, &fft));
         StageScope sc(ctx, ST_FFT_FWD);
-        ZG_TRY(launch_fixed_fft_fwd(s, *fft, grids, sh.size(), C, 1, C, Lm, Lg, batch, 0, G));
+        ZG_TRY(launch_fixed_fft_fwd(s, *fft, grids, sh.size(), C, 1, C, Lm, Lg, batch, G));
     }
     // ---- Legendre (folded over the equator) ----
     {
@@ -2425,7 +2425,7 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
         ZG_TRY(get_fft(ctx, N, &fft));
         StageScope sc(ctx, ST_FFT_INV);
         ZG_TRY(launch_fixed_fft_inv_parity(s, *fft, E, int(sh.nlat), nr, kh, plan.leg.j0u, plan.leg.j0d, Lm, Lg,
-                                           batch, 0, grids, sh.size(), C, 1));
+                                           batch, grids, sh.size(), C, 1));
     }
     return split_finish(ctx);
 }

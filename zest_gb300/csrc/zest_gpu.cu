@@ -433,6 +433,15 @@ int zt_backward_dev(zest_gpu_context* ctx, int zn, int sn, int sp, int Le, int L
     return launch_rfft_inv(s, *fft, G, int(cols), Lg, batch, 0, grids, sh.size(), cols, 1);
 }
 
+// Which longitude transforms of the SH path run in 64-bit fixed point: those of
+// LonLat grids in split precision, with more bits than the tensor products that did
+// them (fixed_fft.cu).  LatLon grids keep the FP64 transform: beside a large mean, or
+// on smooth data, fixed point loses up to 7 bits of the variations against it.  Measured,
+// order 1024 x 8, one direction: 0.36 ms in fixed point, 0.72 in FP64
+// (N = 2048), 0.77 for the inverse from the parity sums; largest error of a grid
+// with variations of 1 beside a mean of 2^20 3.5e-7 and 2.3e-10.
+static bool fixed_st_fft(bool split, bool latlon) { return split && !latlon; }
+
 int st_forward_dev(zest_gpu_context* ctx, int sn, int sp, int layout, int Lg, int Le, int batch,
                    const double* grids, double* coeffs) {
     cudaStream_t s = ctx->stream;
@@ -451,17 +460,15 @@ int st_forward_dev(zest_gpu_context* ctx, int sn, int sp, int layout, int Lg, in
     double* X = ctx->s0.as<double>();
     const bool latlon = layout == ZEST_LAYOUT_LATLON;
     const long long si = latlon ? 1 : sh.nlat, sc_ = latlon ? sh.nlon : 1;  // strides of longitude and latitude
-    if (ctx->precision == ZEST_PRECISION_SPLIT) {
-        {
-            StageScope sc(ctx, ST_FFT_FWD);
-            ZG_TRY(launch_fixed_fft_fwd(s, *fft, grids, sh.size(), si, sc_, int(sh.nlat), Lm, Lg, batch, latlon, X));
-        }
-        return split_st_forward(ctx, *plan, Lg, Lm, batch, X, coeffs, csz);
-    }
+    const bool split = ctx->precision == ZEST_PRECISION_SPLIT;
     {
         StageScope sc(ctx, ST_FFT_FWD);
-        ZG_TRY(launch_rfft_fwd(s, *fft, grids, sh.size(), si, sc_, int(sh.nlat), Lg, batch, latlon, X));
+        if (fixed_st_fft(split, latlon))
+            ZG_TRY(launch_fixed_fft_fwd(s, *fft, grids, sh.size(), si, sc_, int(sh.nlat), Lm, Lg, batch, X));
+        else
+            ZG_TRY(launch_rfft_fwd(s, *fft, grids, sh.size(), si, sc_, int(sh.nlat), Lg, batch, latlon, X));
     }
+    if (split) return split_st_forward(ctx, *plan, Lg, Lm, batch, X, coeffs, csz);
     LegMeta lm;
     lm.P = plan->leg.Pf.as<double>();
     lm.off = plan->leg.off.as<long long>();
@@ -498,8 +505,13 @@ int st_backward_dev(zest_gpu_context* ctx, int sn, int sp, int layout, int Le, i
         ZG_TRY(split_st_backward(ctx, *plan, Lg, Lm, batch, coeffs, csz, &E));
         {
             StageScope sc(ctx, ST_FFT_INV);
-            ZG_TRY(launch_fixed_fft_inv_parity(s, *fft, E, int(sh.nlat), 1, plan->leg.nnodes, plan->leg.j0u,
-                                               plan->leg.j0d, Lm, Lg, batch, latlon, grids, sh.size(), si, sc_));
+            const LegTables& lt = plan->leg;
+            if (fixed_st_fft(true, latlon))
+                ZG_TRY(launch_fixed_fft_inv_parity(s, *fft, E, int(sh.nlat), 1, lt.nnodes, lt.j0u, lt.j0d, Lm, Lg, batch,
+                                                   grids, sh.size(), si, sc_));
+            else
+                ZG_TRY(launch_rfft_inv_parity(s, *fft, E, int(sh.nlat), 1, lt.nnodes, lt.j0u, lt.j0d, Lm, Lg, batch,
+                                              latlon, grids, sh.size(), si, sc_));
         }
         return split_finish(ctx);
     }
