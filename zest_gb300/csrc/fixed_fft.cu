@@ -355,8 +355,8 @@ __global__ void __launch_bounds__(256) fixed_fwd_kernel(const __grid_constant__ 
     }
 }
 
-template <int NC, class In>
-__global__ void __launch_bounds__(256) fixed_inv_kernel(const __grid_constant__ FftPlan plan, int hb, const In src,
+template <int NC>
+__global__ void __launch_bounds__(256) fixed_inv_kernel(const __grid_constant__ FftPlan plan, int hb, const ParityIn src,
                                                            int C, int nm, double* __restrict__ x,
                                                            long long xb, long long si, long long sc) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -481,18 +481,6 @@ int with_nc(const FftPlan& plan, int C, int batch, Go&& go) {
     }
 }
 
-template <class In>
-int launch_inv(cudaStream_t s, const FftPlan& plan, const In& src, int C, int nm, int batch, double* x, long long xb,
-               long long si, long long sc) {
-    if (batch <= 0 || C <= 0) return ZEST_GPU_OK;
-    return with_nc(plan, C, batch, [&](auto nc, size_t smem, dim3 grid) -> int {
-        constexpr int NC = decltype(nc)::value;
-        ZG_TRY(allow_smem(fixed_inv_kernel<NC, In>));
-        fixed_inv_kernel<NC, In><<<grid, 256, smem, s>>>(plan, headroom_bits(plan.N, true), src, C, nm, x, xb, si, sc);
-        return launch_check("fixed_inv_kernel");
-    });
-}
-
 }  // namespace
 
 void fixed_fft_table(const std::vector<double>& tab, std::vector<int4>& itab) {
@@ -519,15 +507,18 @@ int launch_fixed_fft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, l
     });
 }
 
-int launch_fixed_fft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int ms, int batch,
-                         double* x, long long xb, long long si, long long sc) {
-    return launch_inv(s, plan, SpectraIn{F, C, ms}, C, nm, batch, x, xb, si, sc);
-}
-
 int launch_fixed_fft_inv_parity(cudaStream_t s, const FftPlan& plan, const double* E, int nlat, int nrad, int kh,
                                 int j0u, int j0d, int nm, int ms, int batch, double* x, long long xb, long long si,
                                 long long sc) {
-    return launch_inv(s, plan, ParityIn{E, ms, nm, nrad, kh, j0u, j0d, batch}, nlat * nrad, nm, batch, x, xb, si, sc);
+    const int C = nlat * nrad;
+    if (batch <= 0 || C <= 0) return ZEST_GPU_OK;
+    const ParityIn src{E, ms, nm, nrad, kh, j0u, j0d, batch};
+    return with_nc(plan, C, batch, [&](auto nc, size_t smem, dim3 grid) -> int {
+        constexpr int NC = decltype(nc)::value;
+        ZG_TRY(allow_smem(fixed_inv_kernel<NC>));
+        fixed_inv_kernel<NC><<<grid, 256, smem, s>>>(plan, headroom_bits(plan.N, true), src, C, nm, x, xb, si, sc);
+        return launch_check("fixed_inv_kernel");
+    });
 }
 
 }  // namespace zgpu

@@ -48,13 +48,12 @@ int launch_rfft_inv_parity(cudaStream_t s, const FftPlan& plan, const double* E,
                            int j0d, int nm, int ms, int batch, int lon_fast, double* x, long long xb, long long si,
                            long long sc);
 
-// The same transforms in 64-bit fixed point (fixed_fft.cu): F holds ms orders per
-// item, of which m < nm are written or read (the others count as zero).
+// The forward transform and the inverse from parity sums in 64-bit fixed point
+// (fixed_fft.cu): F and E hold ms orders per item, of which m < nm are written or
+// read (the others count as zero).
 void fixed_fft_table(const std::vector<double>& tab, std::vector<int4>& itab);
 int launch_fixed_fft_fwd(cudaStream_t s, const FftPlan& plan, const double* x, long long xb, long long si,
                          long long sc, int C, int nm, int ms, int batch, double* F);
-int launch_fixed_fft_inv(cudaStream_t s, const FftPlan& plan, const double* F, int C, int nm, int ms, int batch,
-                         double* x, long long xb, long long si, long long sc);
 int launch_fixed_fft_inv_parity(cudaStream_t s, const FftPlan& plan, const double* E, int nlat, int nrad, int kh,
                                 int j0u, int j0d, int nm, int ms, int batch, double* x, long long xb, long long si,
                                 long long sc);

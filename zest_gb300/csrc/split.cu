@@ -171,13 +171,6 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&v)[N][4]) {
     for (int a = 0; a < N; ++a)
         asm volatile("" : "+r"(v[a][0]), "+r"(v[a][1]), "+r"(v[a][2]), "+r"(v[a][3]));
 }
-// a * b + c with a 32 x 32 -> 64-bit signed product
-__device__ __forceinline__ long long mad_wide_s32(int a, int b, long long c) {
-    long long r;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
-    return r;
-}
-
 // K-major operand tile of 8 x 16-byte core matrices, no swizzle: the rows of one
 // group of 8 K elements are contiguous (16 bytes each, 8-row groups 128 bytes
 // apart), the next group is kstride bytes further.
@@ -1282,9 +1275,9 @@ __global__ void __launch_bounds__(SP_THREADS, 1)
                             const int i45 = __float2int_rn(__fmaf_rn(__uint_as_float(v[5][j]), 0.00390625f,
                                                                      __uint_as_float(v[4][j])));
                             t = (long long)i01 * 4294967296LL;
-                            t = mad_wide_s32(__float2int_rn(__uint_as_float(v[2][j])), 1 << 24, t);
-                            t = mad_wide_s32(__float2int_rn(__uint_as_float(v[3][j])), 1 << 16, t);
-                            t = mad_wide_s32(i45, 1 << 8, t);
+                            t = mad_wide(__float2int_rn(__uint_as_float(v[2][j])), 1 << 24, t);
+                            t = mad_wide(__float2int_rn(__uint_as_float(v[3][j])), 1 << 16, t);
+                            t = mad_wide(i45, 1 << 8, t);
                         } else {
                             t = i01;
 #pragma unroll

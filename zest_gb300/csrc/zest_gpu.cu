@@ -19,6 +19,7 @@
 #include "context.cuh"
 #include "evaluate.cuh"
 #include "kernels.cuh"
+#include "rotate.cuh"
 #include "split.cuh"
 #include "tables.cuh"
 #include "zest_gpu.h"
@@ -436,10 +437,10 @@ int zt_backward_dev(zest_gpu_context* ctx, int zn, int sn, int sp, int Le, int L
 // Which longitude transforms of the SH path run in 64-bit fixed point: those of
 // LonLat grids in split precision, with more bits than the tensor products that did
 // them (fixed_fft.cu).  LatLon grids keep the FP64 transform: beside a large mean, or
-// on smooth data, fixed point loses up to 7 bits of the variations against it.  Measured,
-// order 1024 x 8, one direction: 0.36 ms in fixed point, 0.72 in FP64
-// (N = 2048), 0.77 for the inverse from the parity sums; largest error of a grid
-// with variations of 1 beside a mean of 2^20 3.5e-7 and 2.3e-10.
+// on smooth data, fixed point loses up to ten bits of the variations against it.
+// Measured, order 1024 x 8, one direction: 0.36 ms in fixed point, 0.72 forward and
+// 0.77 inverse in FP64; largest error of a grid with variations of 1 beside a mean
+// of 2^20 3.5e-7 and 2.3e-10.
 static bool fixed_st_fft(bool split, bool latlon) { return split && !latlon; }
 
 int st_forward_dev(zest_gpu_context* ctx, int sn, int sp, int layout, int Lg, int Le, int batch,
@@ -755,9 +756,8 @@ int rotate_vjp_dev(zest_gpu_context* ctx, int kind, int L, int batch, const doub
         }
         const double* wig;
         ZG_TRY(get_wigner(ctx, L, &wig));
-        const int2* vl;
-        int nvec;
-        ZG_TRY(get_vectors(ctx, kind, L, &vl, &nvec));
+        int nvec = 0;
+        for (int l = 0; l < L; ++l) nvec += vec_count(kind, L, l);
         ZG_TRY(ctx->phase.ensure((size_t)batch * 6 * L * sizeof(double)));
         ZG_TRY(ctx->adj2.ensure((size_t)batch * nvec * 3 * sizeof(double) + 16));
         StageScope sc(ctx, ST_ROTATE);
