@@ -309,11 +309,11 @@ int zest_gpu_zt_rotate_noalloc(void* stream, size_t order, size_t batch, double*
  * Rotates expansion i by euler[3i..3i+2] (in place) and backward-transforms it
  * to a grid of its own order, for n_items expansions.  `orders` (host) must be
  * non-decreasing; `coeffs`, `euler` and `grids` are device buffers, expansions
- * and grids packed back to back in item order.  A call on buffers other than
- * the last call's runs the work eagerly; the second call in a row for the same
- * (orders, buffers, conventions, precision) records it into a CUDA graph on
- * the context, and later ones replay the graph (recorded anew if any of the
- * context's device buffers was freed or reallocated since, e.g. by
+ * and grids packed back to back in item order.  The first call for a given
+ * (orders, buffers, conventions, precision) runs the work eagerly and records
+ * it into a CUDA graph on the context; a later identical call replays the
+ * graph (recorded anew after a call with others, and if any of the context's
+ * device buffers was freed or reallocated since, e.g. by
  * zest_gpu_trim).  Results are those of
  * zest_gpu_zt_rotate + zest_gpu_zt_backward per item; in
  * ZEST_PRECISION_SPLIT (orders up to 256) the rotation runs in 64-bit fixed

@@ -121,9 +121,22 @@ struct RaggedCall {
     }
 };
 
+// A recorded CUDA graph, ready to launch.
+struct RecordedGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    RecordedGraph() = default;
+    RecordedGraph(const RecordedGraph&) = delete;
+    RecordedGraph& operator=(const RecordedGraph&) = delete;
+    ~RecordedGraph() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+    }
+};
+
 // A batch of expansions of different orders (rotate, then backward
 // transform): its device work lists, the last call, and the CUDA graph that
-// replays that call once it has been repeated.
+// replays that call.
 struct RaggedPlan {
     std::vector<int> orders;
     RaggedCall call;
@@ -134,16 +147,8 @@ struct RaggedPlan {
     DevBuf voff_dev;
     std::vector<long long> coff_h, goff_h;
     std::vector<std::tuple<int, int, int>> buckets;            // {order, first item, count}
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    unsigned long long epoch = ~0ull;  // alloc_epoch() after the last call's eager run
-    void drop_graph() {
-        if (exec) cudaGraphExecDestroy(exec);
-        if (graph) cudaGraphDestroy(graph);
-        exec = nullptr;
-        graph = nullptr;
-    }
-    ~RaggedPlan() { drop_graph(); }
+    std::unique_ptr<RecordedGraph> recorded;                   // null where the last call failed
+    unsigned long long epoch = 0;                              // alloc_epoch() when it was recorded
 };
 
 struct TileEntry {

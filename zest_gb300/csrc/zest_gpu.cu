@@ -771,12 +771,13 @@ int rotate_vjp_dev(zest_gpu_context* ctx, int kind, int L, int batch, const doub
 // ---------------------------------------------------------------------------
 // Batches of expansions of different orders: rotate every expansion (one
 // launch over a ragged work list), then backward-transform each group of equal
-// order as one batch.  The offsets and the rotation's work list belong to the
-// orders and are kept for the last ones; a call with other buffers (or conventions)
-// runs eagerly -- the first one builds tables and scratch and autotunes tile
-// shapes -- and a call that repeats the last one is recorded into a CUDA graph and
-// replayed from then on (a single launch from the host).  Rebuilding lists and
-// graph for every change of buffers took 8 ms of 51 for 1,024 items.
+// order as one batch.  A call on other buffers, conventions or orders than the last
+// one's runs eagerly -- building tables, lists and scratch where they are missing,
+// and autotuning tile shapes -- and is recorded into a CUDA graph beside it; a later
+// identical call replays the graph (a single launch from the host).  The offsets and
+// the rotation's work list belong to the orders and are kept for the last ones.
+// Measured, 1,024 items of orders 8 to 128 in split precision: a replay 34.8 ms, the
+// first call on other buffers 36.9, on other orders 48.2.
 static int ragged_sequence(zest_gpu_context* ctx, RaggedPlan& P) {
     const RaggedCall& c = P.call;
     const double* wig;
@@ -825,43 +826,44 @@ static int on_graph_stream(zest_gpu_context* ctx, F&& body) {
 static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp, const std::vector<int>& orders,
                                   double* coeffs, const double* euler, int type, double* grids);
 
-// Runs the sequence of `call` and remembers it: every table, list and buffer that
-// a graph of it needs then exists.  The split GEMMs' wait flag is checked once, at
-// the end, not after every group.
-static int ragged_eager(zest_gpu_context* ctx, RaggedPlan& P, const RaggedCall& call) {
-    if (P.exec) ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // its last replay may still run
-    P.drop_graph();
-    P.call = call;
-    P.epoch = ~0ull;  // no graph of a call that failed
-    ZG_TRY(ctx->phase.ensure((size_t)P.orders.size() * 6 * std::max(P.Lmax, 1) * sizeof(double)));
-    ctx->defer_finish = true;
-    int rc = ragged_sequence(ctx, P);
-    ctx->defer_finish = false;
-    if (call.precision == ZEST_PRECISION_SPLIT) {
-        const int late = split_check_flag(ctx);
-        if (rc == ZEST_GPU_OK) rc = late;
-    }
-    if (rc == ZEST_GPU_OK) P.epoch = alloc_epoch().load(std::memory_order_relaxed);
-    return rc;
-}
-
-// Records the sequence of the plan's last call into a graph (nothing executes).
+// Records the sequence of the plan's call into a graph (nothing executes).
 static int ragged_record(zest_gpu_context* ctx, RaggedPlan& P) {
+    auto r = std::make_unique<RecordedGraph>();
     const bool prof = ctx->prof.on;
     ctx->prof.on = false;
     ZG_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
     const int rc = ragged_sequence(ctx, P);
-    cudaGraph_t g = nullptr;
-    const cudaError_t ec = cudaStreamEndCapture(ctx->stream, &g);
+    const cudaError_t ec = cudaStreamEndCapture(ctx->stream, &r->graph);
     ctx->prof.on = prof;
-    if (rc != ZEST_GPU_OK) {
-        if (g) cudaGraphDestroy(g);
-        return rc;
-    }
+    if (rc != ZEST_GPU_OK) return rc;
     if (ec != cudaSuccess) return fail(ZEST_GPU_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ec));
-    P.graph = g;
-    ZG_CUDA_TRY(cudaGraphInstantiate(&P.exec, g, 0));
+    ZG_CUDA_TRY(cudaGraphInstantiate(&r->exec, r->graph, 0));
+    P.recorded = std::move(r);
     return ZEST_GPU_OK;
+}
+
+// Runs the sequence of `call` -- every table, list and buffer that a graph of it
+// needs then exists -- and, while the device works on it, records it and gives the
+// last call's graph back (for 1,024 items both are done before the device is: no
+// time; 12 items 0.50 ms, a replay 0.35).  The split GEMMs' wait flag is checked
+// once, at the end, not after every group.
+static int ragged_eager(zest_gpu_context* ctx, RaggedPlan& P, const RaggedCall& call) {
+    std::unique_ptr<RecordedGraph> last = std::move(P.recorded);
+    if (last) ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // its last replay may still run
+    P.call = call;
+    ZG_TRY(ctx->phase.ensure((size_t)P.orders.size() * 6 * std::max(P.Lmax, 1) * sizeof(double)));
+    ctx->defer_finish = true;
+    int rc = ragged_sequence(ctx, P);
+    ctx->defer_finish = false;
+    P.epoch = alloc_epoch().load(std::memory_order_relaxed);
+    if (rc == ZEST_GPU_OK) rc = ragged_record(ctx, P);
+    last.reset();
+    if (call.precision == ZEST_PRECISION_SPLIT) {
+        const int late = split_check_flag(ctx);
+        if (rc == ZEST_GPU_OK) rc = late;
+    }
+    if (rc != ZEST_GPU_OK) P.recorded.reset();
+    return rc;
 }
 
 int zt_rotate_backward_ragged_dev(zest_gpu_context* ctx, int zn, int sn, int sp, const std::vector<int>& orders,
@@ -875,11 +877,9 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
     RaggedPlan* P = ctx->ragged.get();
     if (P && P->orders == orders) {
         // the graph's kernels hold pointers to scratch, tables and work lists: a
-        // buffer freed or reallocated since the last run means running eagerly anew
-        const bool again = P->call == call && P->epoch == alloc_epoch().load(std::memory_order_relaxed);
-        if (again && !P->exec) ZG_TRY(ragged_record(ctx, *P));
-        if (again) {
-            ZG_CUDA_TRY(cudaGraphLaunch(P->exec, ctx->stream));
+        // buffer freed or reallocated since it was recorded means recording anew
+        if (P->recorded && P->call == call && P->epoch == alloc_epoch().load(std::memory_order_relaxed)) {
+            ZG_CUDA_TRY(cudaGraphLaunch(P->recorded->exec, ctx->stream));
             return call.precision == ZEST_PRECISION_SPLIT ? split_check_flag(ctx) : ZEST_GPU_OK;
         }
         return ragged_eager(ctx, *P, call);
@@ -918,7 +918,10 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
         ZG_TRY(upload(np->vecl, byl, ctx->stream));
         ZG_TRY(upload(np->voff_dev, np->voff, ctx->stream));
     }
-    if (P && P->exec) ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (P && P->recorded) {
+        ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        np->recorded = std::move(P->recorded);  // given back beside the run
+    }
     ctx->ragged = std::move(np);
     return ragged_eager(ctx, *ctx->ragged, call);
 }
