@@ -222,6 +222,18 @@ namespace zgpu {
 // The plan of the longitude transforms of length N, cached (zest_gpu.cu).
 int get_fft(zest_gpu_context* ctx, int N, const FftPlan** out);
 
+// Gives a variable another value for the lifetime of the object, also where an
+// exception ends it.
+template <class T>
+struct ScopedValue {
+    T& ref;
+    const T before;
+    ScopedValue(T& r, T v) : ref(r), before(r) { ref = v; }
+    ScopedValue(const ScopedValue&) = delete;
+    ScopedValue& operator=(const ScopedValue&) = delete;
+    ~ScopedValue() { ref = before; }
+};
+
 // Brackets one pipeline stage with events when profiling is on.
 struct StageScope {
     zest_gpu_context* ctx;

@@ -812,14 +812,23 @@ static int on_graph_stream(zest_gpu_context* ctx, F&& body) {
         ZG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->graph_ev[0], cudaEventDisableTiming));
         ZG_CUDA_TRY(cudaEventCreateWithFlags(&ctx->graph_ev[1], cudaEventDisableTiming));
     }
-    cudaStream_t user = ctx->stream;
+    const cudaStream_t user = ctx->stream;
     ZG_CUDA_TRY(cudaEventRecord(ctx->graph_ev[0], user));
     ZG_CUDA_TRY(cudaStreamWaitEvent(ctx->graph_stream, ctx->graph_ev[0], 0));
-    ctx->stream = ctx->graph_stream;
-    const int rc = body();
-    ctx->stream = user;
-    ZG_CUDA_TRY(cudaEventRecord(ctx->graph_ev[1], ctx->graph_stream));
-    ZG_CUDA_TRY(cudaStreamWaitEvent(user, ctx->graph_ev[1], 0));
+    auto join = [&]() -> int {
+        ZG_CUDA_TRY(cudaEventRecord(ctx->graph_ev[1], ctx->graph_stream));
+        ZG_CUDA_TRY(cudaStreamWaitEvent(user, ctx->graph_ev[1], 0));
+        return ZEST_GPU_OK;
+    };
+    int rc = ZEST_GPU_OK;
+    try {
+        const ScopedValue<cudaStream_t> stream(ctx->stream, ctx->graph_stream);
+        rc = body();
+    } catch (...) {  // an allocation of the host that failed
+        join();
+        throw;
+    }
+    ZG_TRY(join());
     return rc;
 }
 
@@ -829,12 +838,16 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
 // Records the sequence of the plan's call into a graph (nothing executes).
 static int ragged_record(zest_gpu_context* ctx, RaggedPlan& P) {
     auto r = std::make_unique<RecordedGraph>();
-    const bool prof = ctx->prof.on;
-    ctx->prof.on = false;
+    const ScopedValue<bool> prof(ctx->prof.on, false);
     ZG_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
-    const int rc = ragged_sequence(ctx, P);
+    int rc = ZEST_GPU_OK;
+    try {
+        rc = ragged_sequence(ctx, P);
+    } catch (...) {
+        cudaStreamEndCapture(ctx->stream, &r->graph);
+        throw;
+    }
     const cudaError_t ec = cudaStreamEndCapture(ctx->stream, &r->graph);
-    ctx->prof.on = prof;
     if (rc != ZEST_GPU_OK) return rc;
     if (ec != cudaSuccess) return fail(ZEST_GPU_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ec));
     ZG_CUDA_TRY(cudaGraphInstantiate(&r->exec, r->graph, 0));
@@ -852,9 +865,11 @@ static int ragged_eager(zest_gpu_context* ctx, RaggedPlan& P, const RaggedCall& 
     if (last) ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // its last replay may still run
     P.call = call;
     ZG_TRY(ctx->phase.ensure((size_t)P.orders.size() * 6 * std::max(P.Lmax, 1) * sizeof(double)));
-    ctx->defer_finish = true;
-    int rc = ragged_sequence(ctx, P);
-    ctx->defer_finish = false;
+    int rc = ZEST_GPU_OK;
+    {
+        const ScopedValue<bool> once(ctx->defer_finish, true);
+        rc = ragged_sequence(ctx, P);
+    }
     P.epoch = alloc_epoch().load(std::memory_order_relaxed);
     if (rc == ZEST_GPU_OK) rc = ragged_record(ctx, P);
     last.reset();
