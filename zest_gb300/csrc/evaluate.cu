@@ -255,7 +255,7 @@ int zt_evaluate_dev(zest_gpu_context* ctx, int zn, int sn, int sp, int L, int ba
             for (int m = 0; m < L; ++m) add_tiles(v, m, nlat, (long long)nb * 2 * nrad, bm, bn);
             ZG_TRY(upload_tiles(ctx, E.tiles[1], v, w, &tg));
             v.clear();
-            w = zt_tile_rule(nb * nlon * npts, nlon);
+            w = zt_tile_rule((long long)nb * nlon * npts, nlon);
             zt_tile_shape(w, bm, bn);
             for (int b = 0; b < nb; ++b) add_tiles(v, b, nlon, npts, bm, bn);
             ZG_TRY(upload_tiles(ctx, E.tiles[2], v, w, &tn));
