@@ -462,8 +462,10 @@ int allow_smem(Kern kern) {
     int dev = 0;
     ZG_CUDA_TRY(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(mu);
-    if (!done.insert({reinterpret_cast<const void*>(kern), dev}).second) return ZEST_GPU_OK;
+    const std::pair<const void*, int> key(reinterpret_cast<const void*>(kern), dev);
+    if (done.count(key)) return ZEST_GPU_OK;
     ZG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
+    done.insert(key);
     return ZEST_GPU_OK;
 }
 

@@ -385,8 +385,6 @@ struct LegBwdLoader {
     __device__ int kvalid(const Row& R) const { return (Lm - R.m + 1) / 2; }  // l = m + 2k < Lm
 };
 
-// SH coefficients [b][tri(l,m)][c], rows (m, b, c); k = i: the pair
-// (l = m + 2i, l + 1), zero from Lm on (the two parity operands).
 // rows (m, b, kc) of flm; k = q: flm(l = m + q), zero from Lm on (the data of
 // the unfolded backward Legendre sums, all l of one m in one operand)
 struct LegBwdULoader {
@@ -408,6 +406,8 @@ struct LegBwdULoader {
     __device__ int kvalid(const Row& R) const { return Lm - R.m; }  // l = m + k < Lm
 };
 
+// SH coefficients [b][tri(l,m)][c], rows (m, b, c); k = i: the pair
+// (l = m + 2i, l + 1), zero from Lm on (the two parity operands).
 struct StLegBwdLoader {
     static constexpr bool ROW_FAST = true, TWO = true;
     static constexpr int MODE = SL_PAIR, SHIFT = 0;
@@ -1503,7 +1503,7 @@ struct ZtSplitTables {
     SliceArray leg_bU;
 };
 
-// Sliced Legendre tables of one SH plan (the 128-row operand: no scaled copies).
+// Sliced Legendre tables of one SH plan (the 128-row operand).
 struct StSplitTables {
     int S = 0;
     SliceArray leg_f, leg_bT;
@@ -2426,8 +2426,8 @@ int split_zt_backward(zest_gpu_context* ctx, ZtPlan& plan, int Le, int Lg, int L
 // ===========================================================================
 // Split-precision SH Legendre sums.  The table is the 128-row operand: with
 // 2 x batch data rows per order m the data could not fill a row tile.  The
-// data (the folded spectra, or the coefficients) is the scaled-copy operand,
-// sliced per call; its 2 x batch rows are the columns.
+// data (the folded spectra, or the coefficients) is sliced per call; its 2 x batch
+// rows are the columns.
 // ===========================================================================
 namespace {
 // SH sums always use 8-bit digits and 6 slices; sums longer than 256 run as
