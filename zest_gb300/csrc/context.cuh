@@ -125,6 +125,7 @@ struct RaggedCall {
 struct RecordedGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    bool launched = false;
     RecordedGraph() = default;
     RecordedGraph(const RecordedGraph&) = delete;
     RecordedGraph& operator=(const RecordedGraph&) = delete;

@@ -862,7 +862,7 @@ static int ragged_record(zest_gpu_context* ctx, RaggedPlan& P) {
 // once, at the end, not after every group.
 static int ragged_eager(zest_gpu_context* ctx, RaggedPlan& P, const RaggedCall& call) {
     std::unique_ptr<RecordedGraph> last = std::move(P.recorded);
-    if (last) ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // its last replay may still run
+    if (last && last->launched) ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // it may still run
     P.call = call;
     ZG_TRY(ctx->phase.ensure((size_t)P.orders.size() * 6 * std::max(P.Lmax, 1) * sizeof(double)));
     int rc = ZEST_GPU_OK;
@@ -894,6 +894,7 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
         // the graph's kernels hold pointers to scratch, tables and work lists: a
         // buffer freed or reallocated since it was recorded means recording anew
         if (P->recorded && P->call == call && P->epoch == alloc_epoch().load(std::memory_order_relaxed)) {
+            P->recorded->launched = true;
             ZG_CUDA_TRY(cudaGraphLaunch(P->recorded->exec, ctx->stream));
             return call.precision == ZEST_PRECISION_SPLIT ? split_check_flag(ctx) : ZEST_GPU_OK;
         }
@@ -933,11 +934,8 @@ static int ragged_on_graph_stream(zest_gpu_context* ctx, int zn, int sn, int sp,
         ZG_TRY(upload(np->vecl, byl, ctx->stream));
         ZG_TRY(upload(np->voff_dev, np->voff, ctx->stream));
     }
-    if (P && P->recorded) {
-        ZG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        np->recorded = std::move(P->recorded);  // given back beside the run
-    }
-    ctx->ragged = std::move(np);
+    if (P) np->recorded = std::move(P->recorded);  // given back beside the run
+    ctx->ragged = std::move(np);  // nothing uses the last lists any more: the uploads waited for the stream
     return ragged_eager(ctx, *ctx->ragged, call);
 }
 
