@@ -88,7 +88,10 @@ int zest_gpu_ctx_destroy(zest_gpu_context* ctx);
 const char* zest_gpu_last_error(void);
 /* Precision of the dense contractions; `slices` = number of FP16 digit
  * slices per operand for ZEST_PRECISION_SPLIT (4..6, 0 = default 6), 8-bit
- * digits, sums longer than 256 terms in chunks of at most 256. */
+ * digits, sums longer than 256 terms in chunks of at most 256.  Beside the
+ * contractions, ZEST_PRECISION_SPLIT runs rotations of orders up to 256 and the
+ * longitude transforms of SH LonLat grids and of Zernike grids above order 256
+ * in 64-bit fixed point; SH LatLon grids keep the FP64 longitude transform. */
 int zest_gpu_set_precision(zest_gpu_context* ctx, int precision, int slices);
 int zest_gpu_synchronize(zest_gpu_context* ctx);
 /* Releases cached tables and scratch (they are rebuilt on demand). */
