@@ -123,3 +123,25 @@ def test_buffers_freed_between_calls(precision):
         check(got, want[s])
         assert (got[2] == 0) == (s not in (0, 3)), (s, got[2])
     ctx.close()
+
+
+def test_within_a_capture_of_the_caller():
+    # a call on the context's stream while the caller captures it is part of the caller's
+    # graph, on buffers that the context has run before and on others
+    import zest_gb300 as zg
+    stream = torch.cuda.Stream()
+    ctx = zg.Context(0, stream.cuda_stream)
+    one, two = Batch(ORDERS), Batch(ORDERS)
+    want = [expected(0, ORDERS, s) for s in range(4)]
+    check(one.run(ctx, 0), want[0])
+    check(two.run(ctx, 1), want[1])
+    for s, b in ((2, one), (3, two)):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+            ctx.zt_rotate_backward_ragged(b.orders, b.coeffs, b.euler, b.grids)
+        b.fill(s)
+        graph.replay()
+        torch.cuda.synchronize()
+        check((b.coeffs.cpu().numpy(), b.grids.cpu().numpy()), want[s])
+        check(b.run(ctx, 1), want[1])
+    ctx.close()

@@ -871,7 +871,9 @@ static int ragged_eager(zest_gpu_context* ctx, RaggedPlan& P, const RaggedCall& 
         rc = ragged_sequence(ctx, P);
     }
     P.epoch = alloc_epoch().load(std::memory_order_relaxed);
-    if (rc == ZEST_GPU_OK) rc = ragged_record(ctx, P);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;  // a caller's own capture takes the run as it is
+    ZG_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &cap));
+    if (rc == ZEST_GPU_OK && cap == cudaStreamCaptureStatusNone) rc = ragged_record(ctx, P);
     last.reset();
     if (call.precision == ZEST_PRECISION_SPLIT) {
         const int late = split_check_flag(ctx);
